@@ -304,35 +304,58 @@ __global__ void k_nve2(const int2* __restrict__ chunks, const SysDev* __restrict
 // Lennard-Jones core repulsion of the MD harness (the C1 workload's
 // LJ eps, sigma, r_cut), over the same full neighbour list: adds forces and
 // half the pair energy per particle to force, the system total to energy[s].
-template <typename T4, typename T>
-__global__ void k_lj(const int2* __restrict__ chunks, const SysDev* __restrict__ sys, const T4* __restrict__ pos,
-                     const uint32_t* __restrict__ head, const uint32_t* __restrict__ nn,
-                     const uint32_t* __restrict__ nl, T eps, T sig2, T rc2, T4* __restrict__ force,
-                     double* __restrict__ energy) {
+// TPP lanes share one particle's row (consecutive lanes read consecutive
+// entries) and a 256-particle chunk is spread over TPP CTAs; the kernel is a
+// chain of dependent gathers, so its time is the entries per lane. One lane
+// per particle left 164 of them in series on 4 CTAs (N = 1,000, FP64: 102 us
+// per launch); 32 lanes leave 6 on 125 CTAs (5.8 us).
+template <typename T4, typename T, int TPP>
+__global__ void __launch_bounds__(256)
+    k_lj(const int2* __restrict__ chunks, const SysDev* __restrict__ sys, const T4* __restrict__ pos,
+         const uint32_t* __restrict__ head, const uint32_t* __restrict__ nn, const uint32_t* __restrict__ nl, T eps,
+         T sig2, T rc2, T4* __restrict__ force, double* __restrict__ energy) {
     __shared__ double red[32];
-    const int2 ch = chunks[blockIdx.x];
-    const SysDev S = sys[ch.x];
-    const int i = ch.y + threadIdx.x;
-    const T L[3] = {(T)S.Lxd, (T)S.Lyd, (T)S.Lzd};
-    double e1[1] = {0.0};
-    if (i < S.p_off + S.N) {
+    const int2 ch = chunks[blockIdx.x / TPP];
+    const SysDev& S = sys[ch.x];
+    const int i = ch.y + (blockIdx.x % TPP) * (256 / TPP) + threadIdx.x / TPP, sub = threadIdx.x % TPP;
+    const T Lx = (T)S.Lxd, Ly = (T)S.Lyd, Lz = (T)S.Lzd;
+    const T iLx = (T)1 / Lx, iLy = (T)1 / Ly, iLz = (T)1 / Lz;
+    const bool valid = i < S.p_off + S.N;
+    const int po = S.p_off;
+    T fx = 0, fy = 0, fz = 0, en = 0;
+    if (valid) {
         const T4 pi = pos[i];
-        T fx = 0, fy = 0, fz = 0, en = 0;
         const uint32_t h = head[i], n = nn[i];
-        for (uint32_t k = 0; k < n; ++k) {
-            const T4 pj = pos[S.p_off + (int)nl[h + k]];
-            T d[3] = {pi.x - pj.x, pi.y - pj.y, pi.z - pj.z};
-            for (int a = 0; a < 3; ++a) d[a] -= L[a] * rint(d[a] / L[a]);
-            const T r2 = d[0] * d[0] + d[1] * d[1] + d[2] * d[2];
+        uint32_t jn = sub < n ? nl[h + sub] : 0u;
+        for (uint32_t k = sub; k < n; k += TPP) {
+            const T4 pj = pos[po + (int)jn];
+            if (k + TPP < n) jn = nl[h + k + TPP];  // loaded one step ahead of its gather
+            T dx = pi.x - pj.x, dy = pi.y - pj.y, dz = pi.z - pj.z;
+            // minimum image by the reciprocal box length; it differs from a
+            // division only for pairs at |d| = L/2, beyond every listed cutoff
+            dx -= Lx * rint(dx * iLx);
+            dy -= Ly * rint(dy * iLy);
+            dz -= Lz * rint(dz * iLz);
+            const T r2 = dx * dx + dy * dy + dz * dz;
             if (r2 < rc2 && r2 > 0) {
-                const T s2 = sig2 / r2, s6 = s2 * s2 * s2;
-                const T fdr = (T)24 * eps * ((T)2 * s6 * s6 - s6) / r2;
+                const T i2 = (T)1 / r2, s2 = sig2 * i2, s6 = s2 * s2 * s2;
+                const T fdr = (T)24 * eps * ((T)2 * s6 * s6 - s6) * i2;
                 en += (T)4 * eps * (s6 * s6 - s6);
-                fx += fdr * d[0];
-                fy += fdr * d[1];
-                fz += fdr * d[2];
+                fx += fdr * dx;
+                fy += fdr * dy;
+                fz += fdr * dz;
             }
         }
+    }
+#pragma unroll
+    for (int o = TPP / 2; o > 0; o >>= 1) {
+        fx += __shfl_xor_sync(0xffffffffu, fx, o);
+        fy += __shfl_xor_sync(0xffffffffu, fy, o);
+        fz += __shfl_xor_sync(0xffffffffu, fz, o);
+        en += __shfl_xor_sync(0xffffffffu, en, o);
+    }
+    double e1[1] = {0.0};
+    if (valid && sub == 0) {
         T4 f = force[i];
         f.x += fx;
         f.y += fy;
@@ -389,17 +412,30 @@ __global__ void k64_nve2(const int2* __restrict__ chunks, const SysDev* __restri
     vel[i] = v;
 }
 
+constexpr int LJ_WARP_CHUNKS = 37;  // 148 SMs x 64 warps / 256 particles
+
+template <typename T4, typename T>
+static void lj_launch(const int2* chunks, int n_chunks, const SysDev* sys, const void* pos, const uint32_t* head,
+                      const uint32_t* nn, const uint32_t* nl, double eps, double sigma, double rcut, void* force,
+                      double* energy, cudaStream_t st) {
+    const T e = (T)eps, s2 = (T)(sigma * sigma), r2 = (T)(rcut * rcut);
+    // a warp per particle while that does not oversubscribe the GPU (148 SMs
+    // x 64 warps, 256-particle chunks), else 8 lanes: fewer idle lanes in the
+    // last pass over a row and cheaper reductions
+    if (n_chunks <= LJ_WARP_CHUNKS)
+        k_lj<T4, T, 32><<<n_chunks * 32, 256, 0, st>>>(chunks, sys, (const T4*)pos, head, nn, nl, e, s2, r2, (T4*)force, energy);
+    else
+        k_lj<T4, T, 8><<<n_chunks * 8, 256, 0, st>>>(chunks, sys, (const T4*)pos, head, nn, nl, e, s2, r2, (T4*)force, energy);
+}
+
 cudaError_t launch_lj(const int2* chunks, int n_chunks, const SysDev* sys, const void* pos, const uint32_t* head,
                       const uint32_t* nn, const uint32_t* nl, double eps, double sigma, double rcut, void* force,
                       double* energy, bool f64, cudaStream_t st) {
     if (n_chunks == 0) return cudaSuccess;
     if (f64)
-        k_lj<double4, double><<<n_chunks, 256, 0, st>>>(chunks, sys, (const double4*)pos, head, nn, nl, eps,
-                                                        sigma * sigma, rcut * rcut, (double4*)force, energy);
+        lj_launch<double4, double>(chunks, n_chunks, sys, pos, head, nn, nl, eps, sigma, rcut, force, energy, st);
     else
-        k_lj<float4, float><<<n_chunks, 256, 0, st>>>(chunks, sys, (const float4*)pos, head, nn, nl, (float)eps,
-                                                      (float)(sigma * sigma), (float)(rcut * rcut), (float4*)force,
-                                                      energy);
+        lj_launch<float4, float>(chunks, n_chunks, sys, pos, head, nn, nl, eps, sigma, rcut, force, energy, st);
     return cudaGetLastError();
 }
 
