@@ -187,43 +187,74 @@ __global__ void k_scatter(const int2* __restrict__ chunks, const SysDev* __restr
 // origin of the stencil inside the tile, index), so the permutation equals a
 // stable sort on (key, y origin, index). Grouping equal y origins lets the
 // spreading kernel's warps skip the k-steps whose stencil rows miss theirs.
-// The composite rank key is (oy << 26) | (index - system's first particle).
+// The keys (y origin << 26) | (index - system's first particle) are first
+// counted into one bucket per y origin in shared memory; a key's rank is its
+// bucket's start plus the smaller keys of its own bucket. The comparisons are
+// what bounds a full tile: ranking against the whole tile is n^2, against the
+// bucket n^2 / T (T = 11, 98,304 particles in 125 tiles: 27.8 us against
+// 399 us). Tiles above SORT_CAP particles rank straight from memory.
 // Also gathers the sorted particle records.
 __device__ __forceinline__ uint32_t sort_key(uint32_t v, const uint32_t* __restrict__ rel, int p_off) {
     return (((rel[v] >> 8) & 255u) << 26) | (v - (uint32_t)p_off);
 }
 
-__global__ void k_tile_sort(const uint32_t* __restrict__ start, const uint32_t* __restrict__ perm_u,
-                            uint32_t* __restrict__ perm, const float4* __restrict__ trec,
-                            const uint32_t* __restrict__ rel, float4* __restrict__ srec,
-                            uint32_t* __restrict__ srel, const int* __restrict__ tile_sys,
-                            const SysDev* __restrict__ sys) {
-    __shared__ __align__(16) uint32_t sm[SORT_CAP];
+constexpr int SORT_BUCKETS = 64;  // y origins inside a tile (the tile edge is at most 64)
+
+__global__ void __launch_bounds__(512)
+    k_tile_sort(const uint32_t* __restrict__ start, const uint32_t* __restrict__ perm_u, uint32_t* __restrict__ perm,
+                const float4* __restrict__ trec, const uint32_t* __restrict__ rel, float4* __restrict__ srec,
+                uint32_t* __restrict__ srel, const int* __restrict__ tile_sys, const SysDev* __restrict__ sys) {
+    __shared__ uint32_t sm[SORT_CAP];
+    __shared__ uint32_t cnt[SORT_BUCKETS], beg[SORT_BUCKETS];
     const uint32_t s0 = start[blockIdx.x];
     const uint32_t n = start[blockIdx.x + 1] - s0;
     if (n == 0) return;
-    const int p_off = sys[tile_sys[blockIdx.x]].p_off;
-    const bool cached = n <= (uint32_t)SORT_CAP;
-    const uint32_t n4 = (n + 3u) >> 2;
-    if (cached) {
-        for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) sm[i] = sort_key(perm_u[s0 + i], rel, p_off);
-        // pad to whole 16-byte groups with a value no key is above
-        if (threadIdx.x < 4u * n4 - n) sm[n + threadIdx.x] = 0xffffffffu;
+    const uint32_t p_off = (uint32_t)sys[tile_sys[blockIdx.x]].p_off;
+    if (n <= (uint32_t)SORT_CAP) {
+        if (threadIdx.x < SORT_BUCKETS) cnt[threadIdx.x] = 0u;
+        __syncthreads();
+        for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) {
+            const uint32_t v = perm_u[s0 + i];
+            atomicAdd(&cnt[(rel[v] >> 8) & 255u], 1u);
+        }
+        __syncthreads();
+        if (threadIdx.x < 32) {
+            const int l = threadIdx.x;
+            const uint32_t a = cnt[2 * l], b = cnt[2 * l + 1];
+            uint32_t x = a + b;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
+                if (l >= o) x += y;
+            }
+            beg[2 * l] = x - a - b;
+            beg[2 * l + 1] = x - b;
+            cnt[2 * l] = x - a - b;  // the bucket's fill cursor, its end once filled
+            cnt[2 * l + 1] = x - b;
+        }
+        __syncthreads();
+        for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) {
+            const uint32_t v = perm_u[s0 + i];
+            sm[atomicAdd(&cnt[(rel[v] >> 8) & 255u], 1u)] = v;
+        }
+        __syncthreads();
+        for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) {
+            const uint32_t v = sm[i], rl = rel[v], bk = (rl >> 8) & 255u;
+            const uint32_t b0 = beg[bk], b1 = cnt[bk];
+            const float4 rec = trec[v];
+            uint32_t r = b0;
+            for (uint32_t j = b0; j < b1; ++j) r += sm[j] < v ? 1u : 0u;
+            perm[s0 + r] = v;
+            srec[s0 + r] = rec;
+            srel[s0 + r] = rl;
+        }
+        return;
     }
-    __syncthreads();
     for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) {
         const uint32_t v = perm_u[s0 + i];
-        const uint32_t kv = cached ? sm[i] : sort_key(v, rel, p_off);
+        const uint32_t kv = sort_key(v, rel, (int)p_off);
         uint32_t r = 0;
-        if (cached) {
-            // rank = number of smaller keys, four per shared load
-            for (uint32_t j = 0; j < n4; ++j) {
-                const uint4 u = reinterpret_cast<const uint4*>(sm)[j];
-                r += (u.x < kv ? 1u : 0u) + (u.y < kv ? 1u : 0u) + (u.z < kv ? 1u : 0u) + (u.w < kv ? 1u : 0u);
-            }
-        } else {
-            for (uint32_t j = 0; j < n; ++j) r += (sort_key(perm_u[s0 + j], rel, p_off) < kv) ? 1u : 0u;
-        }
+        for (uint32_t j = 0; j < n; ++j) r += (sort_key(perm_u[s0 + j], rel, (int)p_off) < kv) ? 1u : 0u;
         perm[s0 + r] = v;
         srec[s0 + r] = trec[v];
         srel[s0 + r] = rel[v];
@@ -2052,7 +2083,8 @@ cudaError_t launch_sort(const LaunchArgs& a, cudaStream_t st) {
     k_scan<<<1, 1024, 0, st>>>(a.tile_count, a.tile_start, a.n_tiles);
     if (a.n_chunks) k_scatter<<<a.n_chunks, 256, 0, st>>>(a.chunks, a.sys, a.key, a.tile_start, a.tile_count, a.perm_u);
     if (a.n_tiles)
-        k_tile_sort<<<a.n_tiles, 128, 0, st>>>(a.tile_start, a.perm_u, a.perm, a.trec, a.rel, a.srec, a.srel,
+        // a CTA sized to its tile: full tiles (coarse meshes, dense systems) take 512 threads
+        k_tile_sort<<<a.n_tiles, a.n_chunks * 256LL > 192LL * a.n_tiles ? 512 : 128, 0, st>>>(a.tile_start, a.perm_u, a.perm, a.trec, a.rel, a.srec, a.srel,
                                                a.tile_sys, a.sys);
     return cudaGetLastError();
 }
