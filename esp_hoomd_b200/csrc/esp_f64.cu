@@ -882,7 +882,7 @@ cudaError_t launch64_eval(const Launch64& b, cudaStream_t st) {
         k64_bin<<<a.n_chunks, 256, 0, st>>>(a.chunks, a.sys, a.P, a.T, b.pos_in, b.q_in, b.posq, b.trec, a.rel,
                                             a.key, a.tile_count, a.acc);
     if (lr) {
-        cudaError_t e = launch_scan(a.tile_count, a.tile_start, a.n_tiles, st);
+        cudaError_t e = launch_scan(a.tile_count, a.tile_start, a.n_tiles, a.scan_ws, st);
         if (e != cudaSuccess) return e;
         e = launch_scatter(a.chunks, a.n_chunks, a.sys, a.key, a.tile_start, a.tile_count, a.perm_u, st);
         if (e != cudaSuccess) return e;

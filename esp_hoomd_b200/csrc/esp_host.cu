@@ -266,7 +266,7 @@ struct esp_batch {
     ParamSet* d_pset = nullptr;
     int2 *d_chunks = nullptr, *d_pchunks = nullptr;
     int* d_tile_sys = nullptr;
-    uint32_t *d_tcount = nullptr, *d_tstart = nullptr;
+    uint32_t *d_tcount = nullptr, *d_tstart = nullptr, *d_scan = nullptr;
     float4 *d_posq = nullptr, *d_trec = nullptr, *d_srec = nullptr;
     uint32_t *d_rel = nullptr, *d_key = nullptr, *d_perm_u = nullptr, *d_perm = nullptr, *d_srel = nullptr;
     double* d_rho = nullptr;
@@ -287,12 +287,13 @@ struct esp_batch {
     struct CellGrid {
         DevAlloc mem;
         double rlist = -1;
+        bool half = false;          // cells of rlist / 2 (nlist_half_cells)
         int n_cells = 0, cap = -1;  // cap: row capacity the rows' offsets (nl_off) were laid out for
         std::vector<CellDev> h_cells;
         CellDev* d_cells = nullptr;
         int* d_cell_sys = nullptr;
         uint32_t *d_ckey = nullptr, *d_ccount = nullptr, *d_cstart = nullptr, *d_cperm = nullptr,
-                 *d_slot2idx = nullptr, *d_idx2slot = nullptr;
+                 *d_slot2idx = nullptr, *d_idx2slot = nullptr, *d_scan = nullptr;
         float4 *d_wpos = nullptr, *d_cpos = nullptr;
         int* d_overflow = nullptr;  // [flag, largest row] of the last build
     } cg_nl, cg_pl;
@@ -667,7 +668,7 @@ int esp_batch::plan(const esp_params& p, int ns, const int* N_, const double* bo
     int rc = 0;
     if ((rc = mem.get(d_sys, ns)) || (rc = mem.get(d_pset, psd.size())) || (rc = mem.get(d_chunks, chunks.size())) ||
         (rc = mem.get(d_pchunks, pchunks.size())) || (rc = mem.get(d_tile_sys, n_tiles)) ||
-        (rc = mem.get(d_tcount, n_tiles)) || (rc = mem.get(d_tstart, n_tiles + 1)) || (rc = mem.get(d_posq, totN)) ||
+        (rc = mem.get(d_tcount, n_tiles)) || (rc = mem.get(d_scan, scan_ws_size(n_tiles))) || (rc = mem.get(d_tstart, n_tiles + 1)) || (rc = mem.get(d_posq, totN)) ||
         (rc = mem.get(d_trec, totN)) || (rc = mem.get(d_srec, totN)) || (rc = mem.get(d_rel, totN)) ||
         (rc = mem.get(d_key, totN)) || (rc = mem.get(d_perm_u, totN)) || (rc = mem.get(d_perm, totN)) ||
         (rc = mem.get(d_srel, totN)) || (rc = mem.get(d_rho, m_off)) || (rc = mem.get(d_phi, mp_off)) ||
@@ -891,6 +892,7 @@ LaunchArgs esp_batch::args() const {
     a.n_tiles = n_tiles;
     a.tile_count = d_tcount;
     a.tile_start = d_tstart;
+    a.scan_ws = d_scan;
     a.posq = d_posq;
     a.trec = d_trec;
     a.rel = d_rel;
@@ -1180,13 +1182,22 @@ int esp_batch::setup_cells(CellGrid& g, double rlist, int cap) {
     std::vector<int> cell_sys;
     int c_off = 0;
     long long nl_off = 0;
+    double full = 0;  // cells of edge rlist over all systems
+    for (int s = 0; s < nsys; ++s)
+        full += std::max(1.0, std::floor(box[3 * s] / rlist)) * std::max(1.0, std::floor(box[3 * s + 1] / rlist)) *
+                std::max(1.0, std::floor(box[3 * s + 2] / rlist));
+    g.half = nlist_half_cells(totN, full);
     for (int s = 0; s < nsys; ++s) {
         CellDev& C = g.h_cells[s];
         int nc[3];
         for (int d = 0; d < 3; ++d) {
             if (2.0 * rlist > box[3 * s + d]) return fail(ESP_ERR_INVALID, "rlist must not exceed half the box");
-            nc[d] = std::max(1, (int)std::floor(box[3 * s + d] / rlist));
+            nc[d] = std::max(1, (int)std::floor((g.half ? 2.0 : 1.0) * box[3 * s + d] / rlist));
         }
+        // sparse systems take larger cells: at most 16 per particle
+        const double room = (16.0 * N[s] + 4096.0) / ((double)nc[0] * nc[1] * nc[2]);
+        if (room < 1.0)
+            for (int d = 0; d < 3; ++d) nc[d] = std::max(std::min(nc[d], 5), (int)(nc[d] * std::cbrt(room)));
         C.ncx = nc[0];
         C.ncy = nc[1];
         C.ncz = nc[2];
@@ -1195,15 +1206,18 @@ int esp_batch::setup_cells(CellGrid& g, double rlist, int cap) {
         C.inv_wz = (float)(nc[2] / box[3 * s + 2]);
         C.c_off = c_off;
         C.nl_off = nl_off;
-        for (int c = 0; c < nc[0] * nc[1] * nc[2]; ++c) cell_sys.push_back(s);
-        c_off += nc[0] * nc[1] * nc[2];
+        const long long ncell = (long long)nc[0] * nc[1] * nc[2];
+        if (c_off + ncell >= (1LL << 31)) return fail(ESP_ERR_UNSUPPORTED, "2^31 neighbour-list cells or more");
+        cell_sys.insert(cell_sys.end(), (size_t)ncell, s);
+        c_off += (int)ncell;
         nl_off += (long long)N[s] * cap;
     }
     g.n_cells = c_off;
     int rc = 0;
     if ((rc = g.mem.get(g.d_cells, nsys)) || (rc = g.mem.get(g.d_cell_sys, g.n_cells)) ||
         (rc = g.mem.get(g.d_ckey, totN)) || (rc = g.mem.get(g.d_ccount, g.n_cells)) ||
-        (rc = g.mem.get(g.d_cstart, g.n_cells + 1)) || (rc = g.mem.get(g.d_cperm, totN)) ||
+        (rc = g.mem.get(g.d_cstart, g.n_cells + 1)) || (rc = g.mem.get(g.d_scan, scan_ws_size(g.n_cells))) ||
+        (rc = g.mem.get(g.d_cperm, totN)) ||
         (rc = g.mem.get(g.d_slot2idx, totN)) || (rc = g.mem.get(g.d_idx2slot, totN)) ||
         (rc = g.mem.get(g.d_wpos, totN)) ||
         (rc = g.mem.get(g.d_cpos, totN)) || (rc = g.mem.get(g.d_overflow, 2)))
@@ -1224,11 +1238,13 @@ NlistArgs esp_batch::nlist_args(CellGrid& g, const float* pos4, double rlist, in
     a.cells = g.d_cells;
     a.cell_sys = g.d_cell_sys;
     a.n_cells = g.n_cells;
+    a.half = g.half;
     a.total = totN;
     a.pos = reinterpret_cast<const float4*>(pos4);
     a.ckey = g.d_ckey;
     a.ccount = g.d_ccount;
     a.cstart = g.d_cstart;
+    a.scan_ws = g.d_scan;
     a.perm_u = g.d_cperm;
     a.slot2idx = g.d_slot2idx;
     a.idx2slot = g.d_idx2slot;
@@ -1298,6 +1314,7 @@ int esp_batch::build_pairlist(cudaStream_t st, const float* pos4, double rlist, 
     if (!pos4) return fail(ESP_ERR_INVALID, "null position pointer");
     if (f64) return fail(ESP_ERR_UNSUPPORTED, "the library's pair list serves the FP32 path");
     if ((double)totN * cap >= 4294967296.0) return fail(ESP_ERR_UNSUPPORTED, "pair list of 2^32 entries or more");
+    if (rlist != cg_pl.rlist) drop_graphs();  // captured steps hold the previous cell grid's slot maps
     int rc = setup_cells(cg_pl, rlist, cap);
     if (rc) return rc;
     if (pl_cap != cap) {

@@ -15,15 +15,12 @@
 //       the reference, src/ESPForceCompute.cc:225-232)
 //   k_interp (one CTA per tile), k_interp_q (persistent, tile queue) : force
 //       interpolation, src/ESPForceComputeGPU.cu:292-373 (K6)
-//   k_pair     : EvaluatorPairPSWF over a neighbour list,
-//       src/EvaluatorPairPSWF.h:274-295 with the HOOMD PotentialPair loop
 //   k_exclusions : exclusion correction, src/ESPForceComputeGPU.cu:391-471 (K7)
 //   k_influence: influence-function build (K1), src/ESPForceComputeGPU.cu:157-201
 #include <cuda.h>
 
 #include "esp_common.cuh"
 #include "esp_kernels.h"
-#include "esp_pair.cuh"
 
 namespace espb {
 
@@ -162,6 +159,95 @@ __global__ void __launch_bounds__(1024) k_scan(const uint32_t* __restrict__ cnt,
         carry += total;
     }
     if (threadIdx.x == 0) start[n] = carry;
+}
+
+// Long scans over many CTAs, SCAN_BLK counts each: the CTAs' sums, then each
+// CTA adds the sums before its own and scans its counts.
+constexpr int SCAN_BLK = 256 * SCAN_PER;
+
+__device__ __forceinline__ uint32_t scan_load(const uint32_t* __restrict__ cnt, int i0, int n, bool vec,
+                                              uint32_t (&v)[SCAN_PER]) {
+    if (vec && i0 + SCAN_PER <= n) {
+#pragma unroll
+        for (int k = 0; k < SCAN_PER / 4; ++k) {
+            const uint4 u = reinterpret_cast<const uint4*>(cnt + i0)[k];
+            v[4 * k] = u.x;
+            v[4 * k + 1] = u.y;
+            v[4 * k + 2] = u.z;
+            v[4 * k + 3] = u.w;
+        }
+    } else {
+#pragma unroll
+        for (int k = 0; k < SCAN_PER; ++k) v[k] = i0 + k < n ? cnt[i0 + k] : 0u;
+    }
+    uint32_t t = 0;
+#pragma unroll
+    for (int k = 0; k < SCAN_PER; ++k) t += v[k];
+    return t;
+}
+
+__global__ void __launch_bounds__(256) k_scan_sums(const uint32_t* __restrict__ cnt, uint32_t* __restrict__ ws, int n) {
+    __shared__ uint32_t wsum[8];
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    uint32_t v[SCAN_PER];
+    uint32_t t = scan_load(cnt, blockIdx.x * SCAN_BLK + threadIdx.x * SCAN_PER, n,
+                           (reinterpret_cast<uintptr_t>(cnt) & 15u) == 0, v);
+    t = __reduce_add_sync(0xffffffffu, t);
+    if (lane == 0) wsum[wid] = t;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        uint32_t x = 0;
+#pragma unroll
+        for (int w = 0; w < 8; ++w) x += wsum[w];
+        ws[blockIdx.x] = x;
+    }
+}
+
+__global__ void __launch_bounds__(256)
+    k_scan_apply(const uint32_t* __restrict__ cnt, const uint32_t* __restrict__ ws, uint32_t* __restrict__ start, int n) {
+    __shared__ uint32_t wsum[8], wpre[8];
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    uint32_t pre = 0;
+    for (int b = threadIdx.x; b < (int)blockIdx.x; b += 256) pre += ws[b];
+    pre = __reduce_add_sync(0xffffffffu, pre);
+    const int i0 = blockIdx.x * SCAN_BLK + threadIdx.x * SCAN_PER;
+    uint32_t v[SCAN_PER];
+    const bool vec = ((reinterpret_cast<uintptr_t>(cnt) | reinterpret_cast<uintptr_t>(start)) & 15u) == 0;
+    const uint32_t tsum = scan_load(cnt, i0, n, vec, v);
+    uint32_t x = tsum;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
+        if (lane >= o) x += y;
+    }
+    if (lane == 31) {
+        wsum[wid] = x;
+        wpre[wid] = pre;
+    }
+    __syncthreads();
+    uint32_t run = x - tsum;
+#pragma unroll
+    for (int w = 0; w < 8; ++w) run += wpre[w] + (w < wid ? wsum[w] : 0u);
+    if (vec && i0 + SCAN_PER <= n) {
+#pragma unroll
+        for (int k = 0; k < SCAN_PER / 4; ++k) {
+            uint4 o;
+            o.x = run;
+            o.y = o.x + v[4 * k];
+            o.z = o.y + v[4 * k + 1];
+            o.w = o.z + v[4 * k + 2];
+            run = o.w + v[4 * k + 3];
+            reinterpret_cast<uint4*>(start + i0)[k] = o;
+        }
+    } else {
+#pragma unroll
+        for (int k = 0; k < SCAN_PER; ++k) {
+            if (i0 + k < n) start[i0 + k] = run;
+            run += v[k];
+        }
+    }
+    // the thread past the last count holds the total
+    if (blockIdx.x == gridDim.x - 1 && threadIdx.x == 255) start[n] = run;
 }
 
 // Slot of each particle inside its tile; leaves tile_count at zero so the
@@ -1750,141 +1836,6 @@ __global__ void __launch_bounds__(128, 5)
     asm volatile("cp.async.wait_group 0;\n" ::);
 }
 
-// ============================================================================
-// a8: short-range pair term over a HOOMD-layout neighbour list
-// (neighbours of i: nlist[head[i] + k], k < n_neigh[i], local indices).
-// TPP lanes cooperate on one particle; per pair
-//   pair_eng = qiqj/(4 pi) (1/r - Q(u)/r_c),  u = r^2/r_c^2
-//   force_divr = qiqj/(4 pi) (1/r^3 + 2 Q'(u)/r_c^3)
-// (the split form of EvaluatorPairPSWF::evalForceAndEnergy).
-// ============================================================================
-// EN: pair energies (per particle and per system); without them the split
-// polynomial Q itself is not needed, only Q', and the kernel (40 registers)
-// keeps 6 CTAs per SM resident so that more position gathers are in flight.
-// Each lane loads its next 16-byte row segment of neighbour indices one
-// iteration ahead of the gathers that use it.
-template <int TPP, int NQ, bool VIR, bool EN>
-__global__ void __launch_bounds__(256, EN ? 5 : 6)
-    k_pair(const int2* __restrict__ chunks, const SysDev* __restrict__ sys, const ParamSet* __restrict__ psets,
-           const float4* __restrict__ posq, const uint32_t* __restrict__ head, const uint32_t* __restrict__ nn,
-           const uint32_t* __restrict__ nlist, float4* __restrict__ force, double* __restrict__ acc, int accumulate,
-           const PairCoef pc, float* __restrict__ vpp, int vpitch, const uint32_t* __restrict__ outidx) {
-    __shared__ double red[32 * 7];
-    const int2 ch = chunks[blockIdx.x];
-    const SysDev S = sys[ch.x];
-    const ParamSet& ps = psets[S.pset];
-    PairEval<NQ, VIR, EN> ev{pc};
-    ev.rc2 = ps.rcut2;
-    ev.irc = ps.inv_rcut;
-    ev.irc2 = ps.inv_rcut * ps.inv_rcut;
-    ev.tirc3 = ps.two_inv_rcut3;
-    ev.Lx = S.Lx;
-    ev.Ly = S.Ly;
-    ev.Lz = S.Lz;
-    ev.iLx = S.inv_Lx;
-    ev.iLy = S.inv_Ly;
-    ev.iLz = S.inv_Lz;
-    const int i = ch.y + threadIdx.x / TPP;
-    const int sub = threadIdx.x % TPP;
-    const bool valid = i < S.p_off + S.N;
-    // particles at least r_c from every face (positions are wrapped into
-    // the box) see every in-cutoff neighbour in the same image; a warp whose
-    // particles all are skips the minimum-image wrap (out-of-cutoff pairs
-    // are masked whatever their displacement)
-    bool inner = true;
-    if (valid) {
-        const float4 p = posq[i];
-        const float rc = ps.rcut;
-        inner = p.x >= rc && p.x <= S.Lx - rc && p.y >= rc && p.y <= S.Ly - rc && p.z >= rc && p.z <= S.Lz - rc;
-    }
-    const bool interior = __all_sync(0xffffffffu, inner);
-    if (valid) {
-        const float4 pi = posq[i];
-        const uint32_t n = nn[i], h = head[i];
-        const int po = S.p_off;
-        uint32_t k0 = 0;
-        if ((h & 3u) == 0u) {
-            // 16-byte row segments: each lane streams 4 neighbour indices
-            const uint4* row = reinterpret_cast<const uint4*>(nlist + h);
-            const uint32_t n4 = n >> 2;
-            if (interior) {
-                uint4 jn = sub < n4 ? __ldg(&row[sub]) : make_uint4(0u, 0u, 0u, 0u);
-                for (uint32_t k4 = sub; k4 < n4; k4 += TPP) {
-                    const uint4 jj = jn;  // this row segment; the next one is loaded ahead
-                    if (k4 + TPP < n4) jn = __ldg(&row[k4 + TPP]);
-                    const float4 p0 = __ldg(&posq[po + (int)jj.x]);
-                    const float4 p1 = __ldg(&posq[po + (int)jj.y]);
-                    const float4 p2 = __ldg(&posq[po + (int)jj.z]);
-                    const float4 p3 = __ldg(&posq[po + (int)jj.w]);
-                    ev.template pair<false>(pi, p0);
-                    ev.template pair<false>(pi, p1);
-                    ev.template pair<false>(pi, p2);
-                    ev.template pair<false>(pi, p3);
-                }
-            } else {
-                uint4 jn = sub < n4 ? __ldg(&row[sub]) : make_uint4(0u, 0u, 0u, 0u);
-                for (uint32_t k4 = sub; k4 < n4; k4 += TPP) {
-                    const uint4 jj = jn;
-                    if (k4 + TPP < n4) jn = __ldg(&row[k4 + TPP]);
-                    const float4 p0 = __ldg(&posq[po + (int)jj.x]);
-                    const float4 p1 = __ldg(&posq[po + (int)jj.y]);
-                    const float4 p2 = __ldg(&posq[po + (int)jj.z]);
-                    const float4 p3 = __ldg(&posq[po + (int)jj.w]);
-                    ev.pair(pi, p0);
-                    ev.pair(pi, p1);
-                    ev.pair(pi, p2);
-                    ev.pair(pi, p3);
-                }
-            }
-            k0 = n4 << 2;
-        }
-        for (uint32_t k = k0 + sub; k < n; k += TPP) ev.pair(pi, __ldg(&posq[po + (int)__ldg(&nlist[h + k])]));
-    }
-    float fx = ev.fx, fy = ev.fy, fz = ev.fz, en = ev.en;
-#pragma unroll
-    for (int o = TPP / 2; o > 0; o >>= 1) {
-        fx += __shfl_xor_sync(0xffffffffu, fx, o);
-        fy += __shfl_xor_sync(0xffffffffu, fy, o);
-        fz += __shfl_xor_sync(0xffffffffu, fz, o);
-        en += __shfl_xor_sync(0xffffffffu, en, o);
-    }
-    // rows by slot (the library's pair list): results go to the particle of the slot
-    const int oi = (outidx && valid) ? (int)outidx[i] : i;
-    if (valid && sub == 0) {
-        float4 f = accumulate ? force[oi] : make_float4(0.f, 0.f, 0.f, 0.f);
-        f.x += fx;
-        f.y += fy;
-        f.z += fz;
-        f.w += 0.5f * en;
-        force[oi] = f;
-    }
-    if (VIR && vpp) {
-        // this particle's half of its pairs' virial (HOOMD's per-particle virial)
-        float v[6] = {ev.vxx, ev.vxy, ev.vxz, ev.vyy, ev.vyz, ev.vzz};
-#pragma unroll
-        for (int o = TPP / 2; o > 0; o >>= 1)
-#pragma unroll
-            for (int k = 0; k < 6; ++k) v[k] += __shfl_xor_sync(0xffffffffu, v[k], o);
-        if (valid && sub == 0)
-#pragma unroll
-            for (int k = 0; k < 6; ++k) vpp[(size_t)k * vpitch + oi] += 0.5f * v[k];
-    }
-    if (VIR) {
-        double e[7] = {sub == 0 ? 0.5 * (double)en : 0.0, 0.5 * (double)ev.vxx, 0.5 * (double)ev.vxy,
-                       0.5 * (double)ev.vxz, 0.5 * (double)ev.vyy, 0.5 * (double)ev.vyz, 0.5 * (double)ev.vzz};
-        block_sum_f64<7>(e, red);
-        if (threadIdx.x == 0) {
-            atomicAdd(&acc[ch.x * ACC_STRIDE + ACC_E], e[0]);
-#pragma unroll
-            for (int k = 0; k < 6; ++k) atomicAdd(&acc[ch.x * ACC_STRIDE + ACC_WP + k], e[1 + k]);
-        }
-    } else if (EN) {
-        double e[1] = {sub == 0 ? 0.5 * (double)en : 0.0};
-        block_sum_f64<1>(e, red);
-        if (threadIdx.x == 0) atomicAdd(&acc[ch.x * ACC_STRIDE + ACC_E], e[0]);
-    }
-}
-
 // Energy and virial per system: E = sum_i e_i + E_bg; W = W_k + W_pair + E_bg I.
 // external (may be NULL): the terms no particle owns, {E_bg, W_k + E_bg I}.
 __global__ void k_finalize(const SysDev* __restrict__ sys, const ParamSet* __restrict__ psets, int nsys,
@@ -2060,8 +2011,17 @@ static cudaError_t launch_interp_p(const LaunchArgs& a, cudaStream_t st) {
     return cudaGetLastError();
 }
 
-cudaError_t launch_scan(const uint32_t* cnt, uint32_t* start, int n, cudaStream_t st) {
-    k_scan<<<1, 1024, 0, st>>>(cnt, start, n);
+// One CTA scans up to SCAN_ONE_CTA counts in one round; above, its rounds are
+// serial (the 256-lattice batch's tiles: 21.6 us) and two short kernels over
+// all CTAs take over (8.8 us).
+cudaError_t launch_scan(const uint32_t* cnt, uint32_t* start, int n, uint32_t* ws, cudaStream_t st) {
+    if (ws && n > SCAN_ONE_CTA) {
+        const int nb = (int)scan_ws_size(n);
+        k_scan_sums<<<nb, 256, 0, st>>>(cnt, ws, n);
+        k_scan_apply<<<nb, 256, 0, st>>>(cnt, ws, start, n);
+    } else {
+        k_scan<<<1, 1024, 0, st>>>(cnt, start, n);
+    }
     return cudaGetLastError();
 }
 
@@ -2080,7 +2040,8 @@ cudaError_t launch_bin(const LaunchArgs& a, cudaStream_t st) {
 }
 
 cudaError_t launch_sort(const LaunchArgs& a, cudaStream_t st) {
-    k_scan<<<1, 1024, 0, st>>>(a.tile_count, a.tile_start, a.n_tiles);
+    const cudaError_t e = launch_scan(a.tile_count, a.tile_start, a.n_tiles, a.scan_ws, st);
+    if (e != cudaSuccess) return e;
     if (a.n_chunks) k_scatter<<<a.n_chunks, 256, 0, st>>>(a.chunks, a.sys, a.key, a.tile_start, a.tile_count, a.perm_u);
     if (a.n_tiles)
         // a CTA sized to its tile: full tiles (coarse meshes, dense systems) take 512 threads
@@ -2136,62 +2097,6 @@ cudaError_t launch_fft(const LaunchArgs& a, cudaStream_t st) {
     if (a.n_xitems) k_fftx_inv<<<a.n_xitems, 256, smx, st>>>(a.xitems, a.sys, a.tw, a.spec, a.phi, a.rho);
     if (a.n_pitems) k_fft_plane_inv<<<a.n_pitems, 256, a.smem_plane, st>>>(a.pitems, a.sys, a.tw, a.spec, a.phi, a.rho);
     return cudaGetLastError();
-}
-
-template <int TPP, bool VIR, bool EN>
-static cudaError_t launch_pair_t(const LaunchArgs& a, cudaStream_t st) {
-    // the library's pair list: rows by slot over the slot-ordered positions
-    const PairList* pl = a.plist;
-    const float4* posq = pl ? pl->spos : a.posq;
-    const uint32_t* head = pl ? pl->head : a.nl_head;
-    const uint32_t* nn = pl ? pl->nn : a.nl_n;
-    const uint32_t* nl = pl ? pl->nl : a.nl_list;
-    const uint32_t* outidx = pl ? pl->slot2idx : nullptr;
-#define ESPB_PAIR(NQ)                                                                                          \
-    k_pair<TPP, NQ, VIR, EN><<<a.n_pchunks, 256, 0, st>>>(a.pchunks, a.sys, a.psets, posq, head, nn, nl, a.force, \
-                                                          a.acc, a.accumulate, a.pc, a.virial_pp, a.vpp_pitch,    \
-                                                          outidx)
-    if (a.nq <= 8) ESPB_PAIR(8);
-    else if (a.nq <= 10) ESPB_PAIR(10);
-    else if (a.nq <= 11) ESPB_PAIR(11);
-    else if (a.nq <= 12) ESPB_PAIR(12);
-    else if (a.nq <= 13) ESPB_PAIR(13);
-    else if (a.nq <= 14) ESPB_PAIR(14);
-    else if (a.nq <= 16) ESPB_PAIR(16);
-    else if (a.nq <= 20) ESPB_PAIR(20);
-    else if (a.nq <= 24) ESPB_PAIR(24);
-    else ESPB_PAIR(32);
-#undef ESPB_PAIR
-    return cudaGetLastError();
-}
-
-cudaError_t launch_pair(const LaunchArgs& a, cudaStream_t st) {
-    if (a.n_pchunks == 0) return cudaSuccess;
-    if (a.want_virial) {
-        switch (a.tpp) {
-            case 4: return launch_pair_t<4, true, true>(a, st);
-            case 8: return launch_pair_t<8, true, true>(a, st);
-            case 16: return launch_pair_t<16, true, true>(a, st);
-            case 32: return launch_pair_t<32, true, true>(a, st);
-            default: return cudaErrorInvalidValue;
-        }
-    }
-    if (a.want_energy) {
-        switch (a.tpp) {
-            case 4: return launch_pair_t<4, false, true>(a, st);
-            case 8: return launch_pair_t<8, false, true>(a, st);
-            case 16: return launch_pair_t<16, false, true>(a, st);
-            case 32: return launch_pair_t<32, false, true>(a, st);
-            default: return cudaErrorInvalidValue;
-        }
-    }
-    switch (a.tpp) {
-        case 4: return launch_pair_t<4, false, false>(a, st);
-        case 8: return launch_pair_t<8, false, false>(a, st);
-        case 16: return launch_pair_t<16, false, false>(a, st);
-        case 32: return launch_pair_t<32, false, false>(a, st);
-        default: return cudaErrorInvalidValue;
-    }
 }
 
 // ============================================================================

@@ -60,6 +60,7 @@ struct LaunchArgs {
     int n_tiles = 0;
     uint32_t* tile_count = nullptr;
     uint32_t* tile_start = nullptr;
+    uint32_t* scan_ws = nullptr;  // scan workspace of the tile counts (scan_ws_size)
     const float4* pos_in = nullptr;
     const float* q_in = nullptr;
     float4* posq = nullptr;
@@ -121,7 +122,11 @@ struct LaunchArgs {
     int ex_pitch = 0;
 };
 
-cudaError_t launch_scan(const uint32_t* cnt, uint32_t* start, int n, cudaStream_t st);
+// Exclusive scan of n counts into start[0..n]; ws: scan_ws_size(n) words of the
+// caller's for scans above SCAN_ONE_CTA counts (NULL: one CTA whatever n).
+constexpr int SCAN_ONE_CTA = 1024 * 16;
+inline size_t scan_ws_size(long long n) { return (size_t)((n + 4095) / 4096); }
+cudaError_t launch_scan(const uint32_t* cnt, uint32_t* start, int n, uint32_t* ws, cudaStream_t st);
 cudaError_t launch_scatter(const int2* chunks, int n_chunks, const SysDev* sys, const uint32_t* key,
                            const uint32_t* start, uint32_t* cnt, uint32_t* perm_u, cudaStream_t st);
 cudaError_t launch_bin(const LaunchArgs& a, cudaStream_t st);

@@ -2,6 +2,8 @@
 // These stand in for the HOOMD-blue pieces the reference relies on
 // (NeighborList and the integrator; not vendored in the reference) so the
 // ESP path can run standalone.
+#include <algorithm>
+
 #include "esp_cells.cuh"
 #include "esp_common.cuh"
 #include "esp_kernels.h"
@@ -9,7 +11,7 @@
 
 namespace espb {
 
-// Cell of each particle (cells of edge >= rlist, at least 3 per axis).
+// Cell of each particle.
 __global__ void k_cell_bin(const int2* __restrict__ chunks, const SysDev* __restrict__ sys,
                            const CellDev* __restrict__ cells, const float4* __restrict__ pos,
                            uint32_t* __restrict__ ckey, uint32_t* __restrict__ ccount, float4* __restrict__ wpos) {
@@ -40,39 +42,24 @@ __global__ void k_cell_bin(const int2* __restrict__ chunks, const SysDev* __rest
 }
 
 // Deterministic order inside each cell (ascending particle index) and the
-// cell-sorted positions.
-__global__ void k_cell_sort(const uint32_t* __restrict__ start, const uint32_t* __restrict__ perm_u,
-                            const float4* __restrict__ wpos, float4* __restrict__ cpos,
-                            uint32_t* __restrict__ slot2idx, uint32_t* __restrict__ idx2slot) {
-    __shared__ __align__(16) uint32_t sm[1024];
-    const uint32_t s0 = start[blockIdx.x];
-    const uint32_t n = start[blockIdx.x + 1] - s0;
-    if (n == 0) return;
-    const bool cached = n <= 1024u;
-    const uint32_t n4 = (n + 3u) >> 2;
-    if (cached) {
-        for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) sm[i] = perm_u[s0 + i];
-        // pad to whole 16-byte groups with a value no index is above
-        if (threadIdx.x < 4u * n4 - n) sm[n + threadIdx.x] = 0xffffffffu;
-    }
-    __syncthreads();
-    const uint32_t* src = cached ? sm : perm_u + s0;
-    for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) {
-        const uint32_t v = src[i];
-        uint32_t r = 0;
-        if (cached) {
-            // rank = number of smaller indices, four per shared load
-            for (uint32_t j = 0; j < n4; ++j) {
-                const uint4 u = reinterpret_cast<const uint4*>(sm)[j];
-                r += (u.x < v ? 1u : 0u) + (u.y < v ? 1u : 0u) + (u.z < v ? 1u : 0u) + (u.w < v ? 1u : 0u);
-            }
-        } else {
-            for (uint32_t j = 0; j < n; ++j) r += (src[j] < v) ? 1u : 0u;
-        }
-        cpos[s0 + r] = wpos[v];
-        if (slot2idx) slot2idx[s0 + r] = v;
-        if (idx2slot) idx2slot[v] = s0 + r;
-    }
+// cell-sorted positions. One thread per unsorted slot ranks its particle
+// among its cell's (about 5 at density 1 and rlist 3.4): the cell's indices
+// are neighbours in perm_u, so the loop reads the L1.
+__global__ void __launch_bounds__(256)
+    k_cell_sort(int total, const uint32_t* __restrict__ ckey, const uint32_t* __restrict__ start,
+                const uint32_t* __restrict__ perm_u, const float4* __restrict__ wpos, float4* __restrict__ cpos,
+                uint32_t* __restrict__ slot2idx, uint32_t* __restrict__ idx2slot) {
+    const int t = blockIdx.x * 256 + threadIdx.x;
+    if (t >= total) return;
+    const uint32_t v = perm_u[t];
+    const uint32_t c = ckey[v];
+    const float4 p = wpos[v];
+    const uint32_t b = start[c], e = start[c + 1];
+    uint32_t r = b;
+    for (uint32_t j = b; j < e; ++j) r += perm_u[j] < v ? 1u : 0u;
+    cpos[r] = p;
+    if (slot2idx) slot2idx[r] = v;
+    if (idx2slot) idx2slot[v] = r;
 }
 
 // One CTA per cell, one thread per particle of the cell (passes of
@@ -132,8 +119,8 @@ __device__ __forceinline__ uint32_t nl_scan(const float4* __restrict__ cand, int
 // nn by slot), entries local slots. Rows longer than cap keep their first cap
 // entries and set the overflow flag; overflow[1] receives the longest row.
 template <bool SORTED>
-__global__ void __launch_bounds__(NL_THREADS) k_nlist(const int* __restrict__ cell_sys, const SysDev* __restrict__ sys,
-                                                      const CellDev* __restrict__ cells,
+__global__ void __launch_bounds__(NL_THREADS) k_nlist_cta(const int* __restrict__ cell_sys, const SysDev* __restrict__ sys,
+                                                          const CellDev* __restrict__ cells,
                                                       const uint32_t* __restrict__ cstart,
                                                       const float4* __restrict__ cpos, float rlist2, int cap,
                                                       uint32_t* __restrict__ head, uint32_t* __restrict__ nn,
@@ -196,7 +183,7 @@ __global__ void __launch_bounds__(NL_THREADS) k_nlist(const int* __restrict__ ce
         }
         if (active) {
             head[key] = (uint32_t)hrow;
-            nn[key] = cnt;
+            nn[key] = SORTED ? min(cnt, (uint32_t)cap) : cnt;
             if (cnt > (uint32_t)cap) {
                 atomicOr(overflow, 1);
                 atomicMax(overflow + 1, (int)cnt);
@@ -205,36 +192,254 @@ __global__ void __launch_bounds__(NL_THREADS) k_nlist(const int* __restrict__ ce
     }
 }
 
-// Leaves the excluded partners out of the rows just built (HOOMD's lists
-// hold no excluded pairs): one thread per row with exclusions, in place, the
-// kept entries in their order; the count drops by the entries removed from
-// the stored part. Pair-list rows hold slots, so the excluded indices are
-// mapped to slots first.
-constexpr int NL_MAXEX = 8;  // exclusions per particle held in registers
+// Neighbour rows. One warp per cell; the cell's particles are taken eight at
+// a time, their positions held by every lane, and the surrounding cells'
+// particles stream past, one candidate per lane: a (dz, dy) row of up to five
+// cells is contiguous in the cell-sorted order (two pieces at a periodic
+// face), the rows' candidates are numbered consecutively so that every segment
+// of 32 is full, and the next segment's positions are in flight. A ballot and
+// a population count place each hit in its row, so a row's entries are written
+// in order, neighbouring lanes side by side. Rows list the (dz, dy, dx) cells
+// in that order and ascending slots inside each: they are deterministic. With
+// at least 5 cells on every axis a surrounding cell is one periodic image and
+// its particles are shifted by it; smaller grids visit every cell of the axis
+// and take the minimum image per pair.
+// Bound by issue slots (72% active; 72 registers for 7 CTAs per SM, 96 and
+// fewer CTAs: 20% slower). Cells of half the list radius leave 15.6 rlist^3 of
+// volume to test instead of the CTA kernel's 27, and the work falls into more
+// and shorter warps (nlist_half_cells has both kernels' times). Packed FP32 pairs in
+// the distance test saved no instruction (register moves) and measured 5%
+// slower.
+constexpr int NL_WARPS = 4;
+constexpr int NL_GROUP = 8;  // particles of the cell tested per pass
+constexpr int NL_MAXEX = 8;  // excluded partners per particle kept in shared memory
 
+struct NlGroup {
+    float px[NL_GROUP], py[NL_GROUP], pz[NL_GROUP];
+    uint32_t pos[NL_GROUP];   // next entry of the row - 1
+    uint32_t end[NL_GROUP];   // end of the row's capacity
+    uint32_t hits[NL_GROUP];  // hits before exclusions (EX only)
+};
+
+// Tests candidate c (one per lane) against the group and appends value v to
+// the rows of the particles within range. SELF: c may be one of the group
+// (slot = c's slot, g0 = the group's first slot). EX: excluded partners'
+// slots in exs, nex per particle.
+template <bool MINIMG, bool SELF, bool EX>
+__device__ __forceinline__ void nl_test(NlGroup& g, int ng, float4 c, uint32_t slot, uint32_t v, uint32_t g0,
+                                        const SysDev& S, float rlist2, uint32_t lemask, uint32_t* __restrict__ nl,
+                                        const uint32_t (*exs)[NL_MAXEX], const uint32_t* nex) {
+#pragma unroll
+    for (int i = 0; i < NL_GROUP; ++i) {
+        if (i >= ng) break;
+        float dx = g.px[i] - c.x, dy = g.py[i] - c.y, dz = g.pz[i] - c.z;
+        if (MINIMG) {
+            dx -= S.Lx * rintf(dx * S.inv_Lx);
+            dy -= S.Ly * rintf(dy * S.inv_Ly);
+            dz -= S.Lz * rintf(dz * S.inv_Lz);
+        }
+        const float d2 = dx * dx + dy * dy + dz * dz;
+        bool in = d2 < rlist2;
+        if (SELF) in = in && slot != g0 + i;
+        if (EX) {
+            g.hits[i] += (uint32_t)__popc(__ballot_sync(0xffffffffu, in));
+            for (uint32_t x = 0; x < nex[i]; ++x) in = in && slot != exs[i][x];
+        }
+        const uint32_t inc = (uint32_t)__popc(__ballot_sync(0xffffffffu, in) & lemask);  // hits up to this lane
+        const uint32_t e = g.pos[i] + inc;
+        if (in && e < g.end[i]) nl[e] = v;
+        g.pos[i] += __shfl_sync(0xffffffffu, inc, 31);
+    }
+}
+
+// SORTED = false: HOOMD-layout rows -- the row of particle i at nl_off +
+// local i * cap, entries local particle indices, head/nn indexed by
+// particle. SORTED = true: the library's pair list -- the same layout indexed
+// by the cell-sorted slot (row of slot s at nl_off + local s * cap, head and
+// nn by slot), entries local slots. Rows longer than cap keep their first cap
+// entries, the overflow flag is set and overflow[1] receives the longest row;
+// nn holds the true count in HOOMD rows and the kept entries in the pair list,
+// which the pair kernel walks. EX: the excluded partners are left out of the
+// rows (a row whose hits exceed cap before that counts as overflowing).
+template <bool SORTED, bool EX>
+__global__ void __launch_bounds__(32 * NL_WARPS, EX ? 4 : 7)
+    k_nlist(const int* __restrict__ cell_sys, int n_cells, const SysDev* __restrict__ sys,
+            const CellDev* __restrict__ cells, const uint32_t* __restrict__ cstart, const float4* __restrict__ cpos,
+            float rlist2, uint32_t cap, uint32_t* __restrict__ head, uint32_t* __restrict__ nn,
+            uint32_t* __restrict__ nl, int* __restrict__ overflow, const uint32_t* __restrict__ ex_n,
+            const uint32_t* __restrict__ ex_list, int ex_pitch, const uint32_t* __restrict__ idx2slot) {
+    __shared__ uint4 srow[NL_WARPS][25];     // (dz, dy) row: its two pieces' slots (see below), first candidate
+    __shared__ float2 sshift[NL_WARPS][25];  // its periodic image along y and z
+    __shared__ uint32_t soff[NL_WARPS][28];  // first candidate of each row, then the total
+    __shared__ uint32_t sex[NL_WARPS][EX ? NL_GROUP : 1][NL_MAXEX], snex[NL_WARPS][NL_GROUP];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const uint32_t cidx = blockIdx.x * NL_WARPS + warp;
+    if (cidx >= (uint32_t)n_cells) return;
+    const uint32_t c0 = cstart[cidx], c1 = cstart[cidx + 1];
+    if (c0 + blockIdx.y * NL_GROUP >= c1) return;
+    const int si = cell_sys[cidx];
+    const SysDev& S = sys[si];
+    const CellDev& C = cells[si];
+    const int p_off = S.p_off;
+    const uint32_t lemask = 0xffffffffu >> (31 - lane);
+    const int ncx = C.ncx, ncy = C.ncy, ncz = C.ncz;
+    const int lc = (int)cidx - C.c_off;
+    const int cx = lc % ncx, cy = (lc / ncx) % ncy, cz = lc / (ncx * ncy);
+    const bool minimg = ncx < 5 || ncy < 5 || ncz < 5;
+    const int nry = min(ncy, 5), nrows = nry * min(ncz, 5);
+    const int rself = (ncy >= 5 ? 2 : cy) + nry * (ncz >= 5 ? 2 : cz);  // the cell's own row
+    // five cells from cx - 2; at a face the part beyond it is the second piece
+    // (its last cells' piece first at the low face)
+    const bool wlo = ncx >= 5 && cx < 2, whi = ncx >= 5 && cx + 2 >= ncx;
+    uint32_t len = 0;
+    uint4 t = make_uint4(0u, 0u, 0u, 0u);
+    if (lane < nrows) {
+        int yy = lane % nry, zz = lane / nry;
+        float shy = 0.f, shz = 0.f;
+        if (ncy >= 5) {
+            yy += cy - 2;
+            if (yy < 0) { yy += ncy; shy = -S.Ly; } else if (yy >= ncy) { yy -= ncy; shy = S.Ly; }
+        }
+        if (ncz >= 5) {
+            zz += cz - 2;
+            if (zz < 0) { zz += ncz; shz = -S.Lz; } else if (zz >= ncz) { zz -= ncz; shz = S.Lz; }
+        }
+        const uint32_t* rowc = cstart + C.c_off + (zz * ncy + yy) * ncx;
+        const int xa = wlo ? cx - 2 + ncx : (ncx >= 5 ? cx - 2 : 0);
+        const int xb = wlo || whi || ncx < 5 ? ncx : cx + 3;
+        t.x = rowc[xa];
+        t.y = rowc[xb] - t.x;
+        len = t.y;
+        if (wlo || whi) {
+            t.z = rowc[0];
+            len += rowc[wlo ? cx + 3 : cx + 3 - ncx] - t.z;
+        }
+        sshift[warp][lane] = minimg ? make_float2(0.f, 0.f) : make_float2(shy, shz);
+    }
+    // the rows' candidates numbered consecutively; candidate g of row r is the
+    // slot (g < y ? x : z) + g of its srow entry (slot offsets less the row's
+    // first candidate)
+    uint32_t inc = len;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xffffffffu, inc, o);
+        if (lane >= o) inc += y;
+    }
+    const uint32_t total = __shfl_sync(0xffffffffu, inc, 31);
+    if (lane < nrows) {
+        const uint32_t o = inc - len;
+        soff[warp][lane + 1] = inc;
+        srow[warp][lane] = make_uint4(t.x - o, t.y + o, t.z - t.y - o, 0u);
+        if (lane == 0) soff[warp][0] = 0u;
+    }
+    __syncwarp();
+    const uint32_t self0 = soff[warp][rself], self1 = soff[warp][rself + 1];
+    const float shx1 = wlo && !minimg ? -S.Lx : 0.f, shx2 = whi && !minimg ? S.Lx : 0.f;
+    // several CTAs share a row of cells (grid y) when the cells hold more than a group
+    for (uint32_t g0 = c0 + blockIdx.y * NL_GROUP; g0 < c1; g0 += gridDim.y * NL_GROUP) {
+        const int ng = (int)min(c1 - g0, (uint32_t)NL_GROUP);
+        NlGroup g;
+        uint32_t mykey = 0, myrow = 0;  // lane k < ng: owner and first entry of the k-th row
+#pragma unroll
+        for (int i = 0; i < NL_GROUP; i += 2) {
+            // a missing second particle has a NaN position, which tests false
+            const float4 a = cpos[min(g0 + i, c1 - 1)], b = cpos[min(g0 + i + 1, c1 - 1)];
+            g.px[i] = a.x, g.py[i] = a.y, g.pz[i] = a.z;
+            g.px[i + 1] = b.x, g.py[i + 1] = b.y, g.pz[i + 1] = b.z;
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const uint32_t key = SORTED ? g0 + i + h : (uint32_t)__float_as_int(h ? b.w : a.w);
+                const uint32_t row = (uint32_t)(C.nl_off + (long long)((int)key - p_off) * (long long)cap);
+                g.pos[i + h] = row - 1u;
+                g.end[i + h] = row + cap;
+                g.hits[i + h] = 0u;
+                if (lane == i + h) {
+                    mykey = key;
+                    myrow = row;
+                }
+            }
+            if (EX) {
+#pragma unroll
+                for (int h = 0; h < 2; ++h)
+                    if (lane == i + h && lane < ng) {
+                        const uint32_t idx = (uint32_t)__float_as_int(h ? b.w : a.w);
+                        const uint32_t ne = min(ex_n[idx], (uint32_t)ex_pitch);
+                        uint32_t m = 0;
+                        for (uint32_t x = 0; x < ne && m < NL_MAXEX; ++x) {
+                            const uint32_t jl = ex_list[(size_t)idx * ex_pitch + x];
+                            if (jl < (uint32_t)S.N) sex[warp][lane][m++] = idx2slot[p_off + (int)jl];
+                        }
+                        snex[warp][lane] = m;
+                    }
+            }
+        }
+        if (EX) {
+            if (lane >= ng && lane < NL_GROUP) snex[warp][lane] = 0u;
+            __syncwarp();
+        }
+        // segments of 32 candidates, the next one's positions in flight
+        int r = 0;  // row of this lane's candidate
+        float4 cn = make_float4(0.f, 0.f, 0.f, 0.f);
+        uint32_t slot_n = 0;
+        auto fetch = [&](uint32_t c) {  // candidate c of this lane (a NaN position past the last)
+            cn = make_float4(__int_as_float(0x7fc00000), 0.f, 0.f, 0.f);
+            if (c < total) {
+                while (c >= soff[warp][r + 1]) ++r;
+                const uint4 w = srow[warp][r];
+                const float2 sh = sshift[warp][r];
+                const bool second = c >= w.y;
+                slot_n = (second ? w.z : w.x) + c;
+                cn = cpos[slot_n];
+                cn.x += second ? shx2 : shx1;
+                cn.y += sh.x;
+                cn.z += sh.y;
+            }
+        };
+        fetch(lane);
+        for (uint32_t b0 = 0; b0 < total; b0 += 32) {
+            const float4 c = cn;
+            const uint32_t slot = slot_n, v = (SORTED ? slot : (uint32_t)__float_as_int(c.w)) - (uint32_t)p_off;
+            if (b0 + 32 < total) fetch(b0 + 32 + lane);
+            if (minimg) nl_test<true, true, EX>(g, ng, c, slot, v, g0, S, rlist2, lemask, nl, sex[warp], snex[warp]);
+            else if (b0 < self1 && b0 + 32 > self0)
+                nl_test<false, true, EX>(g, ng, c, slot, v, g0, S, rlist2, lemask, nl, sex[warp], snex[warp]);
+            else nl_test<false, false, EX>(g, ng, c, slot, v, g0, S, rlist2, lemask, nl, sex[warp], snex[warp]);
+        }
+        uint32_t cnt = 0, hits = 0;
+#pragma unroll
+        for (int i = 0; i < NL_GROUP; ++i)
+            if (lane == i) {
+                cnt = g.pos[i] + 1u - myrow;
+                hits = EX ? g.hits[i] : cnt;
+            }
+        if (lane < ng) {
+            head[mykey] = myrow;
+            nn[mykey] = SORTED ? min(cnt, cap) : cnt;
+            if (hits > cap) {
+                atomicOr(overflow, 1);
+                atomicMax(overflow + 1, (int)hits);
+            }
+        }
+        __syncwarp();
+    }
+}
+
+// Leaves the excluded partners out of the rows of particles with more than
+// `done` exclusions: one thread per row, in place, the kept entries in their
+// order; the count drops by the entries removed from the stored part.
 template <bool SORTED>
 __global__ void k_nlist_exclude(const int2* __restrict__ chunks, const SysDev* __restrict__ sys,
                                 const uint32_t* __restrict__ head, uint32_t* __restrict__ nn,
                                 uint32_t* __restrict__ nl, int cap, const uint32_t* __restrict__ ex_n,
                                 const uint32_t* __restrict__ ex_list, int ex_pitch,
-                                const uint32_t* __restrict__ slot2idx, const uint32_t* __restrict__ idx2slot) {
+                                const uint32_t* __restrict__ slot2idx, const uint32_t* __restrict__ idx2slot, int done) {
     const int2 ch = chunks[blockIdx.x];
     const SysDev& S = sys[ch.x];
     const int key = ch.y + threadIdx.x;  // the row: a slot (pair list) or a particle
     if (key >= S.p_off + S.N) return;
     const int i = SORTED ? (int)slot2idx[key] : key;
     const int ne = min((int)ex_n[i], ex_pitch);
-    if (ne == 0) return;
-    uint32_t ex[NL_MAXEX];
-#pragma unroll
-    for (int k = 0; k < NL_MAXEX; ++k) {
-        uint32_t v = 0xffffffffu;
-        if (k < ne) {
-            const uint32_t jl = ex_list[(size_t)i * ex_pitch + k];
-            v = SORTED ? idx2slot[S.p_off + jl] - (uint32_t)S.p_off : jl;
-        }
-        ex[k] = v;
-    }
+    if (ne <= done) return;
     uint32_t* row = nl + head[key];
     const uint32_t cnt = nn[key];
     const uint32_t n = min(cnt, (uint32_t)cap);
@@ -242,11 +447,9 @@ __global__ void k_nlist_exclude(const int2* __restrict__ chunks, const SysDev* _
     for (uint32_t r = 0; r < n; ++r) {
         const uint32_t v = row[r];
         bool drop = false;
-#pragma unroll
-        for (int k = 0; k < NL_MAXEX; ++k) drop |= v == ex[k];
-        for (int k = NL_MAXEX; k < ne; ++k) {  // rows with more exclusions than registers hold
+        for (int k = 0; k < ne; ++k) {
             const uint32_t jl = ex_list[(size_t)i * ex_pitch + k];
-            drop |= v == (SORTED ? idx2slot[S.p_off + jl] - (uint32_t)S.p_off : jl);
+            if (jl < (uint32_t)S.N) drop |= v == (SORTED ? idx2slot[S.p_off + (int)jl] - (uint32_t)S.p_off : jl);
         }
         if (!drop) row[w++] = v;
     }
@@ -452,23 +655,30 @@ cudaError_t launch_nlist(const NlistArgs& a, cudaStream_t st) {
     cudaError_t e = cudaMemsetAsync(a.overflow, 0, 2 * sizeof(int), st);
     if (e != cudaSuccess) return e;
     k_cell_bin<<<a.n_chunks, 256, 0, st>>>(a.chunks, a.sys, a.cells, a.pos, a.ckey, a.ccount, a.wpos);
-    if ((e = launch_scan(a.ccount, a.cstart, a.n_cells, st)) != cudaSuccess) return e;
+    if ((e = launch_scan(a.ccount, a.cstart, a.n_cells, a.scan_ws, st)) != cudaSuccess) return e;
     if ((e = launch_scatter(a.chunks, a.n_chunks, a.sys, a.ckey, a.cstart, a.ccount, a.perm_u, st)) != cudaSuccess)
         return e;
-    k_cell_sort<<<a.n_cells, 256, 0, st>>>(a.cstart, a.perm_u, a.wpos, a.cpos, a.slot2idx, a.idx2slot);
-    if (a.sorted)
-        k_nlist<true><<<a.n_cells, NL_THREADS, 0, st>>>(a.cell_sys, a.sys, a.cells, a.cstart, a.cpos, a.rlist2,
-                                                        a.cap, a.head, a.nn, a.nl, a.overflow);
-    else
-        k_nlist<false><<<a.n_cells, NL_THREADS, 0, st>>>(a.cell_sys, a.sys, a.cells, a.cstart, a.cpos, a.rlist2,
-                                                         a.cap, a.head, a.nn, a.nl, a.overflow);
-    if (a.ex_n) {
-        if (a.sorted)
-            k_nlist_exclude<true><<<a.n_chunks, 256, 0, st>>>(a.chunks, a.sys, a.head, a.nn, a.nl, a.cap, a.ex_n,
-                                                               a.ex_list, a.ex_pitch, a.slot2idx, a.idx2slot);
-        else
-            k_nlist_exclude<false><<<a.n_chunks, 256, 0, st>>>(a.chunks, a.sys, a.head, a.nn, a.nl, a.cap, a.ex_n,
-                                                                a.ex_list, a.ex_pitch, a.slot2idx, a.idx2slot);
+    k_cell_sort<<<(a.total + 255) / 256, 256, 0, st>>>(a.total, a.ckey, a.cstart, a.perm_u, a.wpos, a.cpos, a.slot2idx,
+                                                       a.idx2slot);
+    if (a.half) {
+        // one warp per group of NL_GROUP particles in a cell of the mean occupancy
+        const dim3 grid((a.n_cells + NL_WARPS - 1) / NL_WARPS,
+                        std::min(8, 1 + (int)(a.total / ((long long)NL_GROUP * a.n_cells))));
+        const auto rows = a.sorted ? (a.ex_n ? k_nlist<true, true> : k_nlist<true, false>)
+                                   : (a.ex_n ? k_nlist<false, true> : k_nlist<false, false>);
+        rows<<<grid, 32 * NL_WARPS, 0, st>>>(a.cell_sys, a.n_cells, a.sys, a.cells, a.cstart, a.cpos, a.rlist2,
+                                             (uint32_t)a.cap, a.head, a.nn, a.nl, a.overflow, a.ex_n, a.ex_list,
+                                             a.ex_pitch, a.idx2slot);
+    } else {
+        const auto rows = a.sorted ? k_nlist_cta<true> : k_nlist_cta<false>;
+        rows<<<a.n_cells, NL_THREADS, 0, st>>>(a.cell_sys, a.sys, a.cells, a.cstart, a.cpos, a.rlist2, a.cap, a.head,
+                                               a.nn, a.nl, a.overflow);
+    }
+    const int done = a.half ? NL_MAXEX : 0;  // exclusions per particle left out already
+    if (a.ex_n && a.ex_pitch > done) {
+        const auto rest = a.sorted ? k_nlist_exclude<true> : k_nlist_exclude<false>;
+        rest<<<a.n_chunks, 256, 0, st>>>(a.chunks, a.sys, a.head, a.nn, a.nl, a.cap, a.ex_n, a.ex_list, a.ex_pitch,
+                                         a.slot2idx, a.idx2slot, done);
     }
     return cudaGetLastError();
 }

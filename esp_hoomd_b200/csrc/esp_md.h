@@ -8,6 +8,7 @@
 
 namespace espb {
 
+// Cells of edge >= rlist, or >= rlist / 2 (nlist_half_cells).
 struct CellDev {
     int ncx, ncy, ncz, c_off;  // cell grid and first cell
     float inv_wx, inv_wy, inv_wz;
@@ -21,11 +22,13 @@ struct NlistArgs {
     const CellDev* cells = nullptr;
     const int* cell_sys = nullptr;
     int n_cells = 0;
+    bool half = false;  // cells of rlist / 2: the warp-per-cell kernel
     int total = 0;
     const float4* pos = nullptr;
     uint32_t* ckey = nullptr;
     uint32_t* ccount = nullptr;
     uint32_t* cstart = nullptr;
+    uint32_t* scan_ws = nullptr;  // scan_ws_size(n_cells) words (may be NULL below SCAN_ONE_CTA cells)
     uint32_t* perm_u = nullptr;
     float4* wpos = nullptr;
     float4* cpos = nullptr;
@@ -35,8 +38,8 @@ struct NlistArgs {
     uint32_t* nn = nullptr;
     uint32_t* nl = nullptr;
     int* overflow = nullptr;
-    uint32_t* slot2idx = nullptr;  // cell-sorted slot -> particle (written by the cell sort)
-    uint32_t* idx2slot = nullptr;  // particle -> cell-sorted slot (may be NULL)
+    uint32_t* slot2idx = nullptr;  // cell-sorted slot -> particle (written by the cell sort; may be NULL)
+    uint32_t* idx2slot = nullptr;  // particle -> cell-sorted slot (NULL only without exclusions)
     // true: the library's pair list -- rows, head and counts indexed by the
     // cell-sorted slot, entries local slots; false: HOOMD-layout rows
     // (indexed by particle, entries local particle indices)
@@ -48,6 +51,16 @@ struct NlistArgs {
     int ex_pitch = 0;
 };
 
+// Which of the two row kernels a build takes, from its particles and the cells
+// of edge rlist that they fill: the warp-per-cell kernel on half cells when
+// those cells hold more than a CTA of the other has threads (64), or are fewer
+// than the GPU holds CTAs of it (148 SMs x 14), else one CTA per rlist cell.
+// Measured per build, CTA per rlist cell / warp per half cell: six water boxes
+// (54,000 atoms, 100 per cell) 653 / 219 us; 32 lattices of 8^3 to 14^3 (860
+// cells) 93 / 63 us; 1,000 ions 65 / 33 us; 256 lattices (5.8 million ions, 39
+// per cell) 6.21 / 6.28 ms, and there the pair kernel over cell-ordered rows
+// runs 1.66 against 1.73 ms.
+inline bool nlist_half_cells(double particles, double cells) { return particles > 64.0 * cells || cells < 148.0 * 14.0; }
 cudaError_t launch_nlist(const NlistArgs& a, cudaStream_t st);
 // skip: per-system local ranges of rigid molecules left to launch_settle1 (may be NULL)
 cudaError_t launch_nve1(const int2* chunks, int n_chunks, const SysDev* sys, float4* pos, float4* vel,

@@ -1,9 +1,13 @@
-// Pair arithmetic of the short-range term (k_pair, esp_kernels.cu): per pair
+// Pair arithmetic of the short-range term (k_pair, esp_pair.cu): per pair
 //   pair_eng   = qiqj/(4 pi) (1/r - Q(u)/r_c),  u = r^2/r_c^2
 //   force_divr = qiqj/(4 pi) (1/r^3 + 2 Q'(u)/r_c^3)
 // (the split form of EvaluatorPairPSWF::evalForceAndEnergy,
 // src/EvaluatorPairPSWF.h:274-295), Q and Q' as Horner series in v = 2u - 1
-// with the coefficients in the kernel-parameter constant bank.
+// with the coefficients in the kernel-parameter constant bank. With energies
+// the term is bound by issue slots, so the nearest image is taken without the
+// conversion unit and the reciprocal root without its subnormal path (256
+// lattices, per evaluation: 2.11 to 2.04 ms); without energies by the L1's
+// wavefronts (about 13 per 16-byte gather of a warp), where neither shows.
 #pragma once
 
 #include "esp_common.cuh"
@@ -22,15 +26,22 @@ struct PairEval {
     __device__ __forceinline__ void pair(const float4& pi, const float4& pj) {
         float dx = pi.x - pj.x, dy = pi.y - pj.y, dz = pi.z - pj.z;
         if (WRAP) {
-            dx -= Lx * rintf(dx * iLx);
-            dy -= Ly * rintf(dy * iLy);
-            dz -= Lz * rintf(dz * iLz);
+            // nearest image: 1.5 2^23 + x - 1.5 2^23 rounds x to an integer
+            // (|x| < 2 between wrapped positions; ties sit at |d| = L/2)
+            constexpr float M = 12582912.f;
+            dx = fmaf(-Lx, __fsub_rn(fmaf(dx, iLx, M), M), dx);
+            dy = fmaf(-Ly, __fsub_rn(fmaf(dy, iLy, M), M), dy);
+            dz = fmaf(-Lz, __fsub_rn(fmaf(dz, iLz, M), M), dz);
         }
         const float r2x = dx * dx + dy * dy + dz * dz;
         const bool in = r2x < rc2 && r2x > 0.f;
-        const float r2 = in ? r2x : rc2;
+        // masked pairs take r_c (finite terms times a zero charge); the lower
+        // bound, the smallest normal number, spares the reciprocal root its
+        // subnormal path
+        const float r2 = in ? fmaxf(r2x, 1.17549435e-38f) : rc2;
         {
-            const float ri = rsqrtf(r2);  // hardware estimate, a few ulp
+            float ri;
+            asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(ri) : "f"(r2));  // a few ulp
             const float v = fmaf(2.f * irc2, r2, -1.f);
             float dq = pc.d[NQ - 2];
 #pragma unroll

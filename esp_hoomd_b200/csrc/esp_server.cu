@@ -108,7 +108,7 @@ struct Staging {
 // srel, perm (4 bytes).
 constexpr long long PARTICLE_BYTES = 7 * 16 + 9 * 4;
 constexpr long long MESH_BYTES = 8 + 4 + 8;  // rho (double), phi (float), half spectrum (float2)
-constexpr int MAX_CELLS_AXIS = 40;
+constexpr int MAX_CELLS_AXIS = 80;
 constexpr int MAX_PSETS = 16;
 
 struct Request {
@@ -178,7 +178,7 @@ struct esp_server {
     float* d_q = nullptr;
     uint32_t *d_rel = nullptr, *d_key = nullptr, *d_perm_u = nullptr, *d_perm = nullptr, *d_srel = nullptr,
              *d_head = nullptr, *d_nn = nullptr, *d_ckey = nullptr, *d_cperm = nullptr,
-             *d_ccount = nullptr, *d_cstart = nullptr, *d_nl = nullptr;
+             *d_ccount = nullptr, *d_cstart = nullptr, *d_nl = nullptr, *d_scan = nullptr, *d_cscan = nullptr;
     int* d_tile_sys = nullptr;
     uint32_t *d_tcount = nullptr, *d_tstart = nullptr;
     double* d_rho = nullptr;
@@ -314,7 +314,8 @@ int esp_server::init(const esp_server_config& cfg) {
         (rc = mem.get(d_perm, P_cap)) || (rc = mem.get(d_srel, P_cap)) || (rc = mem.get(d_head, P_cap)) ||
         (rc = mem.get(d_nn, P_cap)) || (rc = mem.get(d_ckey, P_cap)) || (rc = mem.get(d_cperm, max_particles)) ||
         (rc = mem.get(d_cpos, max_particles)) ||
-        (rc = mem.get(d_ccount, C_cap)) || (rc = mem.get(d_cstart, C_cap + 1)) || (rc = mem.get(d_nl, NL_cap)) ||
+        (rc = mem.get(d_ccount, C_cap)) || (rc = mem.get(d_cstart, C_cap + 1)) ||
+        (rc = mem.get(d_cscan, scan_ws_size(C_cap))) || (rc = mem.get(d_scan, scan_ws_size(T_cap))) || (rc = mem.get(d_nl, NL_cap)) ||
         (rc = mem.get(d_tile_sys, T_cap)) || (rc = mem.get(d_tcount, T_cap)) || (rc = mem.get(d_tstart, T_cap + 1)) ||
         (rc = mem.get(d_rho, M_cap)) || (rc = mem.get(d_phi, M_cap)) || (rc = mem.get(d_spec, M_cap)) ||
         (rc = mem.get(d_gtab, G_cap)) || (rc = mem.get(d_tw, tw.size())) ||
@@ -603,10 +604,14 @@ int esp_server::admit(Request* q, Staging& sg) {
     // neighbour list (cell list of this system alone)
     CellDev C{};
     int nc[3];
+    double full = 1;
     for (int d = 0; d < 3; ++d) {
         if (2.0 * rlist > L[d]) return fail(ESP_ERR_INVALID, "rcut + skin must not exceed half the box");
-        nc[d] = std::min(MAX_CELLS_AXIS, std::max(1, (int)std::floor(L[d] / rlist)));
+        full *= std::max(1.0, std::floor(L[d] / rlist));
     }
+    const bool half = nlist_half_cells(r.N, full);
+    for (int d = 0; d < 3; ++d)
+        nc[d] = std::min(MAX_CELLS_AXIS, std::max(1, (int)std::floor((half ? 2.0 : 1.0) * L[d] / rlist)));
     C.ncx = nc[0];
     C.ncy = nc[1];
     C.ncz = nc[2];
@@ -629,11 +634,13 @@ int esp_server::admit(Request* q, Staging& sg) {
     na.cells = d_cells;
     na.cell_sys = d_cell_sys;
     na.n_cells = ncell;
+    na.half = half;
     na.total = r.N;
     na.pos = d_pos;
     na.ckey = d_ckey;
     na.ccount = d_ccount;
     na.cstart = d_cstart;
+    na.scan_ws = d_cscan;
     na.perm_u = d_cperm;
     na.wpos = d_wpos;
     na.cpos = d_cpos;
@@ -738,6 +745,7 @@ int esp_server::launch_round(Staging& sg) {
     a.n_tiles = (int)talloc.high();
     a.tile_count = d_tcount;
     a.tile_start = d_tstart;
+    a.scan_ws = d_scan;
     a.pos_in = d_pos;
     a.q_in = d_q;
     a.posq = d_posq;

@@ -6,6 +6,12 @@ where the rule switches, against the oracle.
   1e-12 relative RMS, sums of ~100 terms; FP32: 2e-5, the rounding of a
   minimum-image displacement (L 2^-24 / r ~ 1.3e-6) amplified 14-fold by
   r^-14).
+* neighbour rows (HOOMD layout and pair list): cells of half the list radius
+  (few cells, or full ones) with 4 and >= 5 cells per axis and both at once and
+  with more than 8 and more than 32 particles in a cell; cells of the list
+  radius, sparse and more than 16,384 of them (scanned by several CTAs); capacities that are no multiple of 4, and more
+  excluded partners than the kernel keeps in shared memory: the rows are the
+  oracle's sets.
 * tile sort: tiles of a few particles, above the 512-thread switch, and above
   the shared-memory capacity (2,048); permutation bit-exact.
 """
@@ -16,6 +22,7 @@ torch = pytest.importorskip("torch")
 pytestmark = pytest.mark.gpu
 
 from esp_hoomd_b200 import native, systems  # noqa: E402
+from esp_hoomd_b200._lib import ESP_SHORT_RANGE  # noqa: E402
 from oracle import esp_ref as R  # noqa: E402
 
 
@@ -72,3 +79,65 @@ def test_tile_sort_bit_exact(n, mesh):
     k_ref, p_ref = R.bin_sort(pos, (L, L, L), (mesh,) * 3, inf["order"], inf["tile"])
     assert np.array_equal(key.cpu().numpy().astype(np.uint32), k_ref)
     assert np.array_equal(perm.cpu().numpy().astype(np.uint32), p_ref)
+
+
+def _rows(head, cnt, lst):
+    return [sorted(lst[h:h + c].tolist()) for h, c in zip(head, cnt)]
+
+
+def _check_lists(pos, box, rlist, cap, excl=None):
+    pos = pos.astype(np.float32).astype(np.float64)
+    n = len(pos)
+    b = native.Batch(native.make_params(rcut=rlist, mesh=(16, 16, 16)), [n], [box])
+    p4 = torch.zeros((n, 4), device="cuda")
+    p4[:, :3] = torch.as_tensor(pos, device="cuda")
+    if excl is not None:
+        b.set_exclusions(torch.as_tensor(excl[0].astype(np.int32), device="cuda"),
+                         torch.as_tensor(excl[1].astype(np.int32), device="cuda"), excl[2])
+    head = torch.zeros(n, dtype=torch.int32, device="cuda")
+    nn = torch.zeros_like(head)
+    nl = torch.zeros(n * cap, dtype=torch.int32, device="cuda")
+    b.build_nlist(p4, rlist, cap, head, nn, nl)
+    b.nlist_check()
+    ref = R.neighbor_list(pos, box, rlist)
+    if excl is not None:
+        ref = R.remove_pairs(ref, *excl)
+    got = tuple(t.cpu().numpy() for t in (head, nn, nl))
+    assert np.array_equal(got[1], ref[1].astype(np.int32))
+    assert _rows(*got) == _rows(ref[0], ref[1], ref[2])
+    # the pair list holds the same pairs: equal forces up to the summation order
+    q = torch.as_tensor(np.where(np.arange(n) % 2 == 0, 1.0, -1.0), dtype=torch.float32, device="cuda")
+    f = [torch.zeros((n, 4), device="cuda") for _ in range(2)]
+    b.compute(p4, q, f[0], nlist=(head, nn, nl), flags=ESP_SHORT_RANGE)
+    b.build_pairlist(p4, rlist, cap)
+    b.pairlist_check()
+    b.compute(p4, q, f[1], flags=ESP_SHORT_RANGE)
+    a, c = (x.double().cpu().numpy()[:, :3] for x in f)
+    assert R.rel_rms(c, a) <= 1e-6
+
+
+@pytest.mark.parametrize("box,n,rlist,cap", [
+    ((7.0, 7.3, 8.4), 400, 3.4, 253),     # 4 cells on every axis
+    ((7.5, 12.0, 31.0), 2500, 3.0, 256),  # 5 cells on one axis, more on the others
+    ((6.2, 20.0, 20.0), 2000, 3.0, 256),  # 4 cells on one axis only
+    ((9.0, 9.0, 9.0), 6000, 2.0, 512),    # 8 particles per cell and more
+    ((40.0, 40.0, 40.0), 300, 1.5, 16),   # a cell holds a particle rarely: cells enlarged
+    ((60.0, 60.0, 60.0), 20000, 2.0, 64),  # 216,000 cells
+])
+def test_neighbour_rows(box, n, rlist, cap):
+    rng = np.random.default_rng(n)
+    _check_lists(rng.uniform(0, 1, (n, 3)) * np.asarray(box), box, rlist, cap)
+
+
+def test_neighbour_rows_of_a_dense_cell():
+    rng = np.random.default_rng(9)
+    pos = np.concatenate([rng.uniform(0, 20.0, (1000, 3)), rng.uniform(5.0, 6.5, (300, 3))])
+    _check_lists(pos, (20.0, 20.0, 20.0), 3.0, 600)
+
+
+@pytest.mark.parametrize("per_mol", [2, 9, 12])  # 1, 8 and 11 excluded partners
+@pytest.mark.parametrize("n_mol,L", [(60, 9.0), (900, 28.0)])  # both row kernels
+def test_neighbour_rows_exclusions(per_mol, n_mol, L):
+    rng = np.random.default_rng(per_mol)
+    pos = np.mod(np.repeat(rng.uniform(0, L, (n_mol, 3)), per_mol, 0) + rng.normal(0, 0.3, (n_mol * per_mol, 3)), L)
+    _check_lists(pos, (L, L, L), 2.0, 256, R.molecule_exclusions(n_mol, per_mol))
