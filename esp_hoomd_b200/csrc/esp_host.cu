@@ -85,22 +85,22 @@ uint32_t radix_plan(int n) {
     return code;
 }
 
-// (PX, PP) pitches of the interpolation tile. A group of G lanes serves one
-// particle (lane c reads stencil plane oz + c) and K = 32 / G groups share a
-// warp. With the plane pitch PP = K (mod 32) a group's lanes fall in the bank
-// class of its row start, and with the row pitch PX a multiple of K that
-// class is the particle's x origin mod K; the kernel orders particles so the
-// K groups of a warp have distinct classes (conflict-free reads).
+// (PX, PP) pitches of the interpolation tile staged by cp.async. A group of G
+// lanes serves one particle (lane c reads stencil plane oz + c) and K = 32 / G
+// groups share a warp. Supports 5..8 (K = 4), as the TMA box: plane pitch = 4
+// (mod 8), so a group's lanes read 8 distinct banks of the class of their x,
+// and row pitch = 0 (mod 4), so that class is x mod 4. Other supports: plane
+// pitch = K (mod 32) and row pitch = 1 (mod K), so that the bank class of a
+// particle is (ox + oy) mod K, close to uniform over a tile (the kernel orders
+// the particles by it).
 void choose_pitch(int P, int E, int& PX, int& PP) {
-    // interpolation region pitches: plane pitch = K (mod 32), so the G lanes
-    // of a particle read G banks K apart; row pitch = 1 (mod K), so the bank
-    // class of a particle is (ox + oy) mod K, close to uniform over a tile
     const int G = P <= 4 ? 4 : (P <= 8 ? 8 : 16);
     const int K = 32 / G;
+    const bool wide = P >= 5 && P <= 8;
     PX = E;
-    while (PX % K != 1) ++PX;
+    while (PX % K != (wide ? 0 : 1)) ++PX;
     PP = E * PX;
-    while (PP % 32 != K) ++PP;
+    while (wide ? PP % 8 != 4 : PP % 32 != K) ++PP;
 }
 
 int build_param_set(double c, double cw, int P, int D, double rcut, PsetHost& h, ParamSet& d, double tol) {

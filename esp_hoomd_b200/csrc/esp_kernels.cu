@@ -630,6 +630,29 @@ __device__ __forceinline__ void mma_tf32(float (&d)[4], uint32_t a0, uint32_t a1
         : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
 
+// CTA y of gridDim.y takes its share of a tile's particles, whole multiples of
+// `unit` but the last: first particle and count (0: none). Tiles fewer than the
+// GPU holds CTAs are shared out this way (tile_split).
+__device__ __forceinline__ void tile_share(uint32_t& s0, int& np, int unit) {
+    if (gridDim.y == 1) return;
+    const int share = ((np + (int)gridDim.y - 1) / (int)gridDim.y + unit - 1) / unit * unit;
+    const int first = share * (int)blockIdx.y;
+    s0 += (uint32_t)first;
+    np = min(share, np - first);
+}
+
+// CTAs per tile of a tile kernel: enough to fill the GPU (148 SMs x per_sm
+// resident CTAs), at most one per `unit` particles of the mean tile and 8.
+// Each stages the region or weights again and flushes its own sums, which the
+// idle SMs pay for: 98,304 particles in 125 tiles (support 6), spreading 90 to
+// 39 us, interpolation 92 to 25; 512 ions in 8 tiles 7.7 to 5.6 and 10.2 to 5.9
+// us. With a CTA per tile for every resident slot it would only add work.
+static int tile_split(const LaunchArgs& a, int per_sm, int unit) {
+    if (a.n_tiles >= 148 * per_sm) return 1;
+    const long long mean = a.n_chunks * 256LL / a.n_tiles;
+    return (int)std::max(1LL, std::min({8LL, 148LL * per_sm / a.n_tiles, (mean + unit - 1) / unit}));
+}
+
 constexpr int SPREAD_CHM = 48;  // particles staged per round (multiple of 8; 4 CTAs of 256 threads per SM)
 constexpr int SPREAD_MS = 24;   // staged row stride: rows of 4 consecutive particles hit disjoint banks
 
@@ -644,9 +667,10 @@ __global__ void __launch_bounds__(256, 4)
     // half of the 16 rows; a warp skips the k-steps that miss its two rows)
     __shared__ int ks_lo[SPREAD_CHM / 8], ks_hi[SPREAD_CHM / 8];
     const int t = blockIdx.x;
-    const uint32_t s0 = start[t];
-    const int np = (int)(start[t + 1] - s0);
-    if (np == 0) return;
+    uint32_t s0 = start[t];
+    int np = (int)(start[t + 1] - s0);
+    tile_share(s0, np, 8);
+    if (np <= 0) return;
     const int si = tile_sys[t];
     const SysDev S = sys[si];
     const ParamSet& ps = psets[S.pset];
@@ -1374,11 +1398,20 @@ __global__ void k_influence(SysDev S, const double* __restrict__ w1d, const doub
 // Each chunk's particle records and output slots are prefetched into shared
 // memory (cp.async) while the previous chunk is interpolated.
 // ============================================================================
+// Weight row of one staged particle: six vectors of P words (wx dwx wy dwy wz
+// dwz). For supports 5..8 each vector fills 8 words and a row 52, so that a
+// lane group reads them 16 bytes at a time (rows of particles that differ mod 8
+// start in different banks); otherwise packed, rows of odd stride.
+__host__ __device__ constexpr bool interp_wide(int P) { return P >= 5 && P <= 8; }
+__host__ __device__ constexpr int interp_vec(int P) { return interp_wide(P) ? 8 : P; }
+__host__ __device__ constexpr int interp_row(int P) { return interp_wide(P) ? 52 : 6 * P + 1; }
+
 // words of the interpolation staging area: the per-chunk weights, or (before
 // the first chunk) the wrapped row offsets, shared row offsets and x
 // indices of the region
 __host__ __device__ inline int interp_stage_words(int P, int CH, int E) {
-    return CH * (6 * P + 1) > 2 * E * E + E ? CH * (6 * P + 1) : 2 * E * E + E;
+    const int w = CH * interp_row(P), t = (2 * E * E + E + 3) & ~3;
+    return w > t ? w : t;
 }
 
 template <int P>
@@ -1411,20 +1444,38 @@ __device__ __forceinline__ bool tma_wait(uint32_t mbar, uint32_t phase) {
 }
 
 // One chunk of a tile's particles (records already in shared memory):
-// window weights and derivatives, the processing order, and the contraction
-// of each particle's stencil with the staged potential region; writes the
-// particles' forces and energies and returns the chunk's energy (FP64).
-// Called by every thread of the CTA (it synchronises).
-template <int P, bool TMA>
-__device__ __forceinline__ double interp_chunk(const float* __restrict__ sm, int PX, int PP, int xoff, int D,
+// window weights and derivatives, and the contraction of each particle's
+// stencil with the staged potential region; writes the particles' forces and
+// energies and returns the chunk's energy (FP64). Called by every thread of
+// the CTA (it synchronises).
+//
+// Shared-memory wavefronts are what bounds it. A group of G lanes serves one
+// particle, lane c reading stencil plane oz + c; the plane pitch puts a group's
+// lanes in the G banks of one class mod K = 32 / G, the class of the point's x.
+// Supports 5..8 (K = 4, row pitch a multiple of 4): group g of a warp walks its
+// stencil's x points starting at the one of class g (plus the region's offset,
+// the same for all), wrapping around, so the four groups read four classes at
+// every step whatever the particles' origins; the x weights are staged already
+// rotated, and all weights are read 16 bytes at a time. Against a
+// conflict-avoiding order of the chunk's particles (1.41 wavefronts per
+// potential load, a barrier) and 4-byte weight loads: 50 to 38 wavefronts per
+// particle, 1.18 to 1.00 ms per evaluation of 256 lattices (5.8 million ions).
+// Folding the four sums over the lanes (4 shuffles instead of 12, one 4-byte
+// store per component) measured 4% slower.
+// Other supports: the particles of a chunk are ordered so that the groups of a
+// warp have distinct classes (ox + oy) mod K where possible.
+template <int P, bool TMA, int PXC>
+__device__ __forceinline__ double interp_chunk(const float* __restrict__ sm, int PXr, int PP, int xoff, int D,
                                                const float* __restrict__ wc, const float4* __restrict__ crec,
                                                const uint32_t* __restrict__ crel, const uint32_t* __restrict__ cprm,
                                                float* __restrict__ wts, float* __restrict__ qv, int* __restrict__ org,
                                                int* __restrict__ order, int nc, float gxs, float gys, float gzs,
                                                double self_coef, float4* __restrict__ force) {
     using C = InterpCfg<P>;
-    constexpr int WS = 6 * P + 1;  // weight row stride (odd: conflict-free broadcasts)
-    constexpr int K = 32 / C::G;   // particle groups per warp
+    constexpr int WS = interp_row(P), V = interp_vec(P);
+    constexpr int K = 32 / C::G;  // particle groups per warp
+    constexpr bool ROT = interp_wide(P);
+    const int PX = PXC ? PXC : PXr;
     const int grp = threadIdx.x / C::G, gl = threadIdx.x % C::G;
     double esum = 0.0;
     {
@@ -1437,90 +1488,117 @@ __device__ __forceinline__ double interp_chunk(const float* __restrict__ sm, int
             if (D == DD) sp.load(&wc[a2 * (D + 1)]);
             for (int p = p0; p < nc; p += nla) {
                 const float4 rec = crec[p];
-                float* W = wts + p * WS + a2;
+                float* W = wts + p * WS;
+                int ax0 = a2;  // slot of the x weight
+                if (ROT) {
+                    ax0 -= (p - (int)(crel[p] & 255u)) & 3;
+                    ax0 += ax0 < 0 ? P : 0;
+                }
 #pragma unroll
                 for (int ax = 0; ax < 3; ++ax) {
                     const float tt = ax == 0 ? rec.x : (ax == 1 ? rec.y : rec.z);
+                    float* Wa = W + ax * 2 * V + (ax == 0 ? ax0 : a2);
                     if (D == DD) {
-                        W[ax * 2 * P] = sp.w(tt);
-                        W[ax * 2 * P + P] = sp.dw(tt);
+                        Wa[0] = sp.w(tt);
+                        Wa[V] = sp.dw(tt);
                     } else {
-                        W[ax * 2 * P] = horner_w(&wc[a2 * (D + 1)], D, tt);
-                        W[ax * 2 * P + P] = horner_dw(&wc[a2 * (D + 1)], D, tt);
+                        Wa[0] = horner_w(&wc[a2 * (D + 1)], D, tt);
+                        Wa[V] = horner_dw(&wc[a2 * (D + 1)], D, tt);
                     }
                 }
             }
         }
-        for (int p = threadIdx.x; p < nc; p += blockDim.x) {
-            qv[p] = crec[p].w;
-            org[p] = (int)crel[p];
-        }
+        if (!ROT)
+            for (int p = threadIdx.x; p < nc; p += blockDim.x) {
+                qv[p] = crec[p].w;
+                org[p] = (int)crel[p];
+            }
     }
     __syncthreads();
-    if (C::CH <= 32 && threadIdx.x < 32) {
-        // processing order: queue position q prefers a particle whose
-        // bank class (ox + oy) mod K is q mod K, so the K groups of a warp
-        // read potential rows in disjoint bank classes (plane pitch = K
-        // mod 32, row pitch = 1 mod K); particles left over fill the free
-        // positions in order
-        const int j = threadIdx.x;
-        const unsigned full = 0xffffffffu, lt = (1u << j) - 1u;
-        const bool valid = j < nc;
-        // bank class of the particle's rows: (ox + oy) mod K for the padded
-        // cp.async layout; ox + xoff mod K for the TMA box (pitches = 0 mod K)
-        const int cls = valid ? ((TMA ? (org[j] & 255) + xoff : (org[j] & 255) + ((org[j] >> 8) & 255)) & (K - 1))
-                              : -1;
-        int rank = 0, cpos = 0;
-        const int pk = j & (K - 1);
+    if (!ROT) {
+        if (C::CH <= 32 && threadIdx.x < 32) {
+            // processing order: queue position q prefers a particle whose
+            // bank class (ox + oy) mod K is q mod K, so the K groups of a warp
+            // read potential rows in disjoint bank classes (plane pitch = K
+            // mod 32, row pitch = 1 mod K); particles left over fill the free
+            // positions in order
+            const int j = threadIdx.x;
+            const unsigned full = 0xffffffffu, lt = (1u << j) - 1u;
+            const bool valid = j < nc;
+            const int cls = valid ? (((org[j] & 255) + ((org[j] >> 8) & 255)) & (K - 1)) : -1;
+            int rank = 0, cpos = 0;
+            const int pk = j & (K - 1);
 #pragma unroll
-        for (int k = 0; k < K; ++k) {
-            const unsigned m = __ballot_sync(full, cls == k);
-            if (cls == k) rank = __popc(m & lt);
-            if (pk == k) cpos = __popc(m);
+            for (int k = 0; k < K; ++k) {
+                const unsigned m = __ballot_sync(full, cls == k);
+                if (cls == k) rank = __popc(m & lt);
+                if (pk == k) cpos = __popc(m);
+            }
+            const int slots = valid ? (nc - cls + K - 1) / K : 0;
+            const bool placed = valid && rank < slots;
+            const unsigned fm = __ballot_sync(full, j < nc && j / K >= cpos);
+            const unsigned lm = __ballot_sync(full, valid && !placed);
+            if (placed) order[cls + K * rank] = j;
+            else if (valid) order[__fns(fm, 0, __popc(lm & lt) + 1)] = j;
+        } else if (C::CH > 32) {
+            for (int p = threadIdx.x; p < nc; p += blockDim.x) order[p] = p;
         }
-        const int slots = valid ? (nc - cls + K - 1) / K : 0;
-        const bool placed = valid && rank < slots;
-        const unsigned fm = __ballot_sync(full, j < nc && j / K >= cpos);
-        const unsigned lm = __ballot_sync(full, valid && !placed);
-        if (placed) order[cls + K * rank] = j;
-        else if (valid) order[__fns(fm, 0, __popc(lm & lt) + 1)] = j;
-    } else if (C::CH > 32) {
-        for (int p = threadIdx.x; p < nc; p += blockDim.x) order[p] = p;
+        __syncthreads();
     }
-    __syncthreads();
     for (int pp = 0; pp < nc; pp += C::NG) {
         const int qq = pp + grp;
-        const int p = qq < nc ? order[qq] : qq;
+        const int p = ROT ? qq : (qq < nc ? order[qq] : qq);
         const bool act = qq < nc && gl < P;
         float pot = 0.f, gx = 0.f, gy = 0.f, gz = 0.f;
         if (act) {
             const float* W = wts + p * WS;
-            float wx[P], dwx[P];
+            float wx[V], dwx[V], wy[V], dwy[V];
+            if (interp_wide(P)) {
 #pragma unroll
-            for (int a2 = 0; a2 < P; ++a2) {
-                wx[a2] = W[a2];
-                dwx[a2] = W[P + a2];
+                for (int h = 0; h < V; h += 4) {
+                    const float4 u0 = *reinterpret_cast<const float4*>(W + h);
+                    const float4 u1 = *reinterpret_cast<const float4*>(W + V + h);
+                    const float4 u2 = *reinterpret_cast<const float4*>(W + 2 * V + h);
+                    const float4 u3 = *reinterpret_cast<const float4*>(W + 3 * V + h);
+                    wx[h] = u0.x, wx[h + 1] = u0.y, wx[h + 2] = u0.z, wx[h + 3] = u0.w;
+                    dwx[h] = u1.x, dwx[h + 1] = u1.y, dwx[h + 2] = u1.z, dwx[h + 3] = u1.w;
+                    wy[h] = u2.x, wy[h + 1] = u2.y, wy[h + 2] = u2.z, wy[h + 3] = u2.w;
+                    dwy[h] = u3.x, dwy[h + 1] = u3.y, dwy[h + 2] = u3.z, dwy[h + 3] = u3.w;
+                }
+            } else {
+#pragma unroll
+                for (int a2 = 0; a2 < P; ++a2) {
+                    wx[a2] = W[a2];
+                    dwx[a2] = W[V + a2];
+                }
             }
-            const int rl = org[p];
+            const int rl = ROT ? (int)crel[p] : org[p];
             const int ox = rl & 255, oy = (rl >> 8) & 255, oz = (rl >> 16) & 255;
             const float* plane = sm + (oz + gl) * PP + oy * PX + ox + xoff;
+            // ROT: slot k of the walk is stencil point (k + rot) mod P; the last
+            // three slots may have wrapped
+            const int rot = ROT ? (p - ox) & 3 : 0;
+            const float* walk = plane + rot;
+            int wrap[3];
+#pragma unroll
+            for (int k = 0; k < 3; ++k) wrap[k] = (ROT && P - 3 + k + rot >= P) ? -P : 0;
             float Sv = 0.f, Dv = 0.f, Sy = 0.f;
 #pragma unroll
             for (int b = 0; b < P; ++b) {
-                const float* row = plane + b * PX;
                 float sr = 0.f, dr = 0.f;
 #pragma unroll
                 for (int a2 = 0; a2 < P; ++a2) {
-                    const float v = row[a2];
+                    const float v = (ROT && a2 >= P - 3) ? (walk + wrap[a2 < P - 3 ? 0 : a2 - (P - 3)])[b * PX + a2]
+                                                         : walk[b * PX + a2];
                     sr = fmaf(v, wx[a2], sr);
                     dr = fmaf(v, dwx[a2], dr);
                 }
-                const float wyb = W[2 * P + b], dwyb = W[3 * P + b];
+                const float wyb = interp_wide(P) ? wy[b] : W[2 * V + b], dwyb = interp_wide(P) ? dwy[b] : W[3 * V + b];
                 Sv = fmaf(sr, wyb, Sv);
                 Dv = fmaf(dr, wyb, Dv);
                 Sy = fmaf(sr, dwyb, Sy);
             }
-            const float wzc = W[4 * P + gl], dwzc = W[5 * P + gl];
+            const float wzc = W[4 * V + gl], dwzc = W[5 * V + gl];
             pot = Sv * wzc;
             gx = Dv * wzc;
             gy = Sy * wzc;
@@ -1534,7 +1612,7 @@ __device__ __forceinline__ double interp_chunk(const float* __restrict__ sm, int
             gz += __shfl_xor_sync(0xffffffffu, gz, o, C::G);
         }
         if (qq < nc && gl == 0) {
-            const float q = qv[p];
+            const float q = ROT ? crec[p].w : qv[p];
             const double e_i = 0.5 * (double)q * pot + self_coef * (double)q * q;
             force[cprm[p]] = make_float4(q * gxs * gx, q * gys * gy, q * gzs * gz, (float)e_i);
             esum += e_i;
@@ -1543,7 +1621,7 @@ __device__ __forceinline__ double interp_chunk(const float* __restrict__ sm, int
     return esum;
 }
 
-template <int P, bool TMA>
+template <int P, bool TMA, int PXC>
 __global__ void __launch_bounds__(128, 6)
     k_interp(const int* __restrict__ tile_sys, const SysDev* __restrict__ sys, const ParamSet* __restrict__ psets,
              int T, int D, int PX, int PP, const uint32_t* __restrict__ start, const uint32_t* __restrict__ perm,
@@ -1555,9 +1633,10 @@ __global__ void __launch_bounds__(128, 6)
     __shared__ double red[32];
     __shared__ __align__(8) uint64_t mbar;
     const int t = blockIdx.x;
-    const uint32_t s0 = start[t];
-    const int np = (int)(start[t + 1] - s0);
-    if (np == 0) return;
+    uint32_t s0 = start[t];
+    int np = (int)(start[t + 1] - s0);
+    tile_share(s0, np, C::NG);
+    if (np <= 0) return;
     const int si = tile_sys[t];
     const SysDev S = sys[si];
     const ParamSet& ps = psets[S.pset];
@@ -1569,7 +1648,7 @@ __global__ void __launch_bounds__(128, 6)
     float4* crec = reinterpret_cast<float4*>(sm + ((E * PP + 3) & ~3));    // [2][CH]
     uint32_t* crel = reinterpret_cast<uint32_t*>(crec + 2 * C::CH);         // [2][CH]
     uint32_t* cprm = crel + 2 * C::CH;                                      // [2][CH]
-    float* wts = reinterpret_cast<float*>(cprm + 2 * C::CH);  // [CH][6P] wx dwx wy dwy wz dwz (index tables first)
+    float* wts = reinterpret_cast<float*>(cprm + 2 * C::CH);  // [CH] weight rows (index tables first)
     float* qv = wts + interp_stage_words(P, C::CH, E);  // [CH] charges
     int* org = reinterpret_cast<int*>(qv + C::CH); // [CH] packed origins
     int* order = org + C::CH;                      // [CH] processing order of the chunk
@@ -1655,7 +1734,7 @@ __global__ void __launch_bounds__(128, 6)
         const int nc = min(C::CH, np - base);
         __syncthreads();  // region / coefficients / records staged; previous chunk consumed
         if (base + C::CH < np) prefetch(base + C::CH, cb ^ 1);
-        esum += interp_chunk<P, TMA>(sm, PX, PP, xoff, D, wc, crec + cb * C::CH, crel + cb * C::CH,
+        esum += interp_chunk<P, TMA, PXC>(sm, PX, PP, xoff, D, wc, crec + cb * C::CH, crel + cb * C::CH,
                                      cprm + cb * C::CH, wts, qv, org, order, nc, gxs, gys, gzs, self_coef, force);
         asm volatile("cp.async.wait_group 0;\n" ::);  // next chunk's records (made visible by the top barrier)
     }
@@ -1681,7 +1760,7 @@ __host__ __device__ inline int interp_q_region_words(int E, int PP) {
 template <int P>
 __host__ __device__ inline int interp_q_smem(int E, int PP) {
     using C = InterpCfg<P>;
-    return 128 + 4 * (2 * interp_q_region_words(E, PP) + C::CH * (6 * P + 1) + 3 * C::CH + P * (MAX_D + 1)) +
+    return 128 + 4 * (2 * interp_q_region_words(E, PP) + C::CH * interp_row(P) + 3 * C::CH + P * (MAX_D + 1)) +
            2 * C::CH * 24;
 }
 
@@ -1703,8 +1782,8 @@ __global__ void __launch_bounds__(128, 5)
     float4* crec = reinterpret_cast<float4*>(reg0 + 2 * RW);       // [2][CH]
     uint32_t* crel = reinterpret_cast<uint32_t*>(crec + 2 * C::CH);  // [2][CH]
     uint32_t* cprm = crel + 2 * C::CH;                               // [2][CH]
-    float* wts = reinterpret_cast<float*>(cprm + 2 * C::CH);         // [CH][6P + 1]
-    float* qv = wts + C::CH * (6 * P + 1);                           // [CH]
+    float* wts = reinterpret_cast<float*>(cprm + 2 * C::CH);         // [CH] weight rows
+    float* qv = wts + C::CH * interp_row(P);                           // [CH]
     int* org = reinterpret_cast<int*>(qv + C::CH);                   // [CH]
     int* order = org + C::CH;                                        // [CH]
     float* wc = reinterpret_cast<float*>(order + C::CH);             // [P][D+1]
@@ -1816,7 +1895,7 @@ __global__ void __launch_bounds__(128, 5)
             } else if (s_tile[b ^ 1] < n_tiles) {
                 prefetch((uint32_t)s_first[b ^ 1], min(C::CH, s_np[b ^ 1]), cbuf ^ 1);
             }
-            esum += interp_chunk<P, true>(reg0 + b * RW, PX, PP, xoff, D, wc, crec + cbuf * C::CH,
+            esum += interp_chunk<P, true, 0>(reg0 + b * RW, PX, PP, xoff, D, wc, crec + cbuf * C::CH,
                                           crel + cbuf * C::CH, cprm + cbuf * C::CH, wts, qv, org, order, nc, gxs, gys,
                                           gzs, self_coef, force);
             cbuf ^= 1;
@@ -1933,7 +2012,7 @@ static cudaError_t launch_spread_p(const LaunchArgs& a, cudaStream_t st) {
     }
     if (a.n_tiles == 0) return cudaSuccess;
     if (mma)
-        k_spread_mma<P><<<a.n_tiles, 256, smem_m, st>>>(a.tile_sys, a.sys, a.psets, a.T, a.D, a.tile_start, a.srec,
+        k_spread_mma<P><<<dim3(a.n_tiles, tile_split(a, 4, SPREAD_CHM)), 256, smem_m, st>>>(a.tile_sys, a.sys, a.psets, a.T, a.D, a.tile_start, a.srec,
                                                         a.srel, a.rho);
     else if (dense)
         k_spread_dense<P><<<a.n_tiles, 256, smem_d, st>>>(a.tile_sys, a.sys, a.psets, a.T, a.D, a.tile_start, a.srec,
@@ -1959,6 +2038,7 @@ static cudaError_t launch_interp_p(const LaunchArgs& a, cudaStream_t st) {
     using C = InterpCfg<P>;
     const int E = a.T + P - 1;
     constexpr bool kTmaForm = P >= 5 && P <= 8;  // 8 lanes per particle: the box pitches give distinct banks
+    constexpr int kPx = kTmaForm ? 20 : 0;       // row pitch of the default tile's box (E = 16), an immediate
     const bool tma = kTmaForm && a.tmaps != nullptr;
     const int PX = tma ? a.tma_bx : a.PX, PP = tma ? a.tma_bx * a.tma_by : a.PP;
     if (a.configure_only) {
@@ -1968,12 +2048,14 @@ static cudaError_t launch_interp_p(const LaunchArgs& a, cudaStream_t st) {
         cudaError_t e = cudaSuccess;
         const int s0 = (int)interp_smem<P>(E, a.PP);
         if (s0 > configured[0]) {
-            e = cudaFuncSetAttribute(k_interp<P, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, s0);
+            e = cudaFuncSetAttribute(k_interp<P, false, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, s0);
             if (e == cudaSuccess) configured[0] = s0;
         }
         const int s1 = (int)interp_smem<P>(E, a.tma_bx * a.tma_by);
         if (e == cudaSuccess && kTmaForm && a.tma_bx > 0 && s1 > configured[1]) {
-            e = cudaFuncSetAttribute(k_interp<P, kTmaForm>, cudaFuncAttributeMaxDynamicSharedMemorySize, s1);
+            e = cudaFuncSetAttribute(k_interp<P, kTmaForm, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, s1);
+            if (e == cudaSuccess)
+                e = cudaFuncSetAttribute(k_interp<P, kTmaForm, kPx>, cudaFuncAttributeMaxDynamicSharedMemorySize, s1);
             if (e == cudaSuccess) configured[1] = s1;
         }
         const int s2 = interp_q_smem<P>(E, a.tma_bx * a.tma_by);
@@ -2001,11 +2083,12 @@ static cudaError_t launch_interp_p(const LaunchArgs& a, cudaStream_t st) {
         return cudaGetLastError();
     }
     if (tma)
-        k_interp<P, kTmaForm><<<a.n_tiles, C::THREADS, interp_smem<P>(E, PP), st>>>(
+        (PX == kPx ? k_interp<P, kTmaForm, kPx> : k_interp<P, kTmaForm, 0>)<<<dim3(a.n_tiles, tile_split(a, 6, C::CH)), C::THREADS,
+                                                                              interp_smem<P>(E, PP), st>>>(
             a.tile_sys, a.sys, a.psets, a.T, a.D, PX, PP, a.tile_start, a.perm, a.srec, a.srel, a.phi, a.force, a.acc,
             reinterpret_cast<const CUtensorMap*>(a.tmaps), a.kerr);
     else
-        k_interp<P, false><<<a.n_tiles, C::THREADS, interp_smem<P>(E, PP), st>>>(
+        k_interp<P, false, 0><<<dim3(a.n_tiles, tile_split(a, 6, C::CH)), C::THREADS, interp_smem<P>(E, PP), st>>>(
             a.tile_sys, a.sys, a.psets, a.T, a.D, PX, PP, a.tile_start, a.perm, a.srec, a.srel, a.phi, a.force, a.acc,
             nullptr, a.kerr);
     return cudaGetLastError();

@@ -12,6 +12,10 @@ where the rule switches, against the oracle.
   radius, sparse and more than 16,384 of them (scanned by several CTAs); capacities that are no multiple of 4, and more
   excluded partners than the kernel keeps in shared memory: the rows are the
   oracle's sets.
+* tile shares: few tiles, their particles shared out over several CTAs, with
+  full, nearly empty and empty tiles at once, supports 5..8 (the rotated walk
+  of the interpolation) and 4 and 10; long-range forces and energy against the
+  oracle within the parity tests' FP32 tolerances (5e-6, 2e-6).
 * tile sort: tiles of a few particles, above the 512-thread switch, and above
   the shared-memory capacity (2,048); permutation bit-exact.
 """
@@ -21,8 +25,8 @@ import pytest
 torch = pytest.importorskip("torch")
 pytestmark = pytest.mark.gpu
 
-from esp_hoomd_b200 import native, systems  # noqa: E402
-from esp_hoomd_b200._lib import ESP_SHORT_RANGE  # noqa: E402
+from esp_hoomd_b200 import native, systems, tables  # noqa: E402
+from esp_hoomd_b200._lib import ESP_LONG_RANGE, ESP_SHORT_RANGE  # noqa: E402
 from oracle import esp_ref as R  # noqa: E402
 
 
@@ -141,3 +145,26 @@ def test_neighbour_rows_exclusions(per_mol, n_mol, L):
     rng = np.random.default_rng(per_mol)
     pos = np.mod(np.repeat(rng.uniform(0, L, (n_mol, 3)), per_mol, 0) + rng.normal(0, 0.3, (n_mol * per_mol, 3)), L)
     _check_lists(pos, (L, L, L), 2.0, 256, R.molecule_exclusions(n_mol, per_mol))
+
+
+@pytest.mark.parametrize("order", [4, 5, 6, 7, 8, 10])
+@pytest.mark.parametrize("n", [37, 700])
+def test_tile_shares(order, n):
+    rng = np.random.default_rng(order * 1000 + n)
+    L = 10.0
+    pos = rng.uniform(0, L, (n, 3))
+    pos[: 3 * n // 4] = rng.uniform(0, 3.0, (3 * n // 4, 3))  # most of them in one tile
+    pos = pos.astype(np.float32).astype(np.float64)
+    q = np.where(np.arange(n) % 2 == 0, 1.0, -1.0)
+    ctx = native.Context(native.make_params(order=order, mesh=(24, 24, 24)), (L, L, L), n)
+    inf = ctx.info()
+    p4 = torch.zeros((n, 4), device="cuda")
+    p4[:, :3] = torch.as_tensor(pos, device="cuda")
+    force = torch.zeros((n, 4), device="cuda")
+    ctx.compute(p4, torch.as_tensor(q, dtype=torch.float32, device="cuda"), force, flags=ESP_LONG_RANGE)
+    prm = tables.ESPParams(mesh=(24, 24, 24), box=(L, L, L), rcut=inf["rcut"],
+                           split=tables.split_cached(inf["c_split"]),
+                           window=tables.window_cached(inf["order"], inf["c_window"], inf["window_degree"]))
+    empty = (np.zeros(n, np.uint32), np.zeros(n, np.uint32), np.zeros(0, np.uint32))
+    _, F, _ = R.esp(pos, q, prm, nlist=empty)
+    assert R.rel_rms(force.double().cpu().numpy()[:, :3], F) <= 5e-6
