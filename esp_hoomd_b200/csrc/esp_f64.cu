@@ -17,7 +17,8 @@
 //   k64_interp              : one CTA per tile, the tile's potential region
 //                             staged in shared memory, eight lanes per
 //                             particle over the stencil rows;
-//   k64_pair, k64_exclusions : as the FP32 kernels, in FP64.
+//   k64_pair, k64_exclusions : as the FP32 kernels, in FP64; the pair term runs
+//                             beside the mesh part.
 // Reference stages: src/ESPForceComputeGPU.cu:157-471 (K1-K7).
 #include <algorithm>
 
@@ -674,27 +675,30 @@ static cudaError_t launch64_interp_p(const Launch64& b, cudaStream_t st) {
 }
 
 // ----------------------------------------------------------------------------
-// pair term (EvaluatorPairPSWF, src/EvaluatorPairPSWF.h:274-295) in FP64:
-// 8 lanes per particle over its neighbour row
+// pair term (EvaluatorPairPSWF, src/EvaluatorPairPSWF.h:274-295) in FP64: TPP
+// lanes per particle over its neighbour row, one neighbour per lane and step.
+// Bound by the FP64 pipe (two series of NQ terms, the reciprocal root and about
+// 30 more operations per pair): the series are unrolled with their coefficients
+// as kernel parameters (constant-bank operands). Read from shared memory in a
+// loop of run-time length, the load, the counter and the branch of each term
+// took as many issue slots as its arithmetic (98,304 water charges, virial: 352
+// us per evaluation, now 280).
 // ----------------------------------------------------------------------------
-// without the virial: 64 registers, four CTAs per SM (measured 1-2% faster than 72 and three)
-template <bool VIR>
+template <int TPP, int NQ, bool VIR>
 __global__ void __launch_bounds__(256, VIR ? 3 : 4)
     k64_pair(const int2* __restrict__ chunks, const SysDev* __restrict__ sys, const ParamSet* __restrict__ psets,
-             const double* __restrict__ qv, int nq, const double4* __restrict__ posq,
-             const uint32_t* __restrict__ head, const uint32_t* __restrict__ nn, const uint32_t* __restrict__ nlist,
-             double4* __restrict__ force, double* __restrict__ acc, int accumulate) {
+             const PairCoef64 pc, const double4* __restrict__ posq, const uint32_t* __restrict__ head,
+             const uint32_t* __restrict__ nn, const uint32_t* __restrict__ nlist, double4* __restrict__ force,
+             double* __restrict__ acc) {
     __shared__ double red[32 * 7];
-    __shared__ double sq[MAX_QC];  // split coefficients (nq <= MAX_QC, checked by the planner)
-    constexpr int TPP = 8;
-    const int2 ch = chunks[blockIdx.x];
-    const SysDev S = sys[ch.x];
+    constexpr int SUB = TPP / 8;  // CTAs per chunk of 32 particles
+    const int2 ch = chunks[blockIdx.x / SUB];
+    const SysDev& S = sys[ch.x];
     const ParamSet& ps = psets[S.pset];
     const double rc = ps.rcut_d, rc2 = rc * rc, irc = 1.0 / rc, irc2 = irc * irc, tirc3 = 2.0 * irc2 * irc;
-    const double iLx = 1.0 / S.Lxd, iLy = 1.0 / S.Lyd, iLz = 1.0 / S.Lzd;
-    for (int c = threadIdx.x; c < nq; c += blockDim.x) sq[c] = qv[c];
-    __syncthreads();
-    const int i = ch.y + threadIdx.x / TPP;
+    const double Lx = S.Lxd, Ly = S.Lyd, Lz = S.Lzd;
+    const double iLx = 1.0 / Lx, iLy = 1.0 / Ly, iLz = 1.0 / Lz;
+    const int i = ch.y + (blockIdx.x % SUB) * (256 / TPP) + threadIdx.x / TPP;
     const int sub = threadIdx.x % TPP;
     const bool valid = i < S.p_off + S.N;
     double fx = 0, fy = 0, fz = 0, en = 0, v[6] = {0, 0, 0, 0, 0, 0};
@@ -704,19 +708,20 @@ __global__ void __launch_bounds__(256, VIR ? 3 : 4)
         // minimum image by the reciprocal box length; a pair that it could image
         // differently from a division sits at |d| = L/2 > r_c
         if (wrap) {
-            dx -= S.Lxd * rint(dx * iLx);
-            dy -= S.Lyd * rint(dy * iLy);
-            dz -= S.Lzd * rint(dz * iLz);
+            dx -= Lx * rint(dx * iLx);
+            dy -= Ly * rint(dy * iLy);
+            dz -= Lz * rint(dz * iLz);
         }
         const double r2 = dx * dx + dy * dy + dz * dz;
         if (r2 < rc2 && r2 > 0.0) {
             const double ri = rsqrt(r2);
             const double vv = fma(2.0 * irc2, r2, -1.0);
-            // Q(v) and dQ/dv in one Horner pass over the staged coefficients
-            double Q = sq[nq - 1], dQ = 0.0;
-            for (int c = nq - 2; c >= 0; --c) {
+            // Q(v) and dQ/dv in one Horner pass
+            double Q = pc.q[NQ - 1], dQ = 0.0;
+#pragma unroll
+            for (int c = NQ - 2; c >= 0; --c) {
                 dQ = fma(dQ, vv, Q);
-                Q = fma(Q, vv, sq[c]);
+                Q = fma(Q, vv, pc.q[c]);
             }
             dQ *= 2.0;  // dQ/du = 2 dQ/dv
             const double qq = pi.w * pj.w * INV_4PI_D;
@@ -738,8 +743,8 @@ __global__ void __launch_bounds__(256, VIR ? 3 : 4)
     // particles at least r_c from every face (posq holds wrapped positions)
     // see every in-cutoff neighbour in the same image: a warp whose particles
     // all are skips the minimum-image wrap (pairs beyond r_c stay masked)
-    const bool inner = !valid || (pi.x >= rc && pi.x <= S.Lxd - rc && pi.y >= rc && pi.y <= S.Lyd - rc &&
-                                  pi.z >= rc && pi.z <= S.Lzd - rc);
+    const bool inner = !valid || (pi.x >= rc && pi.x <= Lx - rc && pi.y >= rc && pi.y <= Ly - rc && pi.z >= rc &&
+                                  pi.z <= Lz - rc);
     const bool interior = __all_sync(0xffffffffu, inner);
     if (valid) {
         // one neighbour per lane and step: streaming 16-byte index segments
@@ -768,12 +773,7 @@ __global__ void __launch_bounds__(256, VIR ? 3 : 4)
         en += __shfl_xor_sync(0xffffffffu, en, o);
     }
     if (valid && sub == 0) {
-        double4 f = accumulate ? force[i] : make_double4(0.0, 0.0, 0.0, 0.0);
-        f.x += fx;
-        f.y += fy;
-        f.z += fz;
-        f.w += 0.5 * en;
-        force[i] = f;
+        force[i] = make_double4(fx, fy, fz, 0.5 * en);
     }
     if (VIR) {
         double e[7] = {sub == 0 ? 0.5 * en : 0.0, 0.5 * v[0], 0.5 * v[1], 0.5 * v[2],
@@ -788,6 +788,37 @@ __global__ void __launch_bounds__(256, VIR ? 3 : 4)
         block_sum_f64<1>(e, red);
         if (threadIdx.x == 0) atomicAdd(&acc[ch.x * ACC_STRIDE + ACC_E], e[0]);
     }
+}
+
+template <int TPP, bool VIR>
+static void launch64_pair_t(const Launch64& b, double4* force, cudaStream_t st) {
+    const LaunchArgs& a = b.a;
+    const int grid = b.n_pchunks * (TPP / 8);
+    // the series padded with zero terms to the next compiled length
+#define ESPB_PAIR64(NQ)                                                                                       \
+    k64_pair<TPP, NQ, VIR><<<grid, 256, 0, st>>>(b.pchunks, a.sys, a.psets, b.pc, b.posq, a.nl_head, a.nl_n, \
+                                                 a.nl_list, force, a.acc)
+    if (b.nq <= 12) ESPB_PAIR64(12);
+    else if (b.nq <= 14) ESPB_PAIR64(14);
+    else if (b.nq <= 16) ESPB_PAIR64(16);
+    else if (b.nq <= 17) ESPB_PAIR64(17);
+    else if (b.nq <= 18) ESPB_PAIR64(18);
+    else if (b.nq <= 19) ESPB_PAIR64(19);
+    else if (b.nq <= 20) ESPB_PAIR64(20);
+    else if (b.nq <= 22) ESPB_PAIR64(22);
+    else if (b.nq <= 24) ESPB_PAIR64(24);
+    else ESPB_PAIR64(32);
+#undef ESPB_PAIR64
+}
+
+// A warp per particle while 8 lanes would leave SMs without a CTA (32 particles
+// each): 1,000 ions, 16.5 us per launch with 8 lanes, 6.5 with 32.
+cudaError_t launch64_pair(const Launch64& b, double4* force, cudaStream_t st) {
+    if (b.n_pchunks == 0) return cudaSuccess;
+    const bool wide = b.n_pchunks <= 148, vir = b.a.want_virial;
+    if (wide) vir ? launch64_pair_t<32, true>(b, force, st) : launch64_pair_t<32, false>(b, force, st);
+    else vir ? launch64_pair_t<8, true>(b, force, st) : launch64_pair_t<8, false>(b, force, st);
+    return cudaGetLastError();
 }
 
 // exclusion correction (src/ESPForceComputeGPU.cu:391-471) in FP64: removes
@@ -875,44 +906,59 @@ cudaError_t launch64_configure(int P, int T) {
     ESPB_DISPATCH_P(configure64_interp_p, P, T);
 }
 
-cudaError_t launch64_eval(const Launch64& b, cudaStream_t st) {
+// force += add (the concurrently computed pair forces and energies)
+__global__ void __launch_bounds__(256)
+    k64_add_forces(const int2* __restrict__ chunks, const SysDev* __restrict__ sys, const double4* __restrict__ add,
+                   double4* __restrict__ force) {
+    const int2 ch = chunks[blockIdx.x];
+    const int i = ch.y + threadIdx.x;
+    if (i >= sys[ch.x].p_off + sys[ch.x].N) return;
+    const double4 b = add[i];
+    double4 f = force[i];
+    f.x += b.x;
+    f.y += b.y;
+    f.z += b.z;
+    f.w += b.w;
+    force[i] = f;
+}
+
+cudaError_t launch64_bin(const Launch64& b, cudaStream_t st) {
     const LaunchArgs& a = b.a;
-    const bool lr = b.long_range, sr = b.short_range;
     if (a.n_chunks)
         k64_bin<<<a.n_chunks, 256, 0, st>>>(a.chunks, a.sys, a.P, a.T, b.pos_in, b.q_in, b.posq, b.trec, a.rel,
                                             a.key, a.tile_count, a.acc);
-    if (lr) {
-        cudaError_t e = launch_scan(a.tile_count, a.tile_start, a.n_tiles, a.scan_ws, st);
-        if (e != cudaSuccess) return e;
-        e = launch_scatter(a.chunks, a.n_chunks, a.sys, a.key, a.tile_start, a.tile_count, a.perm_u, st);
-        if (e != cudaSuccess) return e;
-        if (a.n_tiles) {
-            k64_tile_sort<<<a.n_tiles, 256, 0, st>>>(a.tile_start, a.perm_u, a.perm, b.trec, a.rel, b.srec, a.srel);
-            k64_spread<<<dim3(a.n_tiles, split64(a.n_tiles)), K64S_THREADS, spread64_smem(a.P, a.T), st>>>(
-                a.tile_sys, a.sys, b.wcoef, a.P, a.T, a.D, a.tile_start, b.srec, a.srel, a.rho);
-        }
-        if (b.n_xl) k64_fft_pass<0><<<b.n_xl, F64_WARPS * 32, 0, st>>>(b.xl, a.sys, b.tw, b.cbuf, a.rho, b.phi, b.gtab, a.acc);
-        if (b.n_yl) k64_fft_pass<1><<<b.n_yl, F64_WARPS * 32, 0, st>>>(b.yl, a.sys, b.tw, b.cbuf, a.rho, b.phi, b.gtab, a.acc);
-        if (b.n_zl) k64_fft_pass<2><<<b.n_zl, F64_WARPS * 32, 0, st>>>(b.zl, a.sys, b.tw, b.cbuf, a.rho, b.phi, b.gtab, a.acc);
-        if (b.n_yl) k64_fft_pass<3><<<b.n_yl, F64_WARPS * 32, 0, st>>>(b.yl, a.sys, b.tw, b.cbuf, a.rho, b.phi, b.gtab, a.acc);
-        if (b.n_xl) k64_fft_pass<4><<<b.n_xl, F64_WARPS * 32, 0, st>>>(b.xl, a.sys, b.tw, b.cbuf, a.rho, b.phi, b.gtab, a.acc);
-        if (a.n_tiles) {
-            e = [&]() -> cudaError_t { ESPB_DISPATCH_P(launch64_interp_p, a.P, b, st); }();
-            if (e != cudaSuccess) return e;
-        }
-        if (a.n_chunks && a.ex_n)
-            k64_exclusions<<<a.n_chunks, 256, 0, st>>>(a.chunks, a.sys, a.psets, b.qv, b.nq, b.posq, a.ex_n,
-                                                       a.ex_list, a.ex_pitch, b.force, a.acc);
+    return cudaGetLastError();
+}
+
+cudaError_t launch64_add_forces(const Launch64& b, const double4* add, cudaStream_t st) {
+    const LaunchArgs& a = b.a;
+    if (a.n_chunks) k64_add_forces<<<a.n_chunks, 256, 0, st>>>(a.chunks, a.sys, add, b.force);
+    return cudaGetLastError();
+}
+
+cudaError_t launch64_mesh(const Launch64& b, cudaStream_t st) {
+    const LaunchArgs& a = b.a;
+    cudaError_t e = launch_scan(a.tile_count, a.tile_start, a.n_tiles, a.scan_ws, st);
+    if (e != cudaSuccess) return e;
+    e = launch_scatter(a.chunks, a.n_chunks, a.sys, a.key, a.tile_start, a.tile_count, a.perm_u, st);
+    if (e != cudaSuccess) return e;
+    if (a.n_tiles) {
+        k64_tile_sort<<<a.n_tiles, 256, 0, st>>>(a.tile_start, a.perm_u, a.perm, b.trec, a.rel, b.srec, a.srel);
+        k64_spread<<<dim3(a.n_tiles, split64(a.n_tiles)), K64S_THREADS, spread64_smem(a.P, a.T), st>>>(
+            a.tile_sys, a.sys, b.wcoef, a.P, a.T, a.D, a.tile_start, b.srec, a.srel, a.rho);
     }
-    if (sr && b.n_pchunks)
-    {
-        if (a.want_virial)
-            k64_pair<true><<<b.n_pchunks, 256, 0, st>>>(b.pchunks, a.sys, a.psets, b.qv, b.nq, b.posq, a.nl_head,
-                                                        a.nl_n, a.nl_list, b.force, a.acc, lr ? 1 : 0);
-        else
-            k64_pair<false><<<b.n_pchunks, 256, 0, st>>>(b.pchunks, a.sys, a.psets, b.qv, b.nq, b.posq, a.nl_head,
-                                                         a.nl_n, a.nl_list, b.force, a.acc, lr ? 1 : 0);
+    if (b.n_xl) k64_fft_pass<0><<<b.n_xl, F64_WARPS * 32, 0, st>>>(b.xl, a.sys, b.tw, b.cbuf, a.rho, b.phi, b.gtab, a.acc);
+    if (b.n_yl) k64_fft_pass<1><<<b.n_yl, F64_WARPS * 32, 0, st>>>(b.yl, a.sys, b.tw, b.cbuf, a.rho, b.phi, b.gtab, a.acc);
+    if (b.n_zl) k64_fft_pass<2><<<b.n_zl, F64_WARPS * 32, 0, st>>>(b.zl, a.sys, b.tw, b.cbuf, a.rho, b.phi, b.gtab, a.acc);
+    if (b.n_yl) k64_fft_pass<3><<<b.n_yl, F64_WARPS * 32, 0, st>>>(b.yl, a.sys, b.tw, b.cbuf, a.rho, b.phi, b.gtab, a.acc);
+    if (b.n_xl) k64_fft_pass<4><<<b.n_xl, F64_WARPS * 32, 0, st>>>(b.xl, a.sys, b.tw, b.cbuf, a.rho, b.phi, b.gtab, a.acc);
+    if (a.n_tiles) {
+        e = [&]() -> cudaError_t { ESPB_DISPATCH_P(launch64_interp_p, a.P, b, st); }();
+        if (e != cudaSuccess) return e;
     }
+    if (a.n_chunks && a.ex_n)
+        k64_exclusions<<<a.n_chunks, 256, 0, st>>>(a.chunks, a.sys, a.psets, b.qv, b.nq, b.posq, a.ex_n,
+                                                   a.ex_list, a.ex_pitch, b.force, a.acc);
     return cudaGetLastError();
 }
 

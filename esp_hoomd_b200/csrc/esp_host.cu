@@ -324,12 +324,13 @@ struct esp_batch {
     // second stream for the concurrent pair term, its force array and the
     // fork/join events (created at plan time, kept across re-plans)
     cudaStream_t st2 = nullptr;
+    cudaStream_t st_mesh64 = nullptr;  // the FP64 mode's mesh part, of higher priority
     cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
     float4* d_fsr = nullptr;
     // FP64 mode: tables, records, spectrum and work lists
     bool f64 = false;
     DevAlloc mem64;
-    double4 *d_posq64 = nullptr, *d_trec64 = nullptr, *d_srec64 = nullptr;
+    double4 *d_posq64 = nullptr, *d_trec64 = nullptr, *d_srec64 = nullptr, *d_fsr64 = nullptr;
     double *d_w64 = nullptr, *d_q64 = nullptr, *d_phi64 = nullptr;
     double2 *d_tw64 = nullptr, *d_cbuf = nullptr, *d_gtab64 = nullptr;
     int2 *d_pch64 = nullptr, *d_xl = nullptr, *d_yl = nullptr, *d_zl = nullptr;
@@ -390,6 +391,10 @@ struct esp_batch {
         if (st2) {
             cudaStreamSynchronize(st2);
             cudaStreamDestroy(st2);
+        }
+        if (st_mesh64) {
+            cudaStreamSynchronize(st_mesh64);
+            cudaStreamDestroy(st_mesh64);
         }
         if (ev_fork) cudaEventDestroy(ev_fork);
         if (ev_join) cudaEventDestroy(ev_join);
@@ -794,11 +799,17 @@ int esp_batch::plan64(const std::vector<float2>& tw, long long g_total) {
     n_zl = (int)zl.size();
     int rc = 0;
     if ((rc = mem64.get(d_posq64, totN)) || (rc = mem64.get(d_trec64, totN)) || (rc = mem64.get(d_srec64, totN)) ||
+        (rc = mem64.get(d_fsr64, totN)) ||
         (rc = mem64.get(d_w64, w64.size())) || (rc = mem64.get(d_q64, q64.size())) || (rc = mem64.get(d_phi64, M)) ||
         (rc = mem64.get(d_tw64, tw64.size())) || (rc = mem64.get(d_cbuf, M)) || (rc = mem64.get(d_gtab64, g_total)) ||
         (rc = mem64.get(d_pch64, pch.size())) || (rc = mem64.get(d_xl, xl.size())) || (rc = mem64.get(d_yl, yl.size())) ||
         (rc = mem64.get(d_zl, zl.size())))
         return rc;
+    if (!st_mesh64) {
+        int least = 0, greatest = 0;
+        ESPB_CK(cudaDeviceGetStreamPriorityRange(&least, &greatest));
+        ESPB_CK(cudaStreamCreateWithPriority(&st_mesh64, cudaStreamNonBlocking, greatest));
+    }
     ESPB_CK(cudaMemcpy(d_w64, w64.data(), w64.size() * sizeof(double), cudaMemcpyHostToDevice));
     ESPB_CK(cudaMemcpy(d_q64, q64.data(), q64.size() * sizeof(double), cudaMemcpyHostToDevice));
     ESPB_CK(cudaMemcpy(d_tw64, tw64.data(), tw64.size() * sizeof(double2), cudaMemcpyHostToDevice));
@@ -835,9 +846,8 @@ int esp_batch::compute_f64(cudaStream_t st, const double* pos4, const double* q,
     a.ex_n = ex_n;
     a.ex_list = ex_list;
     a.ex_pitch = ex_pitch;
-    b.long_range = flags & ESP_LONG_RANGE;
-    b.short_range = flags & ESP_SHORT_RANGE;
-    a.add_bg = b.long_range ? 1 : 0;
+    const bool lr = flags & ESP_LONG_RANGE, sr = flags & ESP_SHORT_RANGE;
+    a.add_bg = lr ? 1 : 0;
     b.pos_in = reinterpret_cast<const double4*>(pos4);
     b.q_in = q;
     b.posq = d_posq64;
@@ -847,6 +857,7 @@ int esp_batch::compute_f64(cudaStream_t st, const double* pos4, const double* q,
     b.wcoef = d_w64;
     b.qv = d_q64;
     b.nq = nq64;
+    for (int c = 0; c < MAX_QC; ++c) b.pc.q[c] = c < nq64 ? psh[0].split.qv[c] : 0.0;
     b.tw = d_tw64;
     b.cbuf = d_cbuf;
     b.phi = d_phi64;
@@ -860,9 +871,27 @@ int esp_batch::compute_f64(cudaStream_t st, const double* pos4, const double* q,
     b.n_yl = n_yl;
     b.n_zl = n_zl;
     ESPB_CK(cudaMemsetAsync(d_acc, 0, (size_t)nsys * ACC_STRIDE * sizeof(double), st));
-    ESPB_CK(launch64_eval(b, st));
-    if (!b.long_range)  // the bin stage counted particles per tile; clear for the next call
+    ESPB_CK(launch64_bin(b, st));
+    if (lr && sr) {
+        // the pair term, bound by the FP64 pipe, beside the mesh kernels, bound
+        // by latency: those run on a stream of higher priority, so that their
+        // CTAs start as soon as pair CTAs end and the pair term fills what they
+        // leave (98,304 water charges: 552 us per evaluation, one after the
+        // other 593, the pair term's CTAs first 589)
+        ESPB_CK(cudaEventRecord(ev_fork, st));
+        ESPB_CK(cudaStreamWaitEvent(st_mesh64, ev_fork, 0));
+        ESPB_CK(launch64_mesh(b, st_mesh64));
+        ESPB_CK(cudaEventRecord(ev_join, st_mesh64));
+        ESPB_CK(launch64_pair(b, d_fsr64, st));
+        ESPB_CK(cudaStreamWaitEvent(st, ev_join, 0));
+        ESPB_CK(launch64_add_forces(b, d_fsr64, st));
+    } else if (lr) {
+        ESPB_CK(launch64_mesh(b, st));
+    } else {
+        ESPB_CK(launch64_pair(b, b.force, st));
+        // the bin stage counted particles per tile; clear for the next call
         ESPB_CK(cudaMemsetAsync(d_tcount, 0, (size_t)n_tiles * sizeof(uint32_t), st));
+    }
     ESPB_CK(launch_finalize(a, st));
     return 0;
 }

@@ -142,9 +142,12 @@ cudaError_t launch_add_forces(const int2* chunks, int n_chunks, const SysDev* sy
 // FP64 mode (esp_f64.cu): the shared fields of `a` (descriptors, chunks,
 // tiles, keys, permutation, charge mesh, accumulators, neighbour list,
 // exclusions) plus the FP64 arrays.
+struct PairCoef64 {
+    double q[MAX_QC];  // Q(v), zero past nq
+};
 struct Launch64 {
     LaunchArgs a;
-    bool long_range = true, short_range = true;
+    PairCoef64 pc{};                // split Q(v) as kernel parameters (the pair term)
     const double4* pos_in = nullptr;
     const double* q_in = nullptr;
     double4 *posq = nullptr, *trec = nullptr, *srec = nullptr, *force = nullptr;
@@ -162,7 +165,12 @@ struct Launch64 {
 };
 size_t spread64_smem(int P, int T);
 cudaError_t launch64_configure(int P, int T);
-cudaError_t launch64_eval(const Launch64& b, cudaStream_t st);
+// the stages of an evaluation: binning, the mesh part (sort to interpolation and
+// exclusions) and the pair term, which writes `force`
+cudaError_t launch64_bin(const Launch64& b, cudaStream_t st);
+cudaError_t launch64_mesh(const Launch64& b, cudaStream_t st);
+cudaError_t launch64_pair(const Launch64& b, double4* force, cudaStream_t st);
+cudaError_t launch64_add_forces(const Launch64& b, const double4* add, cudaStream_t st);
 cudaError_t launch_influence64(const SysDev& S, const double* w1d, const double* tq, const double* wq, int nq,
                                double rcut, double psi_floor, double2* gtab, cudaStream_t st);
 cudaError_t launch_finalize(const LaunchArgs& a, cudaStream_t st);

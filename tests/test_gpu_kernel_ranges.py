@@ -16,6 +16,10 @@ where the rule switches, against the oracle.
   full, nearly empty and empty tiles at once, supports 5..8 (the rotated walk
   of the interpolation) and 4 and 10; long-range forces and energy against the
   oracle within the parity tests' FP32 tolerances (5e-6, 2e-6).
+* FP64 pair term: a warp per particle up to 148 chunks of 32 particles, 8 lanes
+  above, with and without the virial, on the last size of the one and the first
+  of the other; against the oracle within the FP64 tests' tolerances (forces
+  1e-8, energy 1e-10, virial 2e-8, the oracle's own finite difference).
 * tile sort: tiles of a few particles, above the 512-thread switch, and above
   the shared-memory capacity (2,048); permutation bit-exact.
 """
@@ -168,3 +172,28 @@ def test_tile_shares(order, n):
     empty = (np.zeros(n, np.uint32), np.zeros(n, np.uint32), np.zeros(0, np.uint32))
     _, F, _ = R.esp(pos, q, prm, nlist=empty)
     assert R.rel_rms(force.double().cpu().numpy()[:, :3], F) <= 5e-6
+
+
+@pytest.mark.parametrize("shape", [(16, 16, 18), (18, 17, 16)])  # 4,608 and 4,896 ions
+@pytest.mark.parametrize("virial", [False, True])
+def test_fp64_pair_lane_counts(shape, virial):
+    s = systems.rocksalt(0, seed=sum(shape), shape=shape)
+    s.pos = s.pos.astype(np.float32).astype(np.float64)
+    nlist = R.neighbor_list(s.pos, s.box, 3.0)
+    ctx = native.Context(native.make_params(mesh=(32, 32, 32), precision=1), s.box, s.N)
+    inf = ctx.info()
+    pos = torch.zeros((s.N, 4), dtype=torch.float64, device="cuda")
+    pos[:, :3] = torch.as_tensor(s.pos, device="cuda")
+    nl = tuple(torch.as_tensor(a.astype(np.int32), device="cuda") for a in nlist)
+    force = torch.zeros_like(pos)
+    energy = torch.zeros(1, dtype=torch.float64, device="cuda")
+    w = torch.zeros(6, dtype=torch.float64, device="cuda") if virial else None
+    ctx.compute_f64(pos, torch.as_tensor(s.q, dtype=torch.float64, device="cuda"), force, energy, w, nlist=nl)
+    prm = tables.ESPParams(mesh=(32, 32, 32), box=tuple(s.box), rcut=inf["rcut"],
+                           split=tables.make_split(inf["c_split"], tol=1e-12),
+                           window=tables.window_cached(inf["order"], inf["c_window"], inf["window_degree"]))
+    E, F, W = R.esp(s.pos, s.q, prm, nlist=nlist)
+    assert R.rel_rms(force.cpu().numpy()[:, :3], F) <= 1e-8
+    assert abs(energy.item() - E) <= 1e-10 * abs(E)
+    if virial:
+        assert np.abs(w.cpu().numpy() - W).max() <= 2e-8 * np.abs(W).max()
