@@ -45,12 +45,12 @@ CAP = 256
 DT = 0.002
 MD_STEPS = 10
 # kernels per launch group (used to count launches in the timed region)
-# bin, scan, scatter, tile_sort, spread, interp, pair, add_forces (the pair
-# term runs on a second stream into its own array), finalize; plus the FFT
-# passes: 3 whole-plane/slab kernels (fft_mode 0) or 5 per-line kernels
+# bin, scan (two kernels over this many tiles), scatter, tile_sort, spread,
+# interp, pair, add_finalize (the pair term runs on a second stream into its
+# own array); plus the FFT passes: 3 whole-plane/slab kernels (fft_mode 0) or 5 per-line kernels
 K_EVAL_BASE = 9
 K_FFT = {0: 3, 1: 5}
-K_NLIST = 5      # cell_bin, scan, scatter, cell_sort, nlist
+K_NLIST = 6      # cell_bin, scan (two kernels), scatter, cell_sort, nlist
 K_NVE = 2
 
 

@@ -24,6 +24,7 @@
 
 #include "esp_common.cuh"
 #include "esp_kernels.h"
+#include "esp_launch.cuh"
 
 namespace espb {
 
@@ -95,6 +96,7 @@ __global__ void k64_tile_sort(const uint32_t* __restrict__ start, const uint32_t
                               uint32_t* __restrict__ perm, const double4* __restrict__ trec,
                               const uint32_t* __restrict__ rel, double4* __restrict__ srec,
                               uint32_t* __restrict__ srel) {
+    after_previous();
     __shared__ uint32_t sm[SORT_CAP];
     const uint32_t s0 = start[blockIdx.x];
     const uint32_t n = start[blockIdx.x + 1] - s0;
@@ -168,6 +170,7 @@ __global__ void __launch_bounds__(K64S_THREADS)
     k64_spread(const int* __restrict__ tile_sys, const SysDev* __restrict__ sys, const double* __restrict__ wcoef,
                int P, int T, int D, const uint32_t* __restrict__ start, const double4* __restrict__ srec,
                const uint32_t* __restrict__ srel, double* __restrict__ rho) {
+    after_previous();
     // [E^2][ES] region | [K64S_CH][K64S_SEG] x segments | [K64S_CH][2P] y, z weights | [P][D+1] window
     // | [K64S_CH] origins | row and column offsets
     extern __shared__ double sreg[];
@@ -379,6 +382,7 @@ __global__ void __launch_bounds__(F64_WARPS * 32)
     k64_fft_pass(const int2* __restrict__ items, const SysDev* __restrict__ sys, const double2* __restrict__ tw,
                  double2* __restrict__ cbuf, double* __restrict__ rho, double* __restrict__ phi,
                  const double2* __restrict__ gtab, double* __restrict__ acc) {
+    after_previous();
     __shared__ double2 sb[F64_WARPS][2][FFT_MAX_N];
     __shared__ double2 stw[FFT_MAX_N];
     __shared__ long long lbase[F64_WARPS];
@@ -549,6 +553,7 @@ __global__ void __launch_bounds__(K64I_WARPS * 32)
                const uint32_t* __restrict__ perm, const double4* __restrict__ srec,
                const uint32_t* __restrict__ srel, const double* __restrict__ phi, double4* __restrict__ force,
                double* __restrict__ acc) {
+    after_previous();
     extern __shared__ double sreg[];  // [E^2][ES] potential region, [P][D+1] window, row and column offsets
     __shared__ double red[32];
     __shared__ double wsh[K64I_WARPS * K64I_PPW][6 * P];  // W x | y | z, then dW x | y | z
@@ -669,8 +674,7 @@ static cudaError_t launch64_interp_p(const Launch64& b, cudaStream_t st) {
     const LaunchArgs& a = b.a;
     // several CTAs per tile when the tiles are few, each staging the region
     // and taking a share of its particles
-    k64_interp<P><<<dim3(a.n_tiles, split64(a.n_tiles)), K64I_WARPS * 32, interp64_smem(a.P, a.T), st>>>(
-        a.tile_sys, a.sys, a.psets, b.wcoef, a.T, a.D, a.tile_start, a.perm, b.srec, a.srel, b.phi, b.force, a.acc);
+    launch_after(a.overlap, k64_interp<P>, dim3(a.n_tiles, split64(a.n_tiles)), K64I_WARPS * 32, interp64_smem(a.P, a.T), st, a.tile_sys, a.sys, a.psets, b.wcoef, a.T, a.D, a.tile_start, a.perm, b.srec, a.srel, b.phi, b.force, a.acc);
     return cudaGetLastError();
 }
 
@@ -828,6 +832,7 @@ __global__ void k64_exclusions(const int2* __restrict__ chunks, const SysDev* __
                                const double4* __restrict__ posq, const uint32_t* __restrict__ n_ex,
                                const uint32_t* __restrict__ ex_list, int ex_pitch, double4* __restrict__ force,
                                double* __restrict__ acc) {
+    after_previous();
     __shared__ double red[32 * 7];
     const int2 ch = chunks[blockIdx.x];
     const SysDev S = sys[ch.x];
@@ -906,22 +911,6 @@ cudaError_t launch64_configure(int P, int T) {
     ESPB_DISPATCH_P(configure64_interp_p, P, T);
 }
 
-// force += add (the concurrently computed pair forces and energies)
-__global__ void __launch_bounds__(256)
-    k64_add_forces(const int2* __restrict__ chunks, const SysDev* __restrict__ sys, const double4* __restrict__ add,
-                   double4* __restrict__ force) {
-    const int2 ch = chunks[blockIdx.x];
-    const int i = ch.y + threadIdx.x;
-    if (i >= sys[ch.x].p_off + sys[ch.x].N) return;
-    const double4 b = add[i];
-    double4 f = force[i];
-    f.x += b.x;
-    f.y += b.y;
-    f.z += b.z;
-    f.w += b.w;
-    force[i] = f;
-}
-
 cudaError_t launch64_bin(const Launch64& b, cudaStream_t st) {
     const LaunchArgs& a = b.a;
     if (a.n_chunks)
@@ -930,34 +919,27 @@ cudaError_t launch64_bin(const Launch64& b, cudaStream_t st) {
     return cudaGetLastError();
 }
 
-cudaError_t launch64_add_forces(const Launch64& b, const double4* add, cudaStream_t st) {
-    const LaunchArgs& a = b.a;
-    if (a.n_chunks) k64_add_forces<<<a.n_chunks, 256, 0, st>>>(a.chunks, a.sys, add, b.force);
-    return cudaGetLastError();
-}
-
 cudaError_t launch64_mesh(const Launch64& b, cudaStream_t st) {
     const LaunchArgs& a = b.a;
-    cudaError_t e = launch_scan(a.tile_count, a.tile_start, a.n_tiles, a.scan_ws, st);
+    cudaError_t e = launch_scan(a.tile_count, a.tile_start, a.n_tiles, a.scan_ws, st, a.overlap);
     if (e != cudaSuccess) return e;
-    e = launch_scatter(a.chunks, a.n_chunks, a.sys, a.key, a.tile_start, a.tile_count, a.perm_u, st);
+    e = launch_scatter(a.chunks, a.n_chunks, a.sys, a.key, a.tile_start, a.tile_count, a.perm_u, st, a.overlap);
     if (e != cudaSuccess) return e;
     if (a.n_tiles) {
-        k64_tile_sort<<<a.n_tiles, 256, 0, st>>>(a.tile_start, a.perm_u, a.perm, b.trec, a.rel, b.srec, a.srel);
-        k64_spread<<<dim3(a.n_tiles, split64(a.n_tiles)), K64S_THREADS, spread64_smem(a.P, a.T), st>>>(
-            a.tile_sys, a.sys, b.wcoef, a.P, a.T, a.D, a.tile_start, b.srec, a.srel, a.rho);
+        launch_after(a.overlap, k64_tile_sort, a.n_tiles, 256, 0, st, a.tile_start, a.perm_u, a.perm, b.trec, a.rel, b.srec, a.srel);
+        launch_after(a.overlap, k64_spread, dim3(a.n_tiles, split64(a.n_tiles)), K64S_THREADS, spread64_smem(a.P, a.T), st, a.tile_sys, a.sys, b.wcoef, a.P, a.T, a.D, a.tile_start, b.srec, a.srel, a.rho);
     }
-    if (b.n_xl) k64_fft_pass<0><<<b.n_xl, F64_WARPS * 32, 0, st>>>(b.xl, a.sys, b.tw, b.cbuf, a.rho, b.phi, b.gtab, a.acc);
-    if (b.n_yl) k64_fft_pass<1><<<b.n_yl, F64_WARPS * 32, 0, st>>>(b.yl, a.sys, b.tw, b.cbuf, a.rho, b.phi, b.gtab, a.acc);
-    if (b.n_zl) k64_fft_pass<2><<<b.n_zl, F64_WARPS * 32, 0, st>>>(b.zl, a.sys, b.tw, b.cbuf, a.rho, b.phi, b.gtab, a.acc);
-    if (b.n_yl) k64_fft_pass<3><<<b.n_yl, F64_WARPS * 32, 0, st>>>(b.yl, a.sys, b.tw, b.cbuf, a.rho, b.phi, b.gtab, a.acc);
-    if (b.n_xl) k64_fft_pass<4><<<b.n_xl, F64_WARPS * 32, 0, st>>>(b.xl, a.sys, b.tw, b.cbuf, a.rho, b.phi, b.gtab, a.acc);
+    if (b.n_xl) launch_after(a.overlap, k64_fft_pass<0>, b.n_xl, F64_WARPS * 32, 0, st, b.xl, a.sys, b.tw, b.cbuf, a.rho, b.phi, b.gtab, a.acc);
+    if (b.n_yl) launch_after(a.overlap, k64_fft_pass<1>, b.n_yl, F64_WARPS * 32, 0, st, b.yl, a.sys, b.tw, b.cbuf, a.rho, b.phi, b.gtab, a.acc);
+    if (b.n_zl) launch_after(a.overlap, k64_fft_pass<2>, b.n_zl, F64_WARPS * 32, 0, st, b.zl, a.sys, b.tw, b.cbuf, a.rho, b.phi, b.gtab, a.acc);
+    if (b.n_yl) launch_after(a.overlap, k64_fft_pass<3>, b.n_yl, F64_WARPS * 32, 0, st, b.yl, a.sys, b.tw, b.cbuf, a.rho, b.phi, b.gtab, a.acc);
+    if (b.n_xl) launch_after(a.overlap, k64_fft_pass<4>, b.n_xl, F64_WARPS * 32, 0, st, b.xl, a.sys, b.tw, b.cbuf, a.rho, b.phi, b.gtab, a.acc);
     if (a.n_tiles) {
         e = [&]() -> cudaError_t { ESPB_DISPATCH_P(launch64_interp_p, a.P, b, st); }();
         if (e != cudaSuccess) return e;
     }
     if (a.n_chunks && a.ex_n)
-        k64_exclusions<<<a.n_chunks, 256, 0, st>>>(a.chunks, a.sys, a.psets, b.qv, b.nq, b.posq, a.ex_n,
+        launch_after(a.overlap, k64_exclusions, a.n_chunks, 256, 0, st, a.chunks, a.sys, a.psets, b.qv, b.nq, b.posq, a.ex_n,
                                                    a.ex_list, a.ex_pitch, b.force, a.acc);
     return cudaGetLastError();
 }

@@ -22,6 +22,7 @@
 #include "esp_b200.h"
 #include "esp_host_util.h"
 #include "esp_kernels.h"
+#include "esp_launch.cuh"
 #include "esp_md.h"
 #include "esp_tables.h"
 
@@ -717,6 +718,7 @@ int esp_batch::plan(const esp_params& p, int ns, const int* N_, const double* bo
     if (!pi.empty()) ESPB_CK(cudaMemcpy(d_p, pi.data(), pi.size() * sizeof(int2), cudaMemcpyHostToDevice));
     if (!si.empty()) ESPB_CK(cudaMemcpy(d_s, si.data(), si.size() * sizeof(int2), cudaMemcpyHostToDevice));
     ESPB_CK(cudaMemset(d_tcount, 0, n_tiles * sizeof(uint32_t)));
+    ESPB_CK(cudaMemset(d_acc, 0, (size_t)ns * ACC_STRIDE * sizeof(double)));
     ESPB_CK(cudaMemset(d_rho, 0, (size_t)std::max<long long>(m_off, 1) * sizeof(double)));
     drop_graphs();
     {
@@ -826,6 +828,18 @@ int esp_batch::plan64(const std::vector<float2>& tw, long long g_total) {
     return 0;
 }
 
+// The accumulators are zero between evaluations: the totals' kernel clears what
+// it has read, and an evaluation that ends before it clears them itself.
+struct AccGuard {
+    double* acc;
+    size_t bytes;
+    cudaStream_t st;
+    bool finalized = false;
+    ~AccGuard() {
+        if (!finalized) cudaMemsetAsync(acc, 0, bytes, st);
+    }
+};
+
 int esp_batch::compute_f64(cudaStream_t st, const double* pos4, const double* q, const unsigned* head,
                            const unsigned* nn, const unsigned* nl, double* force4, double* energy, double* virial,
                            int flags) {
@@ -837,6 +851,7 @@ int esp_batch::compute_f64(cudaStream_t st, const double* pos4, const double* q,
     Launch64 b;
     b.a = args();
     LaunchArgs& a = b.a;
+    a.overlap = overlap_starts(a.n_chunks, st);
     if (energy) a.energy = energy;
     if (virial) a.virial = virial;
     a.want_virial = virial != nullptr;
@@ -870,7 +885,7 @@ int esp_batch::compute_f64(cudaStream_t st, const double* pos4, const double* q,
     b.n_xl = n_xl;
     b.n_yl = n_yl;
     b.n_zl = n_zl;
-    ESPB_CK(cudaMemsetAsync(d_acc, 0, (size_t)nsys * ACC_STRIDE * sizeof(double), st));
+    AccGuard acc_guard{d_acc, (size_t)nsys * ACC_STRIDE * sizeof(double), st};
     ESPB_CK(launch64_bin(b, st));
     if (lr && sr) {
         // the pair term, bound by the FP64 pipe, beside the mesh kernels, bound
@@ -884,8 +899,11 @@ int esp_batch::compute_f64(cudaStream_t st, const double* pos4, const double* q,
         ESPB_CK(cudaEventRecord(ev_join, st_mesh64));
         ESPB_CK(launch64_pair(b, d_fsr64, st));
         ESPB_CK(cudaStreamWaitEvent(st, ev_join, 0));
-        ESPB_CK(launch64_add_forces(b, d_fsr64, st));
-    } else if (lr) {
+        ESPB_CK(launch_add_finalize(a, d_fsr64, b.force, st));
+        acc_guard.finalized = true;
+        return 0;
+    }
+    if (lr) {
         ESPB_CK(launch64_mesh(b, st));
     } else {
         ESPB_CK(launch64_pair(b, b.force, st));
@@ -893,6 +911,7 @@ int esp_batch::compute_f64(cudaStream_t st, const double* pos4, const double* q,
         ESPB_CK(cudaMemsetAsync(d_tcount, 0, (size_t)n_tiles * sizeof(uint32_t), st));
     }
     ESPB_CK(launch_finalize(a, st));
+    acc_guard.finalized = true;
     return 0;
 }
 
@@ -978,6 +997,7 @@ int esp_batch::compute(cudaStream_t st, const float* pos4, const float* q, const
     if ((flags & ESP_SHORT_RANGE) && use_pl && !pl_ready)
         return fail(ESP_ERR_INVALID, "no neighbour list given and no pair list built (esp_batch_build_pairlist)");
     LaunchArgs a = args();
+    a.overlap = overlap_starts(a.n_chunks, st);
     if ((flags & ESP_SHORT_RANGE) && use_pl) a.plist = &pl;
     a.pos_in = reinterpret_cast<const float4*>(pos4);
     a.q_in = q;
@@ -997,7 +1017,7 @@ int esp_batch::compute(cudaStream_t st, const float* pos4, const float* q, const
     const bool lr = flags & ESP_LONG_RANGE, sr = flags & ESP_SHORT_RANGE;
     a.accumulate = lr ? 1 : 0;
     a.add_bg = lr ? 1 : 0;
-    ESPB_CK(cudaMemsetAsync(d_acc, 0, (size_t)nsys * ACC_STRIDE * sizeof(double), st));
+    AccGuard acc_guard{d_acc, (size_t)nsys * ACC_STRIDE * sizeof(double), st};
     timer.begin(ESP_STAGE_BIN, st);
     ESPB_CK(launch_bin(a, st));
     timer.end(st);
@@ -1042,13 +1062,16 @@ int esp_batch::compute(cudaStream_t st, const float* pos4, const float* q, const
     }
     if (fork) {
         ESPB_CK(cudaStreamWaitEvent(st, ev_join, 0));
-        ESPB_CK(launch_add_forces(a.chunks, a.n_chunks, a.sys, d_fsr, a.force, st));
-    } else if (sr) {
-        timer.begin(ESP_STAGE_PAIR, st);
-        ESPB_CK(launch_pair(a, st));
-        timer.end(st);
+        ESPB_CK(launch_add_finalize(a, d_fsr, a.force, st));
+    } else {
+        if (sr) {
+            timer.begin(ESP_STAGE_PAIR, st);
+            ESPB_CK(launch_pair(a, st));
+            timer.end(st);
+        }
+        ESPB_CK(launch_finalize(a, st));
     }
-    ESPB_CK(launch_finalize(a, st));
+    acc_guard.finalized = true;
     return 0;
 }
 
@@ -1184,7 +1207,7 @@ int esp_batch::spread_only(cudaStream_t st, const float* pos4, const float* q, d
     long long M = 0;
     for (const SysDev& S : sd) M += (long long)S.nx * S.ny * S.nz;
     ESPB_CK(cudaMemsetAsync(rho_out, 0, (size_t)M * sizeof(double), st));
-    ESPB_CK(cudaMemsetAsync(d_acc, 0, (size_t)nsys * ACC_STRIDE * sizeof(double), st));
+    AccGuard acc_guard{d_acc, (size_t)nsys * ACC_STRIDE * sizeof(double), st};  // no totals: cleared on return
     LaunchArgs a = args();
     a.pos_in = reinterpret_cast<const float4*>(pos4);
     a.q_in = q;

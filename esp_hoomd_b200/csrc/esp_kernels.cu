@@ -21,6 +21,7 @@
 
 #include "esp_common.cuh"
 #include "esp_kernels.h"
+#include "esp_launch.cuh"
 
 namespace espb {
 
@@ -96,6 +97,7 @@ __global__ void k_bin(const int2* __restrict__ chunks, const SysDev* __restrict_
 constexpr int SCAN_PER = 16;
 
 __global__ void __launch_bounds__(1024) k_scan(const uint32_t* __restrict__ cnt, uint32_t* __restrict__ start, int n) {
+    after_previous();
     __shared__ uint32_t wsum[32];
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const bool vec = ((reinterpret_cast<uintptr_t>(cnt) | reinterpret_cast<uintptr_t>(start)) & 15u) == 0;
@@ -187,6 +189,7 @@ __device__ __forceinline__ uint32_t scan_load(const uint32_t* __restrict__ cnt, 
 }
 
 __global__ void __launch_bounds__(256) k_scan_sums(const uint32_t* __restrict__ cnt, uint32_t* __restrict__ ws, int n) {
+    after_previous();
     __shared__ uint32_t wsum[8];
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     uint32_t v[SCAN_PER];
@@ -205,6 +208,7 @@ __global__ void __launch_bounds__(256) k_scan_sums(const uint32_t* __restrict__ 
 
 __global__ void __launch_bounds__(256)
     k_scan_apply(const uint32_t* __restrict__ cnt, const uint32_t* __restrict__ ws, uint32_t* __restrict__ start, int n) {
+    after_previous();
     __shared__ uint32_t wsum[8], wpre[8];
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     uint32_t pre = 0;
@@ -255,6 +259,7 @@ __global__ void __launch_bounds__(256)
 __global__ void k_scatter(const int2* __restrict__ chunks, const SysDev* __restrict__ sys,
                           const uint32_t* __restrict__ key, const uint32_t* __restrict__ start,
                           uint32_t* __restrict__ cnt, uint32_t* __restrict__ perm_u) {
+    after_previous();
     const int2 ch = chunks[blockIdx.x];
     const SysDev S = sys[ch.x];
     const int i = ch.y + threadIdx.x;
@@ -290,6 +295,7 @@ __global__ void __launch_bounds__(512)
     k_tile_sort(const uint32_t* __restrict__ start, const uint32_t* __restrict__ perm_u, uint32_t* __restrict__ perm,
                 const float4* __restrict__ trec, const uint32_t* __restrict__ rel, float4* __restrict__ srec,
                 uint32_t* __restrict__ srel, const int* __restrict__ tile_sys, const SysDev* __restrict__ sys) {
+    after_previous();
     __shared__ uint32_t sm[SORT_CAP];
     __shared__ uint32_t cnt[SORT_BUCKETS], beg[SORT_BUCKETS];
     const uint32_t s0 = start[blockIdx.x];
@@ -375,6 +381,7 @@ __global__ void __launch_bounds__(SpreadCfg<P>::THREADS)
     k_spread(const int* __restrict__ tile_sys, const SysDev* __restrict__ sys, const ParamSet* __restrict__ psets,
              int T, int D, const uint32_t* __restrict__ start, const float4* __restrict__ srec,
              const uint32_t* __restrict__ srel, double* __restrict__ rho) {
+    after_previous();
     using C = SpreadCfg<P>;
     extern __shared__ float4 smem4[];
     const int t = blockIdx.x;
@@ -496,6 +503,7 @@ __global__ void __launch_bounds__(256)
     k_spread_dense(const int* __restrict__ tile_sys, const SysDev* __restrict__ sys,
                    const ParamSet* __restrict__ psets, int T, int D, const uint32_t* __restrict__ start,
                    const float4* __restrict__ srec, const uint32_t* __restrict__ srel, double* __restrict__ rho) {
+    after_previous();
     extern __shared__ float4 smd4[];
     const int t = blockIdx.x;
     const uint32_t s0 = start[t];
@@ -661,6 +669,7 @@ __global__ void __launch_bounds__(256, 4)
     k_spread_mma(const int* __restrict__ tile_sys, const SysDev* __restrict__ sys, const ParamSet* __restrict__ psets,
                  int T, int D, const uint32_t* __restrict__ start, const float4* __restrict__ srec,
                  const uint32_t* __restrict__ srel, double* __restrict__ rho) {
+    after_previous();
     extern __shared__ float4 smm4[];
     // per k-step of the chunk: the tile rows Y that carry stencil weight
     // (particles are sorted by y origin inside a tile, so most k-steps touch
@@ -978,6 +987,7 @@ __device__ float2* fft_lines(float2* s0, float2* s1, int n, int B, int SB, const
 // A_k = (Z_k + conj Z_{n-k})/2, B_k = (Z_k - conj Z_{n-k})/(2i).
 __global__ void k_fftx_fwd(const int4* __restrict__ items, const SysDev* __restrict__ sys,
                            const float2* __restrict__ tw, const double* __restrict__ rho, float2* __restrict__ spec) {
+    after_previous();
     extern __shared__ float2 sb[];
     const int4 it = items[blockIdx.x];
     const SysDev S = sys[it.x];
@@ -1015,6 +1025,7 @@ __global__ void k_fftx_fwd(const int4* __restrict__ items, const SysDev* __restr
 template <bool INV>
 __global__ void k_ffty(const int4* __restrict__ items, const SysDev* __restrict__ sys,
                        const float2* __restrict__ tw, float2* __restrict__ spec) {
+    after_previous();
     extern __shared__ float2 sb[];
     const int4 it = items[blockIdx.x];
     const SysDev S = sys[it.x];
@@ -1040,6 +1051,7 @@ template <bool VIR>
 __global__ void k_fftz_conv(const int4* __restrict__ items, const SysDev* __restrict__ sys,
                             const float2* __restrict__ tw, const float2* __restrict__ gtab,
                             float2* __restrict__ spec, double* __restrict__ acc) {
+    after_previous();
     extern __shared__ float2 sb[];
     __shared__ double red[32 * 7];
     const int4 it = items[blockIdx.x];
@@ -1105,6 +1117,7 @@ __global__ void k_fftz_conv(const int4* __restrict__ items, const SysDev* __rest
 __global__ void k_fftx_inv(const int4* __restrict__ items, const SysDev* __restrict__ sys,
                            const float2* __restrict__ tw, const float2* __restrict__ spec, float* __restrict__ phi,
                            double* __restrict__ rho) {
+    after_previous();
     extern __shared__ float2 sb[];
     const int4 it = items[blockIdx.x];
     const SysDev S = sys[it.x];
@@ -1170,6 +1183,7 @@ __device__ __forceinline__ int odd_up(int v) { return v | 1; }
 __global__ void __launch_bounds__(256)
     k_fft_plane_fwd(const int2* __restrict__ items, const SysDev* __restrict__ sys, const float2* __restrict__ tw,
                     const double* __restrict__ rho, float2* __restrict__ spec) {
+    after_previous();
     extern __shared__ float2 sb[];
     const int2 it = items[blockIdx.x];
     const SysDev S = sys[it.x];
@@ -1212,6 +1226,7 @@ __global__ void __launch_bounds__(256)
 __global__ void __launch_bounds__(256)
     k_fft_plane_inv(const int2* __restrict__ items, const SysDev* __restrict__ sys, const float2* __restrict__ tw,
                     const float2* __restrict__ spec, float* __restrict__ phi, double* __restrict__ rho) {
+    after_previous();
     extern __shared__ float2 sb[];
     const int2 it = items[blockIdx.x];
     const SysDev S = sys[it.x];
@@ -1279,6 +1294,7 @@ template <bool VIR>
 __global__ void __launch_bounds__(256)
     k_fft_slab_z(const int2* __restrict__ items, const SysDev* __restrict__ sys, const float2* __restrict__ tw,
                  const float2* __restrict__ gtab, float2* __restrict__ spec, double* __restrict__ acc) {
+    after_previous();
     extern __shared__ float2 sb[];
     __shared__ double red[32 * 7];
     const int2 it = items[blockIdx.x];
@@ -1628,6 +1644,7 @@ __global__ void __launch_bounds__(128, 6)
              const float4* __restrict__ srec, const uint32_t* __restrict__ srel, const float* __restrict__ phi,
              float4* __restrict__ force, double* __restrict__ acc, const CUtensorMap* __restrict__ tmaps,
              int* __restrict__ kerr) {
+    after_previous();
     using C = InterpCfg<P>;
     extern __shared__ float4 sm4[];
     __shared__ double red[32];
@@ -1917,13 +1934,13 @@ __global__ void __launch_bounds__(128, 5)
 
 // Energy and virial per system: E = sum_i e_i + E_bg; W = W_k + W_pair + E_bg I.
 // external (may be NULL): the terms no particle owns, {E_bg, W_k + E_bg I}.
-__global__ void k_finalize(const SysDev* __restrict__ sys, const ParamSet* __restrict__ psets, int nsys,
-                           const double* __restrict__ acc, double* __restrict__ energy, double* __restrict__ virial,
-                           int add_bg, double* __restrict__ external) {
-    const int s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= nsys) return;
-    const SysDev S = sys[s];
-    const double* a = acc + s * ACC_STRIDE;
+// Leaves the accumulators at zero for the next evaluation.
+__device__ __forceinline__ void finalize_system(int s, const SysDev* __restrict__ sys,
+                                                const ParamSet* __restrict__ psets, double* __restrict__ acc,
+                                                double* __restrict__ energy, double* __restrict__ virial, int add_bg,
+                                                double* __restrict__ external) {
+    const SysDev& S = sys[s];
+    double* a = acc + s * ACC_STRIDE;
     const double Q = a[ACC_QSUM];
     const double ebg = add_bg ? psets[S.pset].bg_coef * Q * Q / S.V : 0.0;
     const int diag[6] = {1, 0, 0, 1, 0, 1};
@@ -1935,6 +1952,40 @@ __global__ void k_finalize(const SysDev* __restrict__ sys, const ParamSet* __res
         external[7 * s] = ebg;
         for (int k = 0; k < 6; ++k) external[7 * s + 1 + k] = a[ACC_WK + k] + (diag[k] ? ebg : 0.0);
     }
+    for (int k = 0; k < ACC_STRIDE; ++k) a[k] = 0.0;
+}
+
+__global__ void k_finalize(const SysDev* __restrict__ sys, const ParamSet* __restrict__ psets, int nsys,
+                           double* __restrict__ acc, double* __restrict__ energy, double* __restrict__ virial,
+                           int add_bg, double* __restrict__ external) {
+    const int s = blockIdx.x * blockDim.x + threadIdx.x;
+    if (s < nsys) finalize_system(s, sys, psets, acc, energy, virial, add_bg, external);
+}
+
+// force += add (the concurrently computed pair forces and energies); the blocks
+// past the particles' finish the systems' totals: one launch where two short
+// ones took 1.7 and 2.5 us and the gap between them.
+template <typename T4>
+__global__ void __launch_bounds__(256)
+    k_add_finalize(const int2* __restrict__ chunks, int n_chunks, const SysDev* __restrict__ sys,
+                   const ParamSet* __restrict__ psets, int nsys, const T4* __restrict__ add, T4* __restrict__ force,
+                   double* __restrict__ acc, double* __restrict__ energy, double* __restrict__ virial, int add_bg,
+                   double* __restrict__ external) {
+    if ((int)blockIdx.x >= n_chunks) {
+        const int s = ((int)blockIdx.x - n_chunks) * blockDim.x + threadIdx.x;
+        if (s < nsys) finalize_system(s, sys, psets, acc, energy, virial, add_bg, external);
+        return;
+    }
+    const int2 ch = chunks[blockIdx.x];
+    const int i = ch.y + threadIdx.x;
+    if (i >= sys[ch.x].p_off + sys[ch.x].N) return;
+    const T4 b = add[i];
+    T4 f = force[i];
+    f.x += b.x;
+    f.y += b.y;
+    f.z += b.z;
+    f.w += b.w;
+    force[i] = f;
 }
 
 // ============================================================================
@@ -2012,13 +2063,13 @@ static cudaError_t launch_spread_p(const LaunchArgs& a, cudaStream_t st) {
     }
     if (a.n_tiles == 0) return cudaSuccess;
     if (mma)
-        k_spread_mma<P><<<dim3(a.n_tiles, tile_split(a, 4, SPREAD_CHM)), 256, smem_m, st>>>(a.tile_sys, a.sys, a.psets, a.T, a.D, a.tile_start, a.srec,
+        launch_after(a.overlap, k_spread_mma<P>, dim3(a.n_tiles, tile_split(a, 4, SPREAD_CHM)), 256, smem_m, st, a.tile_sys, a.sys, a.psets, a.T, a.D, a.tile_start, a.srec,
                                                         a.srel, a.rho);
     else if (dense)
-        k_spread_dense<P><<<a.n_tiles, 256, smem_d, st>>>(a.tile_sys, a.sys, a.psets, a.T, a.D, a.tile_start, a.srec,
+        launch_after(a.overlap, k_spread_dense<P>, a.n_tiles, 256, smem_d, st, a.tile_sys, a.sys, a.psets, a.T, a.D, a.tile_start, a.srec,
                                                           a.srel, a.rho);
     else
-        k_spread<P><<<a.n_tiles, C::THREADS, smem, st>>>(a.tile_sys, a.sys, a.psets, a.T, a.D, a.tile_start, a.srec,
+        launch_after(a.overlap, k_spread<P>, a.n_tiles, C::THREADS, smem, st, a.tile_sys, a.sys, a.psets, a.T, a.D, a.tile_start, a.srec,
                                                           a.srel, a.rho);
     return cudaGetLastError();
 }
@@ -2083,13 +2134,11 @@ static cudaError_t launch_interp_p(const LaunchArgs& a, cudaStream_t st) {
         return cudaGetLastError();
     }
     if (tma)
-        (PX == kPx ? k_interp<P, kTmaForm, kPx> : k_interp<P, kTmaForm, 0>)<<<dim3(a.n_tiles, tile_split(a, 6, C::CH)), C::THREADS,
-                                                                              interp_smem<P>(E, PP), st>>>(
-            a.tile_sys, a.sys, a.psets, a.T, a.D, PX, PP, a.tile_start, a.perm, a.srec, a.srel, a.phi, a.force, a.acc,
+        launch_after(a.overlap, (PX == kPx ? k_interp<P, kTmaForm, kPx> : k_interp<P, kTmaForm, 0>), dim3(a.n_tiles, tile_split(a, 6, C::CH)), C::THREADS,
+                                                                              interp_smem<P>(E, PP), st, a.tile_sys, a.sys, a.psets, a.T, a.D, PX, PP, a.tile_start, a.perm, a.srec, a.srel, a.phi, a.force, a.acc,
             reinterpret_cast<const CUtensorMap*>(a.tmaps), a.kerr);
     else
-        k_interp<P, false, 0><<<dim3(a.n_tiles, tile_split(a, 6, C::CH)), C::THREADS, interp_smem<P>(E, PP), st>>>(
-            a.tile_sys, a.sys, a.psets, a.T, a.D, PX, PP, a.tile_start, a.perm, a.srec, a.srel, a.phi, a.force, a.acc,
+        launch_after(a.overlap, k_interp<P, false, 0>, dim3(a.n_tiles, tile_split(a, 6, C::CH)), C::THREADS, interp_smem<P>(E, PP), st, a.tile_sys, a.sys, a.psets, a.T, a.D, PX, PP, a.tile_start, a.perm, a.srec, a.srel, a.phi, a.force, a.acc,
             nullptr, a.kerr);
     return cudaGetLastError();
 }
@@ -2097,20 +2146,20 @@ static cudaError_t launch_interp_p(const LaunchArgs& a, cudaStream_t st) {
 // One CTA scans up to SCAN_ONE_CTA counts in one round; above, its rounds are
 // serial (the 256-lattice batch's tiles: 21.6 us) and two short kernels over
 // all CTAs take over (8.8 us).
-cudaError_t launch_scan(const uint32_t* cnt, uint32_t* start, int n, uint32_t* ws, cudaStream_t st) {
+cudaError_t launch_scan(const uint32_t* cnt, uint32_t* start, int n, uint32_t* ws, cudaStream_t st, bool overlap) {
     if (ws && n > SCAN_ONE_CTA) {
         const int nb = (int)scan_ws_size(n);
-        k_scan_sums<<<nb, 256, 0, st>>>(cnt, ws, n);
-        k_scan_apply<<<nb, 256, 0, st>>>(cnt, ws, start, n);
+        launch_after(overlap, k_scan_sums, nb, 256, 0, st, cnt, ws, n);
+        launch_after(overlap, k_scan_apply, nb, 256, 0, st, cnt, ws, start, n);
     } else {
-        k_scan<<<1, 1024, 0, st>>>(cnt, start, n);
+        launch_after(overlap, k_scan, 1, 1024, 0, st, cnt, start, n);
     }
     return cudaGetLastError();
 }
 
 cudaError_t launch_scatter(const int2* chunks, int n_chunks, const SysDev* sys, const uint32_t* key,
-                           const uint32_t* start, uint32_t* cnt, uint32_t* perm_u, cudaStream_t st) {
-    if (n_chunks) k_scatter<<<n_chunks, 256, 0, st>>>(chunks, sys, key, start, cnt, perm_u);
+                           const uint32_t* start, uint32_t* cnt, uint32_t* perm_u, cudaStream_t st, bool overlap) {
+    if (n_chunks) launch_after(overlap, k_scatter, n_chunks, 256, 0, st, chunks, sys, key, start, cnt, perm_u);
     return cudaGetLastError();
 }
 
@@ -2123,12 +2172,12 @@ cudaError_t launch_bin(const LaunchArgs& a, cudaStream_t st) {
 }
 
 cudaError_t launch_sort(const LaunchArgs& a, cudaStream_t st) {
-    const cudaError_t e = launch_scan(a.tile_count, a.tile_start, a.n_tiles, a.scan_ws, st);
+    const cudaError_t e = launch_scan(a.tile_count, a.tile_start, a.n_tiles, a.scan_ws, st, a.overlap);
     if (e != cudaSuccess) return e;
-    if (a.n_chunks) k_scatter<<<a.n_chunks, 256, 0, st>>>(a.chunks, a.sys, a.key, a.tile_start, a.tile_count, a.perm_u);
+    if (a.n_chunks) launch_after(a.overlap, k_scatter, a.n_chunks, 256, 0, st, a.chunks, a.sys, a.key, a.tile_start, a.tile_count, a.perm_u);
     if (a.n_tiles)
         // a CTA sized to its tile: full tiles (coarse meshes, dense systems) take 512 threads
-        k_tile_sort<<<a.n_tiles, a.n_chunks * 256LL > 192LL * a.n_tiles ? 512 : 128, 0, st>>>(a.tile_start, a.perm_u, a.perm, a.trec, a.rel, a.srec, a.srel,
+        launch_after(a.overlap, k_tile_sort, a.n_tiles, a.n_chunks * 256LL > 192LL * a.n_tiles ? 512 : 128, 0, st, a.tile_start, a.perm_u, a.perm, a.trec, a.rel, a.srec, a.srel,
                                                a.tile_sys, a.sys);
     return cudaGetLastError();
 }
@@ -2161,24 +2210,24 @@ cudaError_t launch_fft(const LaunchArgs& a, cudaStream_t st) {
             return e;
         return cudaFuncSetAttribute(k_fft_slab_z<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, FFT_SMEM_MAX);
     }
-    if (a.n_pitems) k_fft_plane_fwd<<<a.n_pitems, 256, a.smem_plane, st>>>(a.pitems, a.sys, a.tw, a.rho, a.spec);
-    if (a.n_xitems) k_fftx_fwd<<<a.n_xitems, 256, smx, st>>>(a.xitems, a.sys, a.tw, a.rho, a.spec);
-    if (a.n_yitems) k_ffty<false><<<a.n_yitems, 256, smy, st>>>(a.yitems, a.sys, a.tw, a.spec);
+    if (a.n_pitems) launch_after(a.overlap, k_fft_plane_fwd, a.n_pitems, 256, a.smem_plane, st, a.pitems, a.sys, a.tw, a.rho, a.spec);
+    if (a.n_xitems) launch_after(a.overlap, k_fftx_fwd, a.n_xitems, 256, smx, st, a.xitems, a.sys, a.tw, a.rho, a.spec);
+    if (a.n_yitems) launch_after(a.overlap, k_ffty<false>, a.n_yitems, 256, smy, st, a.yitems, a.sys, a.tw, a.spec);
     if (a.n_sitems) {
         if (a.want_virial)
-            k_fft_slab_z<true><<<a.n_sitems, 256, a.smem_slab, st>>>(a.sitems, a.sys, a.tw, a.gtab, a.spec, a.acc);
+            launch_after(a.overlap, k_fft_slab_z<true>, a.n_sitems, 256, a.smem_slab, st, a.sitems, a.sys, a.tw, a.gtab, a.spec, a.acc);
         else
-            k_fft_slab_z<false><<<a.n_sitems, 256, a.smem_slab, st>>>(a.sitems, a.sys, a.tw, a.gtab, a.spec, a.acc);
+            launch_after(a.overlap, k_fft_slab_z<false>, a.n_sitems, 256, a.smem_slab, st, a.sitems, a.sys, a.tw, a.gtab, a.spec, a.acc);
     }
     if (a.n_zitems) {
         if (a.want_virial)
-            k_fftz_conv<true><<<a.n_zitems, 256, smz, st>>>(a.zitems, a.sys, a.tw, a.gtab, a.spec, a.acc);
+            launch_after(a.overlap, k_fftz_conv<true>, a.n_zitems, 256, smz, st, a.zitems, a.sys, a.tw, a.gtab, a.spec, a.acc);
         else
-            k_fftz_conv<false><<<a.n_zitems, 256, smz, st>>>(a.zitems, a.sys, a.tw, a.gtab, a.spec, a.acc);
+            launch_after(a.overlap, k_fftz_conv<false>, a.n_zitems, 256, smz, st, a.zitems, a.sys, a.tw, a.gtab, a.spec, a.acc);
     }
-    if (a.n_yitems) k_ffty<true><<<a.n_yitems, 256, smy, st>>>(a.yitems, a.sys, a.tw, a.spec);
-    if (a.n_xitems) k_fftx_inv<<<a.n_xitems, 256, smx, st>>>(a.xitems, a.sys, a.tw, a.spec, a.phi, a.rho);
-    if (a.n_pitems) k_fft_plane_inv<<<a.n_pitems, 256, a.smem_plane, st>>>(a.pitems, a.sys, a.tw, a.spec, a.phi, a.rho);
+    if (a.n_yitems) launch_after(a.overlap, k_ffty<true>, a.n_yitems, 256, smy, st, a.yitems, a.sys, a.tw, a.spec);
+    if (a.n_xitems) launch_after(a.overlap, k_fftx_inv, a.n_xitems, 256, smx, st, a.xitems, a.sys, a.tw, a.spec, a.phi, a.rho);
+    if (a.n_pitems) launch_after(a.overlap, k_fft_plane_inv, a.n_pitems, 256, a.smem_plane, st, a.pitems, a.sys, a.tw, a.spec, a.phi, a.rho);
     return cudaGetLastError();
 }
 
@@ -2197,6 +2246,7 @@ __global__ void k_exclusions(const int2* __restrict__ chunks, const SysDev* __re
                              const uint32_t* __restrict__ n_ex, const uint32_t* __restrict__ ex_list, int ex_pitch,
                              float4* __restrict__ force, double* __restrict__ acc, float* __restrict__ vpp,
                              int vpitch) {
+    after_previous();
     __shared__ double red[32 * 7];
     const int2 ch = chunks[blockIdx.x];
     const SysDev S = sys[ch.x];
@@ -2263,30 +2313,9 @@ __global__ void k_exclusions(const int2* __restrict__ chunks, const SysDev* __re
     }
 }
 
-// force += add (the concurrently computed pair forces and energies).
-__global__ void k_add_forces(const int2* __restrict__ chunks, const SysDev* __restrict__ sys,
-                             const float4* __restrict__ add, float4* __restrict__ force) {
-    const int2 ch = chunks[blockIdx.x];
-    const int i = ch.y + threadIdx.x;
-    if (i >= sys[ch.x].p_off + sys[ch.x].N) return;
-    const float4 b = add[i];
-    float4 f = force[i];
-    f.x += b.x;
-    f.y += b.y;
-    f.z += b.z;
-    f.w += b.w;
-    force[i] = f;
-}
-
-cudaError_t launch_add_forces(const int2* chunks, int n_chunks, const SysDev* sys, const float4* add, float4* force,
-                              cudaStream_t st) {
-    if (n_chunks) k_add_forces<<<n_chunks, 256, 0, st>>>(chunks, sys, add, force);
-    return cudaGetLastError();
-}
-
 cudaError_t launch_exclusions(const LaunchArgs& a, cudaStream_t st) {
     if (a.n_chunks == 0 || !a.ex_n) return cudaSuccess;
-    k_exclusions<<<a.n_chunks, 256, 0, st>>>(a.chunks, a.sys, a.psets, a.posq, a.ex_n, a.ex_list, a.ex_pitch,
+    launch_after(a.overlap, k_exclusions, a.n_chunks, 256, 0, st, a.chunks, a.sys, a.psets, a.posq, a.ex_n, a.ex_list, a.ex_pitch,
                                              a.force, a.acc, a.virial_pp, a.vpp_pitch);
     return cudaGetLastError();
 }
@@ -2295,6 +2324,21 @@ cudaError_t launch_finalize(const LaunchArgs& a, cudaStream_t st) {
     k_finalize<<<(a.nsys + 127) / 128, 128, 0, st>>>(a.sys, a.psets, a.nsys, a.acc, a.energy, a.virial, a.add_bg,
                                                      a.external);
     return cudaGetLastError();
+}
+
+template <typename T4>
+static cudaError_t launch_add_finalize_t(const LaunchArgs& a, const T4* add, T4* force, cudaStream_t st) {
+    k_add_finalize<T4><<<a.n_chunks + (a.nsys + 255) / 256, 256, 0, st>>>(
+        a.chunks, a.n_chunks, a.sys, a.psets, a.nsys, add, force, a.acc, a.energy, a.virial, a.add_bg, a.external);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_add_finalize(const LaunchArgs& a, const float4* add, float4* force, cudaStream_t st) {
+    return launch_add_finalize_t(a, add, force, st);
+}
+
+cudaError_t launch_add_finalize(const LaunchArgs& a, const double4* add, double4* force, cudaStream_t st) {
+    return launch_add_finalize_t(a, add, force, st);
 }
 
 cudaError_t launch_influence(const SysDev& S, const double* w1d, const double* tq, const double* wq, int nq,

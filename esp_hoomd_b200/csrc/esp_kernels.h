@@ -52,6 +52,7 @@ struct LaunchArgs {
     const SysDev* sys = nullptr;
     const ParamSet* psets = nullptr;
     int nsys = 0, P = 8, T = 8, D = 10, PX = 0, PP = 0, tpp = 8, accumulate = 0, nq = 16;
+    bool overlap = false;           // kernels of the mesh part start under the end of the one before (launch_after)
     const int2* chunks = nullptr;   // {sys, first particle}, 256 particles each
     int n_chunks = 0;
     const int2* pchunks = nullptr;  // {sys, first particle}, 256/tpp particles each
@@ -126,9 +127,11 @@ struct LaunchArgs {
 // caller's for scans above SCAN_ONE_CTA counts (NULL: one CTA whatever n).
 constexpr int SCAN_ONE_CTA = 1024 * 16;
 inline size_t scan_ws_size(long long n) { return (size_t)((n + 4095) / 4096); }
-cudaError_t launch_scan(const uint32_t* cnt, uint32_t* start, int n, uint32_t* ws, cudaStream_t st);
+cudaError_t launch_scan(const uint32_t* cnt, uint32_t* start, int n, uint32_t* ws, cudaStream_t st,
+                        bool overlap = false);
 cudaError_t launch_scatter(const int2* chunks, int n_chunks, const SysDev* sys, const uint32_t* key,
-                           const uint32_t* start, uint32_t* cnt, uint32_t* perm_u, cudaStream_t st);
+                           const uint32_t* start, uint32_t* cnt, uint32_t* perm_u, cudaStream_t st,
+                           bool overlap = false);
 cudaError_t launch_bin(const LaunchArgs& a, cudaStream_t st);
 cudaError_t launch_sort(const LaunchArgs& a, cudaStream_t st);
 cudaError_t launch_spread(const LaunchArgs& a, cudaStream_t st);
@@ -136,8 +139,9 @@ cudaError_t launch_fft(const LaunchArgs& a, cudaStream_t st);
 cudaError_t launch_interp(const LaunchArgs& a, cudaStream_t st);
 cudaError_t launch_pair(const LaunchArgs& a, cudaStream_t st);
 cudaError_t launch_exclusions(const LaunchArgs& a, cudaStream_t st);
-cudaError_t launch_add_forces(const int2* chunks, int n_chunks, const SysDev* sys, const float4* add, float4* force,
-                              cudaStream_t st);
+// force += add (the concurrently computed pair term), and launch_finalize's totals
+cudaError_t launch_add_finalize(const LaunchArgs& a, const float4* add, float4* force, cudaStream_t st);
+cudaError_t launch_add_finalize(const LaunchArgs& a, const double4* add, double4* force, cudaStream_t st);
 
 // FP64 mode (esp_f64.cu): the shared fields of `a` (descriptors, chunks,
 // tiles, keys, permutation, charge mesh, accumulators, neighbour list,
@@ -170,7 +174,6 @@ cudaError_t launch64_configure(int P, int T);
 cudaError_t launch64_bin(const Launch64& b, cudaStream_t st);
 cudaError_t launch64_mesh(const Launch64& b, cudaStream_t st);
 cudaError_t launch64_pair(const Launch64& b, double4* force, cudaStream_t st);
-cudaError_t launch64_add_forces(const Launch64& b, const double4* add, cudaStream_t st);
 cudaError_t launch_influence64(const SysDev& S, const double* w1d, const double* tq, const double* wq, int nq,
                                double rcut, double psi_floor, double2* gtab, cudaStream_t st);
 cudaError_t launch_finalize(const LaunchArgs& a, cudaStream_t st);

@@ -32,6 +32,7 @@
 #include "esp_b200.h"
 #include "esp_host_util.h"
 #include "esp_kernels.h"
+#include "esp_launch.cuh"
 #include "esp_md.h"
 #include "esp_tables.h"
 
@@ -791,6 +792,7 @@ int esp_server::launch_round(Staging& sg) {
     a.nl_head = d_head;
     a.nl_n = d_nn;
     a.nl_list = d_nl;
+    a.overlap = overlap_starts(a.n_chunks, st);
     const float dt = active.empty() ? 0.f : (float)active[0]->r.dt;
     // NVE first half for the systems past their first evaluation; systems
     // of one round share dt (checked at submit)

@@ -20,6 +20,12 @@ where the rule switches, against the oracle.
   above, with and without the virial, on the last size of the one and the first
   of the other; against the oracle within the FP64 tests' tolerances (forces
   1e-8, energy 1e-10, virial 2e-8, the oracle's own finite difference).
+* overlapped starts (below 192 chunks of 256 particles) and accumulators left
+  clear: two position sets in turn through one context with nothing waited for,
+  and after a charge spread and a long-range-only call, give what a fresh
+  context gives for each (FP32 1e-6 of the RMS force and of the energies'
+  magnitudes, the order of the FP64 mesh sums seen through one FP32 rounding
+  per stage; FP64 1e-12).
 * tile sort: tiles of a few particles, above the 512-thread switch, and above
   the shared-memory capacity (2,048); permutation bit-exact.
 """
@@ -197,3 +203,41 @@ def test_fp64_pair_lane_counts(shape, virial):
     assert abs(energy.item() - E) <= 1e-10 * abs(E)
     if virial:
         assert np.abs(w.cpu().numpy() - W).max() <= 2e-8 * np.abs(W).max()
+
+
+@pytest.mark.parametrize("shape", [(8, 8, 8), (18, 20, 22), (36, 36, 38)])  # 2, 31 and 193 chunks
+@pytest.mark.parametrize("f64", [False, True])
+def test_back_to_back_evaluations(shape, f64):
+    dt = torch.float64 if f64 else torch.float32
+    par = native.make_params(mesh=(30, 32, 36), precision=int(f64))
+    sets = []
+    for seed in (1, 2):
+        s = systems.rocksalt(0, seed=seed, shape=shape)
+        p4 = torch.zeros((s.N, 4), dtype=dt, device="cuda")
+        p4[:, :3] = torch.as_tensor(s.pos, device="cuda")
+        nl = tuple(torch.as_tensor(a.astype(np.int32), device="cuda") for a in R.neighbor_list(s.pos, s.box, 3.0))
+        sets.append((p4, torch.as_tensor(s.q, dtype=dt, device="cuda"), nl))
+
+    def run(ctx, p4, q, nl, **kw):
+        f, e = torch.zeros_like(p4), torch.zeros(1, dtype=torch.float64, device="cuda")
+        (ctx.compute_f64 if f64 else ctx.compute)(p4, q, f, e, nlist=nl, **kw)
+        return f, e
+
+    want = []
+    for a in sets:
+        want.append(run(native.Context(par, s.box, s.N), *a))
+        torch.cuda.synchronize()
+    ctx = native.Context(par, s.box, s.N)
+    got = []
+    for k in range(6):
+        if k == 3:
+            run(ctx, *sets[0][:2], None, flags=ESP_LONG_RANGE)
+            if not f64:
+                ctx.spread(*sets[1][:2])
+        got.append([run(ctx, *a) for a in sets])
+    torch.cuda.synchronize()
+    tol = 1e-12 if f64 else 1e-6
+    for pair in got:
+        for (f, e), (F, E) in zip(pair, want):
+            assert R.rel_rms(f.double().cpu().numpy()[:, :3], F.double().cpu().numpy()[:, :3]) <= tol
+            assert abs(e.item() - E.item()) <= tol * F[:, 3].double().abs().sum().item()
