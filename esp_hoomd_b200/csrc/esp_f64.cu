@@ -921,12 +921,18 @@ cudaError_t launch64_bin(const Launch64& b, cudaStream_t st) {
 
 cudaError_t launch64_mesh(const Launch64& b, cudaStream_t st) {
     const LaunchArgs& a = b.a;
-    cudaError_t e = launch_scan(a.tile_count, a.tile_start, a.n_tiles, a.scan_ws, st, a.overlap);
-    if (e != cudaSuccess) return e;
-    e = launch_scatter(a.chunks, a.n_chunks, a.sys, a.key, a.tile_start, a.tile_count, a.perm_u, st, a.overlap);
-    if (e != cudaSuccess) return e;
+    cudaError_t e;
+    if (a.sort_direct) {
+        if ((e = launch_sort_direct(a, b.trec, b.srec, st)) != cudaSuccess) return e;
+    } else {
+        if ((e = launch_scan(a.tile_count, a.tile_start, a.n_tiles, a.scan_ws, st, a.overlap)) != cudaSuccess) return e;
+        e = launch_scatter(a.chunks, a.n_chunks, a.sys, a.key, a.tile_start, a.tile_count, a.perm_u, st, a.overlap);
+        if (e != cudaSuccess) return e;
+        if (a.n_tiles)
+            launch_after(a.overlap, k64_tile_sort, a.n_tiles, 256, 0, st, a.tile_start, a.perm_u, a.perm, b.trec, a.rel,
+                         b.srec, a.srel);
+    }
     if (a.n_tiles) {
-        launch_after(a.overlap, k64_tile_sort, a.n_tiles, 256, 0, st, a.tile_start, a.perm_u, a.perm, b.trec, a.rel, b.srec, a.srel);
         launch_after(a.overlap, k64_spread, dim3(a.n_tiles, split64(a.n_tiles)), K64S_THREADS, spread64_smem(a.P, a.T), st, a.tile_sys, a.sys, b.wcoef, a.P, a.T, a.D, a.tile_start, b.srec, a.srel, a.rho);
     }
     if (b.n_xl) launch_after(a.overlap, k64_fft_pass<0>, b.n_xl, F64_WARPS * 32, 0, st, b.xl, a.sys, b.tw, b.cbuf, a.rho, b.phi, b.gtab, a.acc);

@@ -260,6 +260,7 @@ struct esp_batch {
     std::vector<PsetHost> psh;
     std::vector<ParamSet> psd;
     std::vector<double> c_split, c_win;
+    bool sort_direct = false;  // small enough for the one-kernel sort
     int n_chunks = 0, n_pchunks = 0, n_x = 0, n_y = 0, n_z = 0;
     DevAlloc mem;
     // device
@@ -665,6 +666,9 @@ int esp_batch::plan(const esp_params& p, int ns, const int* N_, const double* bo
     n_p = (int)pi.size();
     n_s = (int)si.size();
     n_chunks = (int)chunks.size();
+    long long reads = 0;
+    for (const SysDev& S : sd) reads += (long long)S.N * S.ntx * S.nty * S.ntz;
+    sort_direct = sort_is_direct(n_chunks, reads, p.precision == ESP_FP64);
     n_pchunks = (int)pchunks.size();
     n_x = (int)xi.size();
     n_y = (int)yi.size();
@@ -852,6 +856,7 @@ int esp_batch::compute_f64(cudaStream_t st, const double* pos4, const double* q,
     b.a = args();
     LaunchArgs& a = b.a;
     a.overlap = overlap_starts(a.n_chunks, st);
+    a.sort_direct = a.overlap && sort_direct;
     if (energy) a.energy = energy;
     if (virial) a.virial = virial;
     a.want_virial = virial != nullptr;
@@ -998,6 +1003,7 @@ int esp_batch::compute(cudaStream_t st, const float* pos4, const float* q, const
         return fail(ESP_ERR_INVALID, "no neighbour list given and no pair list built (esp_batch_build_pairlist)");
     LaunchArgs a = args();
     a.overlap = overlap_starts(a.n_chunks, st);
+    a.sort_direct = a.overlap && sort_direct;
     if ((flags & ESP_SHORT_RANGE) && use_pl) a.plist = &pl;
     a.pos_in = reinterpret_cast<const float4*>(pos4);
     a.q_in = q;

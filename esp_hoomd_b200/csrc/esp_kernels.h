@@ -53,6 +53,7 @@ struct LaunchArgs {
     const ParamSet* psets = nullptr;
     int nsys = 0, P = 8, T = 8, D = 10, PX = 0, PP = 0, tpp = 8, accumulate = 0, nq = 16;
     bool overlap = false;           // kernels of the mesh part start under the end of the one before (launch_after)
+    bool sort_direct = false;       // scan, scatter and tile sort as one kernel (tiles and particles in one order)
     const int2* chunks = nullptr;   // {sys, first particle}, 256 particles each
     int n_chunks = 0;
     const int2* pchunks = nullptr;  // {sys, first particle}, 256/tpp particles each
@@ -134,6 +135,18 @@ cudaError_t launch_scatter(const int2* chunks, int n_chunks, const SysDev* sys, 
                            bool overlap = false);
 cudaError_t launch_bin(const LaunchArgs& a, cudaStream_t st);
 cudaError_t launch_sort(const LaunchArgs& a, cudaStream_t st);
+// Rule of the one-kernel sort, for evaluations whose kernels overlap (`reads`:
+// particles x tiles, summed over the systems). FP32, host launches: 512 ions
+// 44.8 against 42.9 us, 4,096 57.4 against 52.4, 12,963 water charges 99.7
+// against 95.7 (0.8M reads), but 21,000 97.1 against 108.2 and 13,824 ions in
+// 216 tiles (3.0M) 73.8 against 74.4. FP64, the mesh part on a stream of its
+// own: 12,963 charges 149.1 against 143.3, 21,000 180.0 against 174.5 (15M),
+// 30,000 even, 60,000 362 against 395.
+inline bool sort_is_direct(int n_chunks, long long reads, bool f64) {
+    return f64 ? n_chunks <= 96 && reads <= 16000000 : n_chunks <= 64 && reads <= 2000000;
+}
+// sort of the FP64 records (sort_direct)
+cudaError_t launch_sort_direct(const LaunchArgs& a, const double4* trec, double4* srec, cudaStream_t st);
 cudaError_t launch_spread(const LaunchArgs& a, cudaStream_t st);
 cudaError_t launch_fft(const LaunchArgs& a, cudaStream_t st);
 cudaError_t launch_interp(const LaunchArgs& a, cudaStream_t st);

@@ -26,6 +26,9 @@ where the rule switches, against the oracle.
   context gives for each (FP32 1e-6 of the RMS force and of the energies'
   magnitudes, the order of the FP64 mesh sums seen through one FP32 rounding
   per stage; FP64 1e-12).
+* one-kernel sort (small systems): tiles above the shared-memory
+  capacity, both sides of its 64 chunks; long-range forces against the oracle
+  (FP32 5e-6, FP64 1e-8).
 * tile sort: tiles of a few particles, above the 512-thread switch, and above
   the shared-memory capacity (2,048); permutation bit-exact.
 """
@@ -241,3 +244,29 @@ def test_back_to_back_evaluations(shape, f64):
         for (f, e), (F, E) in zip(pair, want):
             assert R.rel_rms(f.double().cpu().numpy()[:, :3], F.double().cpu().numpy()[:, :3]) <= tol
             assert abs(e.item() - E.item()) <= tol * F[:, 3].double().abs().sum().item()
+
+
+@pytest.mark.parametrize("n,mesh", [(400, 24), (4200, 24), (6000, 12), (16384, 24), (16640, 24)])
+@pytest.mark.parametrize("f64", [False, True])
+def test_one_kernel_sort(n, mesh, f64):
+    # long-range forces through the sort of a whole evaluation: one kernel up to
+    # 64 chunks (the last size is above; the third has tiles above 2,048 particles)
+    rng = np.random.default_rng(n)
+    L = 10.0
+    pos = rng.uniform(0, L, (n, 3)).astype(np.float32).astype(np.float64)
+    q = np.where(np.arange(n) % 2 == 0, 1.0, -1.0)
+    dt = torch.float64 if f64 else torch.float32
+    ctx = native.Context(native.make_params(order=6, mesh=(mesh,) * 3, precision=int(f64)), (L, L, L), n)
+    inf = ctx.info()
+    p4 = torch.zeros((n, 4), dtype=dt, device="cuda")
+    p4[:, :3] = torch.as_tensor(pos, device="cuda")
+    force = torch.zeros_like(p4)
+    run = ctx.compute_f64 if f64 else ctx.compute
+    for _ in range(2):  # the second finds the tile counts clear
+        run(p4, torch.as_tensor(q, dtype=dt, device="cuda"), force, flags=ESP_LONG_RANGE)
+    split = tables.make_split(inf["c_split"], tol=1e-12) if f64 else tables.split_cached(inf["c_split"])
+    prm = tables.ESPParams(mesh=(mesh,) * 3, box=(L, L, L), rcut=inf["rcut"], split=split,
+                           window=tables.window_cached(inf["order"], inf["c_window"], inf["window_degree"]))
+    empty = (np.zeros(n, np.uint32), np.zeros(n, np.uint32), np.zeros(0, np.uint32))
+    _, F, _ = R.esp(pos, q, prm, nlist=empty)
+    assert R.rel_rms(force.double().cpu().numpy()[:, :3], F) <= (1e-8 if f64 else 5e-6)
