@@ -792,6 +792,10 @@ int esp_server::launch_round(Staging& sg) {
     a.nl_head = d_head;
     a.nl_n = d_nn;
     a.nl_list = d_nl;
+    // pair energies only in rounds that end a request: every other round's are overwritten
+    a.want_energy = 0;
+    for (const Request* q : active)
+        if (q->steps_done + (q->evaluated ? 1 : 0) >= q->r.nsteps) a.want_energy = 1;
     a.overlap = overlap_starts(a.n_chunks, st);
     const float dt = active.empty() ? 0.f : (float)active[0]->r.dt;
     // NVE first half for the systems past their first evaluation; systems
