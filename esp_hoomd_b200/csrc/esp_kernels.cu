@@ -1290,7 +1290,8 @@ __global__ void k_fftx_inv(const int4* __restrict__ items, const SysDev* __restr
 // ----------------------------------------------------------------------------
 __device__ __forceinline__ int odd_up(int v) { return v | 1; }
 
-__global__ void __launch_bounds__(256)
+template <int NT>
+__global__ void __launch_bounds__(NT)
     k_fft_plane_fwd(const int2* __restrict__ items, const SysDev* __restrict__ sys, const float2* __restrict__ tw,
                     const double* __restrict__ rho, float2* __restrict__ spec) {
     after_previous();
@@ -1333,7 +1334,8 @@ __global__ void __launch_bounds__(256)
     }
 }
 
-__global__ void __launch_bounds__(256)
+template <int NT>
+__global__ void __launch_bounds__(NT)
     k_fft_plane_inv(const int2* __restrict__ items, const SysDev* __restrict__ sys, const float2* __restrict__ tw,
                     const float2* __restrict__ spec, float* __restrict__ phi, double* __restrict__ rho) {
     after_previous();
@@ -1400,8 +1402,8 @@ __global__ void __launch_bounds__(256)
 
 // z pass over a whole xz-slab (fixed y): forward, energy/virial (VIR: when
 // the virial is requested), influence multiply, inverse.
-template <bool VIR>
-__global__ void __launch_bounds__(256)
+template <bool VIR, int NT>
+__global__ void __launch_bounds__(NT)
     k_fft_slab_z(const int2* __restrict__ items, const SysDev* __restrict__ sys, const float2* __restrict__ tw,
                  const float2* __restrict__ gtab, float2* __restrict__ spec, double* __restrict__ acc) {
     after_previous();
@@ -2297,6 +2299,58 @@ cudaError_t launch_spread(const LaunchArgs& a, cudaStream_t st) { ESPB_DISPATCH_
 
 cudaError_t launch_interp(const LaunchArgs& a, cudaStream_t st) { ESPB_DISPATCH_P(launch_interp_p, a.P, a, st); }
 
+template <int NT>
+static cudaError_t configure_fft_t() {
+    cudaError_t e;
+    if ((e = cudaFuncSetAttribute(k_fft_plane_fwd<NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, FFT_SMEM_MAX)))
+        return e;
+    if ((e = cudaFuncSetAttribute(k_fft_plane_inv<NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, FFT_SMEM_MAX)))
+        return e;
+    if ((e = cudaFuncSetAttribute(k_fft_slab_z<true, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, FFT_SMEM_MAX)))
+        return e;
+    return cudaFuncSetAttribute(k_fft_slab_z<false, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, FFT_SMEM_MAX);
+}
+template <int NT>
+static void launch_plane_fwd(const LaunchArgs& a, cudaStream_t st) {
+    launch_after(a.overlap, k_fft_plane_fwd<NT>, a.n_pitems, NT, a.smem_plane, st, a.pitems, a.sys, a.tw, a.rho, a.spec);
+}
+template <int NT>
+static void launch_plane_inv(const LaunchArgs& a, cudaStream_t st) {
+    launch_after(a.overlap, k_fft_plane_inv<NT>, a.n_pitems, NT, a.smem_plane, st, a.pitems, a.sys, a.tw, a.spec, a.phi,
+                 a.rho);
+}
+template <int NT>
+static void launch_slab(const LaunchArgs& a, cudaStream_t st) {
+    if (a.want_virial)
+        launch_after(a.overlap, k_fft_slab_z<true, NT>, a.n_sitems, NT, a.smem_slab, st, a.sitems, a.sys, a.tw, a.gtab,
+                     a.spec, a.acc);
+    else
+        launch_after(a.overlap, k_fft_slab_z<false, NT>, a.n_sitems, NT, a.smem_slab, st, a.sitems, a.sys, a.tw, a.gtab,
+                     a.spec, a.acc);
+}
+#define ESPB_FFT_THREADS(NT, FN, ...)              \
+    do {                                           \
+        if ((NT) == 1024) FN<1024>(__VA_ARGS__);   \
+        else if ((NT) == 512) FN<512>(__VA_ARGS__); \
+        else FN<256>(__VA_ARGS__);                 \
+    } while (0)
+
+// Threads per plane or slab. The passes are bound by latency, so an SM that
+// holds one or two CTAs wants larger ones: few CTAs in the launch (one system:
+// 64 planes of 64 x 64, evaluation 108.1 / 101.8 / 99.5 us with 256 / 512 /
+// 1,024 threads; 36 of 36 x 36 76.4 / 67.5 / 69.3; 16 of 16 x 16 40.9 / 41.8 /
+// 44.7), or planes that fill the shared memory (eight systems, 128 x 128, one
+// CTA per SM: 4 MD steps 14.99 / 13.78 / 13.43 ms; 108 x 108, two: 7.97 / 7.73 /
+// 8.20). With three or more resident CTAs larger ones only wait longer at their
+// barriers (eight systems, 96 x 96: 5.62 / 5.70 / 6.12 ms; the 256-lattice
+// batch, 10 steps: 67.1 / 71.8 / 82.5 ms).
+static int fft_threads(int ctas, int smem) {
+    const int pts = smem / 16;  // points of the largest plane, two buffers of 8 bytes each
+    const int resident = std::min((ctas + 147) / 148, smem > 113 * 1024 ? 1 : (smem > 80 * 1024 ? 2 : 3));
+    if (resident <= 1) return pts >= 2000 ? 1024 : (pts >= 250 ? 512 : 256);
+    return resident == 2 && pts >= 1500 ? 512 : 256;
+}
+
 cudaError_t launch_fft(const LaunchArgs& a, cudaStream_t st) {
     // attributes allow the largest transform; launches request what the
     // batch's longest line on that axis needs (occupancy for small meshes)
@@ -2313,23 +2367,14 @@ cudaError_t launch_fft(const LaunchArgs& a, cudaStream_t st) {
         if ((e = cudaFuncSetAttribute(k_fftz_conv<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smyz))) return e;
         if ((e = cudaFuncSetAttribute(k_fftz_conv<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smyz)))
             return e;
-        if ((e = cudaFuncSetAttribute(k_fft_plane_fwd, cudaFuncAttributeMaxDynamicSharedMemorySize, FFT_SMEM_MAX)))
-            return e;
-        if ((e = cudaFuncSetAttribute(k_fft_plane_inv, cudaFuncAttributeMaxDynamicSharedMemorySize, FFT_SMEM_MAX)))
-            return e;
-        if ((e = cudaFuncSetAttribute(k_fft_slab_z<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, FFT_SMEM_MAX)))
-            return e;
-        return cudaFuncSetAttribute(k_fft_slab_z<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, FFT_SMEM_MAX);
+        if ((e = configure_fft_t<256>()) || (e = configure_fft_t<512>())) return e;
+        return configure_fft_t<1024>();
     }
-    if (a.n_pitems) launch_after(a.overlap, k_fft_plane_fwd, a.n_pitems, 256, a.smem_plane, st, a.pitems, a.sys, a.tw, a.rho, a.spec);
+    const int nt_p = fft_threads(a.n_pitems, (int)a.smem_plane), nt_s = fft_threads(a.n_sitems, (int)a.smem_slab);
+    if (a.n_pitems) ESPB_FFT_THREADS(nt_p, launch_plane_fwd, a, st);
     if (a.n_xitems) launch_after(a.overlap, k_fftx_fwd, a.n_xitems, 256, smx, st, a.xitems, a.sys, a.tw, a.rho, a.spec);
     if (a.n_yitems) launch_after(a.overlap, k_ffty<false>, a.n_yitems, 256, smy, st, a.yitems, a.sys, a.tw, a.spec);
-    if (a.n_sitems) {
-        if (a.want_virial)
-            launch_after(a.overlap, k_fft_slab_z<true>, a.n_sitems, 256, a.smem_slab, st, a.sitems, a.sys, a.tw, a.gtab, a.spec, a.acc);
-        else
-            launch_after(a.overlap, k_fft_slab_z<false>, a.n_sitems, 256, a.smem_slab, st, a.sitems, a.sys, a.tw, a.gtab, a.spec, a.acc);
-    }
+    if (a.n_sitems) ESPB_FFT_THREADS(nt_s, launch_slab, a, st);
     if (a.n_zitems) {
         if (a.want_virial)
             launch_after(a.overlap, k_fftz_conv<true>, a.n_zitems, 256, smz, st, a.zitems, a.sys, a.tw, a.gtab, a.spec, a.acc);
@@ -2338,7 +2383,7 @@ cudaError_t launch_fft(const LaunchArgs& a, cudaStream_t st) {
     }
     if (a.n_yitems) launch_after(a.overlap, k_ffty<true>, a.n_yitems, 256, smy, st, a.yitems, a.sys, a.tw, a.spec);
     if (a.n_xitems) launch_after(a.overlap, k_fftx_inv, a.n_xitems, 256, smx, st, a.xitems, a.sys, a.tw, a.spec, a.phi, a.rho);
-    if (a.n_pitems) launch_after(a.overlap, k_fft_plane_inv, a.n_pitems, 256, a.smem_plane, st, a.pitems, a.sys, a.tw, a.spec, a.phi, a.rho);
+    if (a.n_pitems) ESPB_FFT_THREADS(nt_p, launch_plane_inv, a, st);
     return cudaGetLastError();
 }
 

@@ -29,6 +29,9 @@ where the rule switches, against the oracle.
 * one-kernel sort (small systems): tiles above the shared-memory
   capacity, both sides of its 64 chunks; long-range forces against the oracle
   (FP32 5e-6, FP64 1e-8).
+* FFT passes with 256, 512 and 1,024 threads per plane or slab, one and three
+  systems: forces, energy and virial against the oracle within the parity
+  tests' FP32 tolerances (5e-6, 2e-6, 1e-5).
 * tile sort: tiles of a few particles, above the 512-thread switch, and above
   the shared-memory capacity (2,048); permutation bit-exact.
 """
@@ -270,3 +273,31 @@ def test_one_kernel_sort(n, mesh, f64):
     empty = (np.zeros(n, np.uint32), np.zeros(n, np.uint32), np.zeros(0, np.uint32))
     _, F, _ = R.esp(pos, q, prm, nlist=empty)
     assert R.rel_rms(force.double().cpu().numpy()[:, :3], F) <= (1e-8 if f64 else 5e-6)
+
+
+@pytest.mark.parametrize("mesh,copies", [((16, 18, 20), 1), ((20, 24, 30), 1), ((64, 60, 72), 1), ((64, 60, 72), 3),
+                                         ((128, 120, 27), 1)])
+def test_fft_block_sizes(mesh, copies):
+    s = systems.rocksalt(8, seed=sum(mesh))
+    s.pos = s.pos.astype(np.float32).astype(np.float64)
+    nlist = R.neighbor_list(s.pos, s.box, 3.0)
+    b = native.Batch(native.make_params(mesh=mesh), [s.N] * copies, [s.box] * copies)
+    inf = native.Context(native.make_params(mesh=mesh), s.box, s.N).info()
+    pos = torch.zeros((s.N * copies, 4), device="cuda")
+    pos[:, :3] = torch.as_tensor(np.tile(s.pos, (copies, 1)), device="cuda")
+    q = torch.as_tensor(np.tile(s.q, copies), dtype=torch.float32, device="cuda")
+    head = np.concatenate([nlist[0] + k * len(nlist[2]) for k in range(copies)])
+    nl = tuple(torch.as_tensor(a.astype(np.int32), device="cuda")
+               for a in (head, np.tile(nlist[1], copies), np.tile(nlist[2], copies)))
+    force = torch.zeros_like(pos)
+    energy = torch.zeros(copies, dtype=torch.float64, device="cuda")
+    w = torch.zeros((copies, 6), dtype=torch.float64, device="cuda")
+    b.compute(pos, q, force, energy, w, nlist=nl)
+    prm = tables.ESPParams(mesh=mesh, box=tuple(s.box), rcut=inf["rcut"], split=tables.split_cached(inf["c_split"]),
+                           window=tables.window_cached(inf["order"], inf["c_window"], inf["window_degree"]))
+    E, F, W = R.esp(s.pos, s.q, prm, nlist=nlist)
+    f = force.double().cpu().numpy().reshape(copies, s.N, 4)
+    for k in range(copies):
+        assert R.rel_rms(f[k, :, :3], F) <= 5e-6
+        assert abs(energy[k].item() - E) <= 2e-6 * abs(E)
+        assert np.abs(w[k].cpu().numpy() - W).max() <= 1e-5 * np.abs(W).max()
