@@ -16,7 +16,11 @@ constexpr int MAX_D = 15;      // window polynomial degree limit
 constexpr int MAX_QC = 32;     // split polynomial coefficients
 constexpr int ACC_STRIDE = 24; // doubles of per-system accumulators
 constexpr int FFT_MAX_N = 256; // longest 1D transform (2/3/5-smooth)
-constexpr int FFT_B_YZ = 16;   // columns per CTA in the y/z passes
+// Columns per CTA in the y/z passes: 8 (25 KB of shared memory at 200 points, 5
+// CTAs per SM by registers) where 16 let 4 of them wait out their stages (mesh
+// 200^3: z pass 77.5 -> 63.0 us, y passes 38.1 -> 33.7). The x passes keep 8
+// row pairs: with 4 they took 47.7 / 52.9 us instead of 36.3 / 48.2.
+constexpr int FFT_B_YZ = 8;
 constexpr int FFT_B_X = 8;     // row pairs per CTA in the x passes
 constexpr int FFT_SB_X = 9;    // padded line stride of the x passes (bank-conflict free)
 constexpr float INV_4PI_F = 0.0795774715459476678f;
