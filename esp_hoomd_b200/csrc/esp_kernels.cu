@@ -1,7 +1,7 @@
 // ESP hot-path kernels for sm_100a.
 //
 // Stage map to the reference (slweng0321/ESP_HOOMD):
-//   k_bin / k_scan / k_scatter / k_tile_sort : new particle binning + stable
+//   k_bin / k_scan / k_scatter / k_tile_sort(_direct) : new particle binning + stable
 //       sort (nearest reference code: makeFraction+floorf in
 //       src/ESPForceComputeGPU.cu:228-236)
 //   k_spread_mma (tensor-core tiles; default), k_spread_dense, k_spread :
