@@ -192,4 +192,29 @@ struct SegPoly {
         default: return cudaErrorInvalidValue;       \
     }
 
+// Buckets of the per-tile sorts: y origins inside a tile (the tile edge is at most 64), or ranges of
+// particle indices.
+constexpr int SORT_BUCKETS = 64;
+
+// starts of the buckets from their counts (first warp); cnt becomes the fill
+// cursor, a bucket's end once it is filled
+__device__ __forceinline__ void bucket_starts(uint32_t* cnt, uint32_t* beg) {
+    if (threadIdx.x >= 32) return;
+    const int l = threadIdx.x;
+    const uint32_t a = cnt[2 * l], b = cnt[2 * l + 1];
+    uint32_t x = a + b;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
+        if (l >= o) x += y;
+    }
+    beg[2 * l] = x - a - b;
+    beg[2 * l + 1] = x - b;
+    cnt[2 * l] = x - a - b;
+    cnt[2 * l + 1] = x - b;
+}
+
+// shift that puts index offsets up to `range` into the buckets, in order
+__device__ __forceinline__ int index_bucket_shift(uint32_t range) { return max(0, 26 - __clz((int)range)); }
+
 }  // namespace espb

@@ -289,25 +289,6 @@ __device__ __forceinline__ uint32_t sort_key(uint32_t v, const uint32_t* __restr
     return (((rel[v] >> 8) & 255u) << 26) | (v - (uint32_t)p_off);
 }
 
-constexpr int SORT_BUCKETS = 64;  // y origins inside a tile (the tile edge is at most 64)
-
-// starts of the buckets from their counts (first warp); cnt becomes the fill
-// cursor, a bucket's end once it is filled
-__device__ __forceinline__ void bucket_starts(uint32_t* cnt, uint32_t* beg) {
-    if (threadIdx.x >= 32) return;
-    const int l = threadIdx.x;
-    const uint32_t a = cnt[2 * l], b = cnt[2 * l + 1];
-    uint32_t x = a + b;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
-        if (l >= o) x += y;
-    }
-    beg[2 * l] = x - a - b;
-    beg[2 * l + 1] = x - b;
-    cnt[2 * l] = x - a - b;
-    cnt[2 * l + 1] = x - b;
-}
 
 __global__ void __launch_bounds__(512)
     k_tile_sort(const uint32_t* __restrict__ start, const uint32_t* __restrict__ perm_u, uint32_t* __restrict__ perm,
@@ -375,13 +356,16 @@ __global__ void __launch_bounds__(DIRECT_THREADS)
                        uint32_t* __restrict__ perm, const T4* __restrict__ trec, const uint32_t* __restrict__ rel,
                        T4* __restrict__ srec, uint32_t* __restrict__ srel) {
     after_previous();
-    __shared__ uint32_t raw[SORT_CAP], sm[BY_Y ? SORT_CAP : 1];
-    __shared__ uint32_t cnt[SORT_BUCKETS], beg[SORT_BUCKETS], n_in, n_less;
+    __shared__ uint32_t raw[SORT_CAP], sm[SORT_CAP];
+    __shared__ uint32_t cnt[SORT_BUCKETS], beg[SORT_BUCKETS], n_in, n_less, lo, hi;
     constexpr int U = 8;  // keys in flight per thread
     const uint32_t t = blockIdx.x;
     const SysDev& S = sys[tile_sys[t]];
     const int p_off = S.p_off, N = S.N;
-    if (threadIdx.x == 0) n_in = n_less = 0u;
+    if (threadIdx.x == 0) {
+        n_in = n_less = hi = 0u;
+        lo = 0xffffffffu;
+    }
     if (threadIdx.x < SORT_BUCKETS) cnt[threadIdx.x] = 0u;
     __syncthreads();
     uint32_t less = 0;
@@ -429,25 +413,31 @@ __global__ void __launch_bounds__(DIRECT_THREADS)
         }
         return;
     }
-    const uint32_t* src = raw;
-    if constexpr (BY_Y) {
-        for (uint32_t i = threadIdx.x; i < n; i += DIRECT_THREADS) atomicAdd(&cnt[(rel[raw[i]] >> 8) & 255u], 1u);
+    // bucket of a particle: its y origin, or its index's range
+    int sh = 0;
+    if constexpr (!BY_Y) {
+        for (uint32_t i = threadIdx.x; i < n; i += DIRECT_THREADS) {
+            atomicMin(&lo, raw[i]);
+            atomicMax(&hi, raw[i]);
+        }
         __syncthreads();
-        bucket_starts(cnt, beg);
-        __syncthreads();
-        for (uint32_t i = threadIdx.x; i < n; i += DIRECT_THREADS) sm[atomicAdd(&cnt[(rel[raw[i]] >> 8) & 255u], 1u)] = raw[i];
-        __syncthreads();
-        src = sm;
+        sh = index_bucket_shift(hi - lo);
     }
+    auto bucket = [&](uint32_t v) { return BY_Y ? (rel[v] >> 8) & 255u : (v - lo) >> sh; };
+    for (uint32_t i = threadIdx.x; i < n; i += DIRECT_THREADS) atomicAdd(&cnt[bucket(raw[i])], 1u);
+    __syncthreads();
+    bucket_starts(cnt, beg);
+    __syncthreads();
+    for (uint32_t i = threadIdx.x; i < n; i += DIRECT_THREADS) sm[atomicAdd(&cnt[bucket(raw[i])], 1u)] = raw[i];
+    __syncthreads();
     for (uint32_t i = threadIdx.x; i < n; i += DIRECT_THREADS) {
-        const uint32_t v = src[i], rl = rel[v], bk = (rl >> 8) & 255u;
-        const uint32_t b0 = BY_Y ? beg[bk] : 0u, b1 = BY_Y ? cnt[bk] : n;
+        const uint32_t v = sm[i], bk = bucket(v), b0 = beg[bk], b1 = cnt[bk];
         const T4 rec = trec[v];
         uint32_t r = b0;
-        for (uint32_t j = b0; j < b1; ++j) r += src[j] < v ? 1u : 0u;
+        for (uint32_t j = b0; j < b1; ++j) r += sm[j] < v ? 1u : 0u;
         perm[s0 + r] = v;
         srec[s0 + r] = rec;
-        srel[s0 + r] = rl;
+        srel[s0 + r] = rel[v];
     }
 }
 
