@@ -214,6 +214,15 @@ __device__ __forceinline__ void bucket_starts(uint32_t* cnt, uint32_t* beg) {
     cnt[2 * l + 1] = x - b;
 }
 
+// Entries of a neighbour row that may be read: n, or the row capacity when
+// *limit is set (the library built the rows and one of them overflowed, so that
+// n may be a count its row does not hold).
+__device__ __forceinline__ uint32_t row_entries(uint32_t n, const uint32_t* __restrict__ limit) {
+    if (!limit) return n;
+    const uint32_t l = *limit;
+    return l ? min(n, l) : n;
+}
+
 // shift that puts index offsets up to `range` into the buckets, in order
 __device__ __forceinline__ int index_bucket_shift(uint32_t range) { return max(0, 26 - __clz((int)range)); }
 

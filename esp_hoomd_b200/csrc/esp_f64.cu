@@ -725,8 +725,8 @@ template <int TPP, int NQ, bool VIR>
 __global__ void __launch_bounds__(256, VIR ? 3 : 4)
     k64_pair(const int2* __restrict__ chunks, const SysDev* __restrict__ sys, const ParamSet* __restrict__ psets,
              const PairCoef64 pc, const double4* __restrict__ posq, const uint32_t* __restrict__ head,
-             const uint32_t* __restrict__ nn, const uint32_t* __restrict__ nlist, double4* __restrict__ force,
-             double* __restrict__ acc) {
+             const uint32_t* __restrict__ nn, const uint32_t* __restrict__ nlist,
+             const uint32_t* __restrict__ row_limit, double4* __restrict__ force, double* __restrict__ acc) {
     __shared__ double red[32 * 7];
     constexpr int SUB = TPP / 8;  // CTAs per chunk of 32 particles
     const int2 ch = chunks[blockIdx.x / SUB];
@@ -786,7 +786,7 @@ __global__ void __launch_bounds__(256, VIR ? 3 : 4)
     if (valid) {
         // one neighbour per lane and step: streaming 16-byte index segments
         // with four gathers in flight per lane measured 2-6% slower here
-        const uint32_t n = nn[i], h = head[i];
+        const uint32_t n = row_entries(nn[i], row_limit), h = head[i];
         // the next neighbour index is loaded one step ahead of its gather
         uint32_t jn = sub < n ? nlist[h + sub] : 0u;
         if (interior)
@@ -834,7 +834,7 @@ static void launch64_pair_t(const Launch64& b, double4* force, cudaStream_t st) 
     // the series padded with zero terms to the next compiled length
 #define ESPB_PAIR64(NQ)                                                                                       \
     k64_pair<TPP, NQ, VIR><<<grid, 256, 0, st>>>(b.pchunks, a.sys, a.psets, b.pc, b.posq, a.nl_head, a.nl_n, \
-                                                 a.nl_list, force, a.acc)
+                                                 a.nl_list, a.row_limit, force, a.acc)
     if (b.nq <= 12) ESPB_PAIR64(12);
     else if (b.nq <= 14) ESPB_PAIR64(14);
     else if (b.nq <= 16) ESPB_PAIR64(16);

@@ -297,10 +297,24 @@ struct esp_batch {
         uint32_t *d_ckey = nullptr, *d_ccount = nullptr, *d_cstart = nullptr, *d_cperm = nullptr,
                  *d_slot2idx = nullptr, *d_idx2slot = nullptr, *d_scan = nullptr;
         float4 *d_wpos = nullptr, *d_cpos = nullptr;
-        int* d_overflow = nullptr;  // [flag, largest row] of the last build
     } cg_nl, cg_pl;
     int setup_cells(CellGrid& g, double rlist, int cap);
     NlistArgs nlist_args(CellGrid& g, const float* pos4, double rlist, int cap) const;
+    // overflow states (NLIST_STATE words each) of the last HOOMD-layout and
+    // pair-list builds; they outlive cell grids and plans, captured steps
+    // hold their address
+    DevAlloc ovmem;
+    int *d_nl_state = nullptr, *d_pl_state = nullptr;
+    uint32_t* d_nn_limited = nullptr;
+    int nn_limited_n = 0;
+    int list_states();
+    // how many entries the rows of (head, nl) hold when the library's last
+    // build wrote them and overflowed; that build may still be running
+    const uint32_t* row_limit(const unsigned* head, const unsigned* nl) const {
+        return d_nl_state && head && head == nl_last_head && nl == nl_last_nl
+                   ? reinterpret_cast<const uint32_t*>(d_nl_state) + 2
+                   : nullptr;
+    }
     // the library's pair list: rows by cell-sorted slot, and the
     // slot-ordered positions the bin stage writes for it
     DevAlloc plmem;
@@ -363,11 +377,12 @@ struct esp_batch {
         bool with_energy;
         bool f64 = false;                               // md_run_f64 steps
         double lj_eps = 0, lj_sigma = 0, lj_rcut = 0;   // md_run_f64's Lennard-Jones term (sigma 0: none)
+        const void* row_limit = nullptr;                // of the rows head, nl
         bool operator==(const GraphKey& o) const {
             return pos == o.pos && vel == o.vel && q == o.q && head == o.head && nn == o.nn && nl == o.nl &&
                    force == o.force && energy == o.energy && virial == o.virial && dt == o.dt &&
                    with_energy == o.with_energy && f64 == o.f64 && lj_eps == o.lj_eps && lj_sigma == o.lj_sigma &&
-                   lj_rcut == o.lj_rcut;
+                   lj_rcut == o.lj_rcut && row_limit == o.row_limit;
         }
     };
     // captured MD steps, one per distinct set of caller pointers; a few
@@ -863,6 +878,7 @@ int esp_batch::compute_f64(cudaStream_t st, const double* pos4, const double* q,
     a.nl_head = head;
     a.nl_n = nn;
     a.nl_list = nl;
+    a.row_limit = row_limit(head, nl);
     a.ex_n = ex_n;
     a.ex_list = ex_list;
     a.ex_pitch = ex_pitch;
@@ -1020,7 +1036,9 @@ int esp_batch::compute(cudaStream_t st, const float* pos4, const float* q, const
     a.nl_head = head;
     a.nl_n = nn;
     a.nl_list = nl;
+    a.row_limit = row_limit(head, nl);
     const bool lr = flags & ESP_LONG_RANGE, sr = flags & ESP_SHORT_RANGE;
+    if (sr && a.row_limit) a.nn_limited = d_nn_limited;
     a.accumulate = lr ? 1 : 0;
     a.add_bg = lr ? 1 : 0;
     AccGuard acc_guard{d_acc, (size_t)nsys * ACC_STRIDE * sizeof(double), st};
@@ -1113,7 +1131,8 @@ int esp_batch::md_run(cudaStream_t st, float* pos4, float* vel4, const float* q,
         timer.end(st);
         return rc;
     };
-    const GraphKey key{pos4, vel4, q, head, nn, nl, force4, energy, virial, dt, false};
+    GraphKey key{pos4, vel4, q, head, nn, nl, force4, energy, virial, dt, false};
+    key.row_limit = row_limit(head, nl);
     return run_steps(st, key, step, nsteps, use_graph && !timer.on);
 }
 
@@ -1136,8 +1155,8 @@ int esp_batch::md_run_f64(cudaStream_t st, double* pos4, double* vel4, const dou
         rc = compute_f64(st, pos4, q, head, nn, nl, force4, energy, virial, ESP_ALL);
         if (rc) return rc;
         if (lj)
-            ESPB_CK(launch_lj(d_chunks, n_chunks, d_sys, pos4, head, nn, nl, lj_eps, lj_sigma, lj_rcut, force4, energy,
-                              true, st));
+            ESPB_CK(launch_lj(d_chunks, n_chunks, d_sys, pos4, head, nn, nl, row_limit(head, nl), lj_eps, lj_sigma,
+                              lj_rcut, force4, energy, true, st));
         return nve2(st, pos4, vel4, force4, dt, true);
     };
     GraphKey key{pos4, vel4, q, head, nn, nl, force4, energy, virial, dt, false};
@@ -1145,6 +1164,7 @@ int esp_batch::md_run_f64(cudaStream_t st, double* pos4, double* vel4, const dou
     key.lj_eps = lj ? lj_eps : 0.0;
     key.lj_sigma = lj ? lj_sigma : 0.0;
     key.lj_rcut = lj ? lj_rcut : 0.0;
+    key.row_limit = row_limit(head, nl);
     return run_steps(st, key, step, nsteps, use_graph != 0);
 }
 
@@ -1284,13 +1304,28 @@ int esp_batch::setup_cells(CellGrid& g, double rlist, int cap) {
         (rc = g.mem.get(g.d_cperm, totN)) ||
         (rc = g.mem.get(g.d_slot2idx, totN)) || (rc = g.mem.get(g.d_idx2slot, totN)) ||
         (rc = g.mem.get(g.d_wpos, totN)) ||
-        (rc = g.mem.get(g.d_cpos, totN)) || (rc = g.mem.get(g.d_overflow, 2)))
+        (rc = g.mem.get(g.d_cpos, totN)))
         return rc;
     ESPB_CK(cudaMemcpy(g.d_cells, g.h_cells.data(), nsys * sizeof(CellDev), cudaMemcpyHostToDevice));
     ESPB_CK(cudaMemcpy(g.d_cell_sys, cell_sys.data(), g.n_cells * sizeof(int), cudaMemcpyHostToDevice));
     ESPB_CK(cudaMemset(g.d_ccount, 0, g.n_cells * sizeof(uint32_t)));
     g.rlist = rlist;
     g.cap = cap;
+    return 0;
+}
+
+int esp_batch::list_states() {
+    int rc = 0;
+    if (totN > nn_limited_n) {
+        if ((rc = ovmem.get(d_nn_limited, totN))) return rc;
+        nn_limited_n = totN;
+    }
+    if (d_nl_state) return 0;
+    int* p = nullptr;
+    if ((rc = ovmem.get(p, 2 * NLIST_STATE))) return rc;
+    ESPB_CK(cudaMemset(p, 0, 2 * NLIST_STATE * sizeof(int)));
+    d_nl_state = p;
+    d_pl_state = p + NLIST_STATE;
     return 0;
 }
 
@@ -1316,7 +1351,6 @@ NlistArgs esp_batch::nlist_args(CellGrid& g, const float* pos4, double rlist, in
     a.cpos = g.d_cpos;
     a.rlist2 = (float)(rlist * rlist);
     a.cap = cap;
-    a.overflow = g.d_overflow;
     a.ex_n = ex_n;
     a.ex_list = ex_list;
     a.ex_pitch = ex_pitch;
@@ -1329,9 +1363,11 @@ int esp_batch::build_nlist(cudaStream_t st, const float* pos4, double rlist, int
     if (!pos4 || !head || !nn || !nl) return fail(ESP_ERR_INVALID, "null pointer");
     if ((double)totN * cap >= 4294967296.0)
         return fail(ESP_ERR_UNSUPPORTED, "HOOMD-layout rows address 32-bit offsets: totN * cap must be below 2^32");
-    int rc = setup_cells(cg_nl, rlist, cap);
+    int rc = list_states();
+    if (!rc) rc = setup_cells(cg_nl, rlist, cap);
     if (rc) return rc;
     NlistArgs a = nlist_args(cg_nl, pos4, rlist, cap);
+    a.overflow = d_nl_state;
     a.head = head;
     a.nn = nn;
     a.nl = nl;
@@ -1343,7 +1379,7 @@ int esp_batch::build_nlist(cudaStream_t st, const float* pos4, double rlist, int
     timer.end(st);
     // the overflow flag is read lazily (esp_batch_nlist_check, or the next
     // compute / md_run over these rows): no host synchronisation here
-    ESPB_CK(cudaMemcpyAsync(h_nl_ovf, cg_nl.d_overflow, 2 * sizeof(int), cudaMemcpyDeviceToHost, st));
+    ESPB_CK(cudaMemcpyAsync(h_nl_ovf, d_nl_state, 2 * sizeof(int), cudaMemcpyDeviceToHost, st));
     ESPB_CK(cudaEventRecord(nl_ev, st));
     nl_last_head = head;
     nl_last_nl = nl;
@@ -1379,7 +1415,8 @@ int esp_batch::build_pairlist(cudaStream_t st, const float* pos4, double rlist, 
     if (f64) return fail(ESP_ERR_UNSUPPORTED, "the library's pair list serves the FP32 path");
     if ((double)totN * cap >= 4294967296.0) return fail(ESP_ERR_UNSUPPORTED, "pair list of 2^32 entries or more");
     if (rlist != cg_pl.rlist) drop_graphs();  // captured steps hold the previous cell grid's slot maps
-    int rc = setup_cells(cg_pl, rlist, cap);
+    int rc = list_states();
+    if (!rc) rc = setup_cells(cg_pl, rlist, cap);
     if (rc) return rc;
     if (pl_cap != cap) {
         plmem.release();
@@ -1396,12 +1433,14 @@ int esp_batch::build_pairlist(cudaStream_t st, const float* pos4, double rlist, 
     a.head = d_pl_head;
     a.nn = d_pl_nn;
     a.nl = d_pl_nl;
+    a.overflow = d_pl_state;
+    a.clamp_counts = true;
     a.sorted = true;
     timer.begin(ESP_STAGE_NLIST, st);
     ESPB_CK(launch_nlist(a, st));
     timer.end(st);
     // the overflow flag is read lazily: no host synchronisation here
-    ESPB_CK(cudaMemcpyAsync(h_pl_ovf, cg_pl.d_overflow, 2 * sizeof(int), cudaMemcpyDeviceToHost, st));
+    ESPB_CK(cudaMemcpyAsync(h_pl_ovf, d_pl_state, 2 * sizeof(int), cudaMemcpyDeviceToHost, st));
     ESPB_CK(cudaEventRecord(pl_ev, st));
     pl.slot2idx = cg_pl.d_slot2idx;
     pl.idx2slot = cg_pl.d_idx2slot;
@@ -1928,8 +1967,8 @@ int esp_batch_lj(esp_batch* b, void* stream, const float* pos4, const unsigned* 
                  const unsigned* nlist, double epsilon, double sigma, double r_cut, float* force4, double* energy) {
     if (!b || !pos4 || !head || !n_neigh || !nlist || !force4) return fail(ESP_ERR_INVALID, "null argument");
     if (!(sigma > 0) || !(r_cut > 0)) return fail(ESP_ERR_INVALID, "sigma and r_cut must be positive");
-    ESPB_CK(launch_lj(b->d_chunks, b->n_chunks, b->d_sys, pos4, head, n_neigh, nlist, epsilon, sigma, r_cut, force4,
-                      energy, false, (cudaStream_t)stream));
+    ESPB_CK(launch_lj(b->d_chunks, b->n_chunks, b->d_sys, pos4, head, n_neigh, nlist, b->row_limit(head, nlist),
+                      epsilon, sigma, r_cut, force4, energy, false, (cudaStream_t)stream));
     return 0;
 }
 
@@ -1938,8 +1977,8 @@ int esp_batch_lj_f64(esp_batch* b, void* stream, const double* pos4, const unsig
                      double* energy) {
     if (!b || !pos4 || !head || !n_neigh || !nlist || !force4) return fail(ESP_ERR_INVALID, "null argument");
     if (!(sigma > 0) || !(r_cut > 0)) return fail(ESP_ERR_INVALID, "sigma and r_cut must be positive");
-    ESPB_CK(launch_lj(b->d_chunks, b->n_chunks, b->d_sys, pos4, head, n_neigh, nlist, epsilon, sigma, r_cut, force4,
-                      energy, true, (cudaStream_t)stream));
+    ESPB_CK(launch_lj(b->d_chunks, b->n_chunks, b->d_sys, pos4, head, n_neigh, nlist, b->row_limit(head, nlist),
+                      epsilon, sigma, r_cut, force4, energy, true, (cudaStream_t)stream));
     return 0;
 }
 

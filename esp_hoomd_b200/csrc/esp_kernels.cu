@@ -33,7 +33,9 @@ __global__ void k_bin(const int2* __restrict__ chunks, const SysDev* __restrict_
                       const float4* __restrict__ pos_in, const float* __restrict__ q_in,
                       float4* __restrict__ posq, float4* __restrict__ trec, uint32_t* __restrict__ rel,
                       uint32_t* __restrict__ key, uint32_t* __restrict__ tile_count, double* __restrict__ acc,
-                      const uint32_t* __restrict__ idx2slot, float4* __restrict__ spos) {
+                      const uint32_t* __restrict__ idx2slot, float4* __restrict__ spos,
+                      const uint32_t* __restrict__ nn, const uint32_t* __restrict__ row_limit,
+                      uint32_t* __restrict__ nn_limited) {
     __shared__ double red[32 * 2];
     const int2 ch = chunks[blockIdx.x];
     const SysDev S = sys[ch.x];
@@ -73,6 +75,7 @@ __global__ void k_bin(const int2* __restrict__ chunks, const SysDev* __restrict_
         posq[i] = make_float4(x, y, z, q);
         // the pair list's slot-ordered copy (rows of that list index it)
         if (spos) spos[idx2slot[i]] = make_float4(x, y, z, q);
+        if (nn_limited) nn_limited[i] = row_entries(nn[i], row_limit);
         trec[i] = make_float4(tt[0], tt[1], tt[2], q);
         rel[i] = (uint32_t)(i0m[0] - tx * T) | ((uint32_t)(i0m[1] - ty * T) << 8) |
                  ((uint32_t)(i0m[2] - tz * T) << 16);
@@ -2269,7 +2272,7 @@ cudaError_t launch_bin(const LaunchArgs& a, cudaStream_t st) {
     if (a.n_chunks == 0) return cudaSuccess;
     k_bin<<<a.n_chunks, 256, 0, st>>>(a.chunks, a.sys, a.P, a.T, a.pos_in, a.q_in, a.posq, a.trec, a.rel, a.key,
                                       a.tile_count, a.acc, a.plist ? a.plist->idx2slot : nullptr,
-                                      a.plist ? a.plist->spos : nullptr);
+                                      a.plist ? a.plist->spos : nullptr, a.nl_n, a.row_limit, a.nn_limited);
     return cudaGetLastError();
 }
 

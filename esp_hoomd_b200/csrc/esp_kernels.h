@@ -102,6 +102,11 @@ struct LaunchArgs {
     const uint32_t* nl_head = nullptr;
     const uint32_t* nl_n = nullptr;
     const uint32_t* nl_list = nullptr;
+    const uint32_t* row_limit = nullptr;  // entries of a row that may be read (row_entries; NULL: n_neigh)
+    // with a row limit the FP32 bin stage writes the limited counts here and the
+    // pair term reads them (a limit inside k_pair costs it 1-4%: its register
+    // allocation is at the edge)
+    uint32_t* nn_limited = nullptr;
     // HOOMD ForceCompute outputs: per-particle virial virial_pp[k * vpp_pitch + i]
     // (k = xx, xy, xz, yy, yz, zz; pair and exclusion terms, cleared by the
     // host first) and per system the terms no particle owns,

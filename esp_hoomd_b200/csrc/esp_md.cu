@@ -117,14 +117,16 @@ __device__ __forceinline__ uint32_t nl_scan(const float4* __restrict__ cand, int
 // particle. SORTED = true: the library's pair list -- the same layout indexed
 // by the cell-sorted slot (row of slot s at nl_off + local s * cap, head and
 // nn by slot), entries local slots. Rows longer than cap keep their first cap
-// entries and set the overflow flag; overflow[1] receives the longest row.
+// entries and set the overflow flag; overflow[1] receives the longest row and
+// overflow[2] the row capacity. nn holds the counts up to nn_max.
 template <bool SORTED>
 __global__ void __launch_bounds__(NL_THREADS) k_nlist_cta(const int* __restrict__ cell_sys, const SysDev* __restrict__ sys,
                                                           const CellDev* __restrict__ cells,
                                                       const uint32_t* __restrict__ cstart,
                                                       const float4* __restrict__ cpos, float rlist2, int cap,
                                                       uint32_t* __restrict__ head, uint32_t* __restrict__ nn,
-                                                      uint32_t* __restrict__ nl, int* __restrict__ overflow) {
+                                                      uint32_t* __restrict__ nl, int* __restrict__ overflow,
+                                                      uint32_t nn_max) {
     __shared__ float4 cand[NL_STAGE];
     __shared__ CellNbhd nb;
     const uint32_t cidx = blockIdx.x;
@@ -183,10 +185,11 @@ __global__ void __launch_bounds__(NL_THREADS) k_nlist_cta(const int* __restrict_
         }
         if (active) {
             head[key] = (uint32_t)hrow;
-            nn[key] = SORTED ? min(cnt, (uint32_t)cap) : cnt;
+            nn[key] = min(cnt, nn_max);
             if (cnt > (uint32_t)cap) {
                 atomicOr(overflow, 1);
                 atomicMax(overflow + 1, (int)cnt);
+                overflow[2] = cap;
             }
         }
     }
@@ -257,9 +260,10 @@ __device__ __forceinline__ void nl_test(NlGroup& g, int ng, float4 c, uint32_t s
 // particle. SORTED = true: the library's pair list -- the same layout indexed
 // by the cell-sorted slot (row of slot s at nl_off + local s * cap, head and
 // nn by slot), entries local slots. Rows longer than cap keep their first cap
-// entries, the overflow flag is set and overflow[1] receives the longest row;
-// nn holds the true count in HOOMD rows and the kept entries in the pair list,
-// which the pair kernel walks. EX: the excluded partners are left out of the
+// entries, the overflow flag is set, overflow[1] receives the longest row and
+// overflow[2] the row capacity. nn holds the counts up to nn_max: the true ones
+// in a caller's HOOMD rows, whose readers then take no more than overflow[2]
+// entries, the kept ones in the pair list and in a server's rows. EX: the excluded partners are left out of the
 // rows (a row whose hits exceed cap before that counts as overflowing).
 template <bool SORTED, bool EX>
 __global__ void __launch_bounds__(32 * NL_WARPS, EX ? 4 : 7)
@@ -267,7 +271,8 @@ __global__ void __launch_bounds__(32 * NL_WARPS, EX ? 4 : 7)
             const CellDev* __restrict__ cells, const uint32_t* __restrict__ cstart, const float4* __restrict__ cpos,
             float rlist2, uint32_t cap, uint32_t* __restrict__ head, uint32_t* __restrict__ nn,
             uint32_t* __restrict__ nl, int* __restrict__ overflow, const uint32_t* __restrict__ ex_n,
-            const uint32_t* __restrict__ ex_list, int ex_pitch, const uint32_t* __restrict__ idx2slot) {
+            const uint32_t* __restrict__ ex_list, int ex_pitch, const uint32_t* __restrict__ idx2slot,
+            uint32_t nn_max) {
     __shared__ uint4 srow[NL_WARPS][25];     // (dz, dy) row: its two pieces' slots (see below), first candidate
     __shared__ float2 sshift[NL_WARPS][25];  // its periodic image along y and z
     __shared__ uint32_t soff[NL_WARPS][28];  // first candidate of each row, then the total
@@ -414,10 +419,11 @@ __global__ void __launch_bounds__(32 * NL_WARPS, EX ? 4 : 7)
             }
         if (lane < ng) {
             head[mykey] = myrow;
-            nn[mykey] = SORTED ? min(cnt, cap) : cnt;
+            nn[mykey] = min(cnt, nn_max);
             if (hits > cap) {
                 atomicOr(overflow, 1);
                 atomicMax(overflow + 1, (int)hits);
+                overflow[2] = (int)cap;
             }
         }
         __syncwarp();
@@ -515,8 +521,9 @@ __global__ void k_nve2(const int2* __restrict__ chunks, const SysDev* __restrict
 template <typename T4, typename T, int TPP>
 __global__ void __launch_bounds__(256)
     k_lj(const int2* __restrict__ chunks, const SysDev* __restrict__ sys, const T4* __restrict__ pos,
-         const uint32_t* __restrict__ head, const uint32_t* __restrict__ nn, const uint32_t* __restrict__ nl, T eps,
-         T sig2, T rc2, T4* __restrict__ force, double* __restrict__ energy) {
+         const uint32_t* __restrict__ head, const uint32_t* __restrict__ nn, const uint32_t* __restrict__ nl,
+         const uint32_t* __restrict__ row_limit, T eps, T sig2, T rc2, T4* __restrict__ force,
+         double* __restrict__ energy) {
     __shared__ double red[32];
     const int2 ch = chunks[blockIdx.x / TPP];
     const SysDev& S = sys[ch.x];
@@ -528,7 +535,7 @@ __global__ void __launch_bounds__(256)
     T fx = 0, fy = 0, fz = 0, en = 0;
     if (valid) {
         const T4 pi = pos[i];
-        const uint32_t h = head[i], n = nn[i];
+        const uint32_t h = head[i], n = row_entries(nn[i], row_limit);
         uint32_t jn = sub < n ? nl[h + sub] : 0u;
         for (uint32_t k = sub; k < n; k += TPP) {
             const T4 pj = pos[po + (int)jn];
@@ -619,26 +626,30 @@ constexpr int LJ_WARP_CHUNKS = 37;  // 148 SMs x 64 warps / 256 particles
 
 template <typename T4, typename T>
 static void lj_launch(const int2* chunks, int n_chunks, const SysDev* sys, const void* pos, const uint32_t* head,
-                      const uint32_t* nn, const uint32_t* nl, double eps, double sigma, double rcut, void* force,
-                      double* energy, cudaStream_t st) {
+                      const uint32_t* nn, const uint32_t* nl, const uint32_t* row_limit, double eps, double sigma,
+                      double rcut, void* force, double* energy, cudaStream_t st) {
     const T e = (T)eps, s2 = (T)(sigma * sigma), r2 = (T)(rcut * rcut);
     // a warp per particle while that does not oversubscribe the GPU (148 SMs
     // x 64 warps, 256-particle chunks), else 8 lanes: fewer idle lanes in the
     // last pass over a row and cheaper reductions
     if (n_chunks <= LJ_WARP_CHUNKS)
-        k_lj<T4, T, 32><<<n_chunks * 32, 256, 0, st>>>(chunks, sys, (const T4*)pos, head, nn, nl, e, s2, r2, (T4*)force, energy);
+        k_lj<T4, T, 32><<<n_chunks * 32, 256, 0, st>>>(chunks, sys, (const T4*)pos, head, nn, nl, row_limit, e, s2, r2,
+                                                       (T4*)force, energy);
     else
-        k_lj<T4, T, 8><<<n_chunks * 8, 256, 0, st>>>(chunks, sys, (const T4*)pos, head, nn, nl, e, s2, r2, (T4*)force, energy);
+        k_lj<T4, T, 8><<<n_chunks * 8, 256, 0, st>>>(chunks, sys, (const T4*)pos, head, nn, nl, row_limit, e, s2, r2,
+                                                     (T4*)force, energy);
 }
 
 cudaError_t launch_lj(const int2* chunks, int n_chunks, const SysDev* sys, const void* pos, const uint32_t* head,
-                      const uint32_t* nn, const uint32_t* nl, double eps, double sigma, double rcut, void* force,
-                      double* energy, bool f64, cudaStream_t st) {
+                      const uint32_t* nn, const uint32_t* nl, const uint32_t* row_limit, double eps, double sigma,
+                      double rcut, void* force, double* energy, bool f64, cudaStream_t st) {
     if (n_chunks == 0) return cudaSuccess;
     if (f64)
-        lj_launch<double4, double>(chunks, n_chunks, sys, pos, head, nn, nl, eps, sigma, rcut, force, energy, st);
+        lj_launch<double4, double>(chunks, n_chunks, sys, pos, head, nn, nl, row_limit, eps, sigma, rcut, force, energy,
+                                   st);
     else
-        lj_launch<float4, float>(chunks, n_chunks, sys, pos, head, nn, nl, eps, sigma, rcut, force, energy, st);
+        lj_launch<float4, float>(chunks, n_chunks, sys, pos, head, nn, nl, row_limit, eps, sigma, rcut, force, energy,
+                                 st);
     return cudaGetLastError();
 }
 
@@ -652,7 +663,7 @@ cudaError_t launch_nve64(int half, const int2* chunks, int n_chunks, const SysDe
 
 cudaError_t launch_nlist(const NlistArgs& a, cudaStream_t st) {
     if (a.n_chunks == 0) return cudaSuccess;
-    cudaError_t e = cudaMemsetAsync(a.overflow, 0, 2 * sizeof(int), st);
+    cudaError_t e = cudaMemsetAsync(a.overflow, 0, NLIST_STATE * sizeof(int), st);
     if (e != cudaSuccess) return e;
     k_cell_bin<<<a.n_chunks, 256, 0, st>>>(a.chunks, a.sys, a.cells, a.pos, a.ckey, a.ccount, a.wpos);
     if ((e = launch_scan(a.ccount, a.cstart, a.n_cells, a.scan_ws, st)) != cudaSuccess) return e;
@@ -660,6 +671,7 @@ cudaError_t launch_nlist(const NlistArgs& a, cudaStream_t st) {
         return e;
     k_cell_sort<<<(a.total + 255) / 256, 256, 0, st>>>(a.total, a.ckey, a.cstart, a.perm_u, a.wpos, a.cpos, a.slot2idx,
                                                        a.idx2slot);
+    const uint32_t nn_max = a.clamp_counts ? (uint32_t)a.cap : 0xffffffffu;
     if (a.half) {
         // one warp per group of NL_GROUP particles in a cell of the mean occupancy
         const dim3 grid((a.n_cells + NL_WARPS - 1) / NL_WARPS,
@@ -668,11 +680,11 @@ cudaError_t launch_nlist(const NlistArgs& a, cudaStream_t st) {
                                    : (a.ex_n ? k_nlist<false, true> : k_nlist<false, false>);
         rows<<<grid, 32 * NL_WARPS, 0, st>>>(a.cell_sys, a.n_cells, a.sys, a.cells, a.cstart, a.cpos, a.rlist2,
                                              (uint32_t)a.cap, a.head, a.nn, a.nl, a.overflow, a.ex_n, a.ex_list,
-                                             a.ex_pitch, a.idx2slot);
+                                             a.ex_pitch, a.idx2slot, nn_max);
     } else {
         const auto rows = a.sorted ? k_nlist_cta<true> : k_nlist_cta<false>;
         rows<<<a.n_cells, NL_THREADS, 0, st>>>(a.cell_sys, a.sys, a.cells, a.cstart, a.cpos, a.rlist2, a.cap, a.head,
-                                               a.nn, a.nl, a.overflow);
+                                               a.nn, a.nl, a.overflow, nn_max);
     }
     const int done = a.half ? NL_MAXEX : 0;  // exclusions per particle left out already
     if (a.ex_n && a.ex_pitch > done) {

@@ -8,6 +8,8 @@
 
 namespace espb {
 
+constexpr int NLIST_STATE = 3;
+
 // Cells of edge >= rlist, or >= rlist / 2 (nlist_half_cells).
 struct CellDev {
     int ncx, ncy, ncz, c_off;  // cell grid and first cell
@@ -37,7 +39,10 @@ struct NlistArgs {
     uint32_t* head = nullptr;
     uint32_t* nn = nullptr;
     uint32_t* nl = nullptr;
-    int* overflow = nullptr;
+    int* overflow = nullptr;  // NLIST_STATE words: overflow flag, longest row, row capacity once a row overflowed (else 0)
+    // false: nn holds the true counts, above cap too (the reader limits them by
+    // overflow[2]); true: at most cap
+    bool clamp_counts = false;
     uint32_t* slot2idx = nullptr;  // cell-sorted slot -> particle (written by the cell sort; may be NULL)
     uint32_t* idx2slot = nullptr;  // particle -> cell-sorted slot (NULL only without exclusions)
     // true: the library's pair list -- rows, head and counts indexed by the
@@ -68,8 +73,8 @@ cudaError_t launch_nve1(const int2* chunks, int n_chunks, const SysDev* sys, flo
 cudaError_t launch_nve2(const int2* chunks, int n_chunks, const SysDev* sys, float4* vel, const float4* force,
                         float dt, cudaStream_t st);
 cudaError_t launch_lj(const int2* chunks, int n_chunks, const SysDev* sys, const void* pos, const uint32_t* head,
-                      const uint32_t* nn, const uint32_t* nl, double eps, double sigma, double rcut, void* force,
-                      double* energy, bool f64, cudaStream_t st);
+                      const uint32_t* nn, const uint32_t* nl, const uint32_t* row_limit, double eps, double sigma,
+                      double rcut, void* force, double* energy, bool f64, cudaStream_t st);
 cudaError_t launch_nve64(int half, const int2* chunks, int n_chunks, const SysDev* sys, double4* pos, double4* vel,
                          const double4* force, double dt, cudaStream_t st, const int2* skip = nullptr);
 // Rigid (O, H, H) molecules (esp_settle.cu): work items {system, first atom

@@ -140,7 +140,7 @@ static cudaError_t launch_pair_t(const LaunchArgs& a, cudaStream_t st) {
     const PairList* pl = a.plist;
     const float4* posq = pl ? pl->spos : a.posq;
     const uint32_t* head = pl ? pl->head : a.nl_head;
-    const uint32_t* nn = pl ? pl->nn : a.nl_n;
+    const uint32_t* nn = pl ? pl->nn : (a.nn_limited ? a.nn_limited : a.nl_n);
     const uint32_t* nl = pl ? pl->nl : a.nl_list;
     const uint32_t* outidx = pl ? pl->slot2idx : nullptr;
 #define ESPB_PAIR(NQ)                                                                                          \

@@ -1,0 +1,135 @@
+"""Calls that go wrong leave the caller's results and the library's memory sound.
+
+* rows longer than their capacity, in an evaluation that is queued before the
+  host can know of the overflow: every term reads the entries that the rows
+  hold, no more (the same bits as over a list cut to the capacity by the caller);
+* a served request whose rows overflow fails alone.
+"""
+import numpy as np
+import pytest
+
+torch = pytest.importorskip("torch")
+pytestmark = pytest.mark.gpu
+
+from esp_hoomd_b200 import native, systems  # noqa: E402
+from esp_hoomd_b200._lib import ESP_SHORT_RANGE, EspError  # noqa: E402
+
+RLIST, CAP, SHORT = 3.4, 256, 64  # the lattice's rows hold about 164 entries
+
+
+def _system(n=12, seed=31):
+    s = systems.rocksalt(n, seed=seed)
+    p4 = np.zeros((s.N, 4), np.float32)
+    p4[:, :3] = s.pos
+    v4 = np.zeros((s.N, 4), np.float32)
+    v4[:, :3] = s.vel
+    v4[:, 3] = s.mass
+    return s, torch.as_tensor(p4, device="cuda"), torch.as_tensor(v4, device="cuda"), \
+        torch.as_tensor(s.q, dtype=torch.float32, device="cuda")
+
+
+def _rows(n, cap):
+    return (torch.zeros(n, dtype=torch.int32, device="cuda"), torch.zeros(n, dtype=torch.int32, device="cuda"),
+            torch.zeros(n * cap, dtype=torch.int32, device="cuda"))
+
+
+def _overflowing(b, pos, short):
+    # the build waits behind a sleeping stream, so that it cannot have completed
+    # when the caller's evaluation is queued (a build with another capacity than
+    # the last one's waits for the stream: the first of the two)
+    b.build_nlist(pos, RLIST, SHORT, *_rows(pos.shape[0], SHORT))
+    torch.cuda._sleep(100_000_000)
+    b.build_nlist(pos, RLIST, SHORT, *short)
+
+
+def _cut(rows):
+    return rows[0].clone(), rows[1].clamp(max=SHORT), rows[2].clone()
+
+
+@pytest.mark.parametrize("n", [12, 46])  # rows of the warp-per-cell and of the CTA-per-cell kernel
+@pytest.mark.parametrize("term", ["pair", "pair64", "lj", "lj64"])
+def test_overflowed_rows_are_read_to_their_capacity(term, n):
+    f64 = term.endswith("64")
+    dt = torch.float64 if f64 else torch.float32
+    s, pos, _, q = _system(n)
+    b = native.Batch(native.make_params(precision=int(f64)), [s.N], [s.box])
+    p, qq = pos.to(dt), q.to(dt)
+
+    def run(rows):
+        f = torch.zeros((s.N, 4), dtype=dt, device="cuda")
+        if term.startswith("lj"):
+            b.lj(p, rows, 1.0, 0.9, 2.5, f)
+        elif f64:
+            b.compute_f64(p, qq, f, nlist=rows, flags=ESP_SHORT_RANGE)
+        else:
+            b.compute(p, qq, f, nlist=rows, flags=ESP_SHORT_RANGE)
+        return f
+
+    full = _rows(s.N, CAP)
+    b.build_nlist(pos, RLIST, CAP, *full)
+    want_full = run(full)
+    short = _rows(s.N, SHORT)
+    _overflowing(b, pos, short)
+    got = run(short)
+    with pytest.raises(EspError) as ei:
+        b.nlist_check()
+    assert ei.value.code == -5
+    assert int(short[1].max()) > SHORT  # the needed counts stay
+    assert torch.equal(got, run(_cut(short)))
+    # rows that fit are read whole again
+    b.build_nlist(pos, RLIST, CAP, *full)
+    assert torch.equal(run(full), want_full)
+
+
+def test_md_steps_over_overflowed_rows():
+    s, pos, vel, q = _system()
+    b = native.Batch(native.make_params(), [s.N], [s.box])
+
+    def run(rows):
+        x, v = pos.clone(), vel.clone()
+        f = torch.zeros((s.N, 4), device="cuda")
+        e = torch.zeros(1, dtype=torch.float64, device="cuda")
+        b.md_run(x, v, q, f, e, None, rows, 2, 0.002)
+        return x
+
+    full, short = _rows(s.N, CAP), _rows(s.N, SHORT)
+    b.build_nlist(pos, RLIST, CAP, *full)
+    run(full)
+    _overflowing(b, pos, short)
+    got = run(short)
+    with pytest.raises(EspError):
+        b.nlist_check()
+    # two steps: the FP64 mesh sums' order shows through FP32 rounding only
+    assert torch.allclose(got, run(_cut(short)), rtol=0, atol=1e-5)
+
+
+@pytest.mark.parametrize("n", [12, 46])  # both row kernels
+def test_served_request_with_overflowing_rows_fails_alone(n):
+    srv = native.Server(native.make_params(), hbm_budget=2 << 30, max_systems=8, max_particles=131072)
+    s = systems.rocksalt(n, seed=77)
+    p4 = np.zeros((s.N, 4), np.float32)
+    p4[:, :3] = s.pos
+    v4 = np.zeros((s.N, 4), np.float32)
+    v4[:, 3] = 1.0
+    q = s.q.astype(np.float32)
+
+    def submit(cap):
+        f = np.zeros((s.N, 4), np.float32)
+        return srv.submit(p4, q, s.box, 3.0, vel4=v4, nsteps=3, nlist_cap=cap, out_force4=f), f
+
+    out = [submit(cap) for cap in (SHORT, 0, 0)]
+    srv.start()
+    srv.wait_all(120)
+    assert [srv.status(r)["state"] for r, _ in out] == [-5, 2, 2]
+    ref = out[2][1][:, :3].astype(np.float64)
+
+    def rel(f):
+        return np.sqrt(((f[:, :3] - ref) ** 2).sum() / (ref ** 2).sum())
+
+    assert rel(out[1][1]) <= 1e-6
+    # the server goes on serving
+    rid, f = submit(0)
+    srv.wait_all(120)
+    assert srv.status(rid)["state"] == 2
+    assert rel(f) <= 1e-6
+    srv.close()
