@@ -1259,10 +1259,11 @@ int esp_batch::setup_cells(CellGrid& g, double rlist, int cap) {
         g.cap = cap;
         return 0;
     }
-    g.mem.release();
-    g.rlist = -1;
-    g.cap = -1;
-    g.h_cells.assign(nsys, CellDev{});
+    // everything that can be refused is looked at before anything is released
+    for (int s = 0; s < nsys; ++s)
+        for (int d = 0; d < 3; ++d)
+            if (2.0 * rlist > box[3 * s + d]) return fail(ESP_ERR_INVALID, "rlist must not exceed half the box");
+    std::vector<CellDev> cells(nsys);
     std::vector<int> cell_sys;
     int c_off = 0;
     long long nl_off = 0;
@@ -1270,14 +1271,12 @@ int esp_batch::setup_cells(CellGrid& g, double rlist, int cap) {
     for (int s = 0; s < nsys; ++s)
         full += std::max(1.0, std::floor(box[3 * s] / rlist)) * std::max(1.0, std::floor(box[3 * s + 1] / rlist)) *
                 std::max(1.0, std::floor(box[3 * s + 2] / rlist));
-    g.half = nlist_half_cells(totN, full);
+    const bool half = nlist_half_cells(totN, full);
     for (int s = 0; s < nsys; ++s) {
-        CellDev& C = g.h_cells[s];
+        CellDev& C = cells[s];
         int nc[3];
-        for (int d = 0; d < 3; ++d) {
-            if (2.0 * rlist > box[3 * s + d]) return fail(ESP_ERR_INVALID, "rlist must not exceed half the box");
-            nc[d] = std::max(1, (int)std::floor((g.half ? 2.0 : 1.0) * box[3 * s + d] / rlist));
-        }
+        for (int d = 0; d < 3; ++d)
+            nc[d] = std::max(1, (int)std::floor((half ? 2.0 : 1.0) * box[3 * s + d] / rlist));
         // sparse systems take larger cells: at most 16 per particle
         const double room = (16.0 * N[s] + 4096.0) / ((double)nc[0] * nc[1] * nc[2]);
         if (room < 1.0)
@@ -1296,6 +1295,11 @@ int esp_batch::setup_cells(CellGrid& g, double rlist, int cap) {
         c_off += (int)ncell;
         nl_off += (long long)N[s] * cap;
     }
+    g.mem.release();
+    g.rlist = -1;
+    g.cap = -1;
+    g.h_cells = std::move(cells);
+    g.half = half;
     g.n_cells = c_off;
     int rc = 0;
     if ((rc = g.mem.get(g.d_cells, nsys)) || (rc = g.mem.get(g.d_cell_sys, g.n_cells)) ||
@@ -1414,6 +1418,10 @@ int esp_batch::build_pairlist(cudaStream_t st, const float* pos4, double rlist, 
     if (!pos4) return fail(ESP_ERR_INVALID, "null position pointer");
     if (f64) return fail(ESP_ERR_UNSUPPORTED, "the library's pair list serves the FP32 path");
     if ((double)totN * cap >= 4294967296.0) return fail(ESP_ERR_UNSUPPORTED, "pair list of 2^32 entries or more");
+    // a rebuild that fails from here on leaves no list: the arrays of the last
+    // one may be gone, and its rows are not those that were asked for
+    pl_ready = pl_pending = pl_overflow = false;
+    pl = PairList{};
     if (rlist != cg_pl.rlist) drop_graphs();  // captured steps hold the previous cell grid's slot maps
     int rc = list_states();
     if (!rc) rc = setup_cells(cg_pl, rlist, cap);

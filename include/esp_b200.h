@@ -290,7 +290,8 @@ int esp_batch_nlist_check(esp_batch* b, int* needed_cap);
  * (totN * cap below 2^32). Does not synchronise: overflow is reported as for
  * esp_batch_build_nlist, by esp_batch_pairlist_check and by the first
  * esp_batch_compute / esp_batch_md_run over the list that finds the build
- * finished. */
+ * finished. A build that is refused for its rlist or fails leaves no list:
+ * evaluations without rows return ESP_ERR_INVALID until the next one. */
 int esp_batch_build_pairlist(esp_batch* b, void* stream, const float* pos4, double rlist, int cap);
 int esp_batch_pairlist_check(esp_batch* b, int* needed_cap);
 

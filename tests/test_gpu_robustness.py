@@ -3,7 +3,9 @@
 * rows longer than their capacity, in an evaluation that is queued before the
   host can know of the overflow: every term reads the entries that the rows
   hold, no more (the same bits as over a list cut to the capacity by the caller);
-* a served request whose rows overflow fails alone.
+* a served request whose rows overflow fails alone;
+* a refused pair-list rebuild leaves no list, and the next one works; refused
+  HOOMD-layout rebuilds leave the caller's rows usable.
 """
 import numpy as np
 import pytest
@@ -133,3 +135,43 @@ def test_served_request_with_overflowing_rows_fails_alone(n):
     assert srv.status(rid)["state"] == 2
     assert rel(f) <= 1e-6
     srv.close()
+
+
+def test_refused_pairlist_rebuild_leaves_no_list():
+    s, pos, vel, q = _system()
+    b = native.Batch(native.make_params(), [s.N], [s.box])
+    f = [torch.zeros((s.N, 4), device="cuda") for _ in range(2)]
+    e = torch.zeros(1, dtype=torch.float64, device="cuda")
+    b.build_pairlist(pos, RLIST, CAP)
+    b.compute(pos, q, f[0], flags=ESP_SHORT_RANGE)
+    b.md_run(pos.clone(), vel.clone(), q, f[1], e, None, None, 2, 0.002)  # captured over that list
+    with pytest.raises(EspError) as ei:
+        b.build_pairlist(pos, 0.51 * min(s.box), CAP)
+    assert ei.value.code == -1
+    for call in (lambda: b.compute(pos, q, f[1], flags=ESP_SHORT_RANGE),
+                 lambda: b.md_run(pos.clone(), vel.clone(), q, f[1], e, None, None, 2, 0.002),
+                 b.pairlist_check):
+        with pytest.raises(EspError) as ei:
+            call()
+        assert ei.value.code == -1
+    b.build_pairlist(pos, RLIST, CAP)
+    b.pairlist_check()
+    b.compute(pos, q, f[1], flags=ESP_SHORT_RANGE)
+    assert torch.equal(f[0], f[1])
+
+
+def test_refused_row_rebuild_keeps_the_rows():
+    s, pos, _, q = _system()
+    b = native.Batch(native.make_params(), [s.N], [s.box])
+    rows = _rows(s.N, CAP)
+    f = [torch.zeros((s.N, 4), device="cuda") for _ in range(3)]
+    b.build_nlist(pos, RLIST, CAP, *rows)
+    b.compute(pos, q, f[0], nlist=rows, flags=ESP_SHORT_RANGE)
+    with pytest.raises(EspError) as ei:
+        b.build_nlist(pos, 0.51 * min(s.box), CAP, *rows)
+    assert ei.value.code == -1
+    b.compute(pos, q, f[1], nlist=rows, flags=ESP_SHORT_RANGE)
+    b.build_nlist(pos, RLIST, CAP, *rows)
+    b.nlist_check()
+    b.compute(pos, q, f[2], nlist=rows, flags=ESP_SHORT_RANGE)
+    assert torch.equal(f[0], f[1]) and torch.equal(f[0], f[2])
