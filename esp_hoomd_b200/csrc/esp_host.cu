@@ -448,6 +448,10 @@ struct esp_batch {
                 bool want_energy = true, float* virial_pp = nullptr, int vpp_pitch = 0,
                 double* external = nullptr);
     int spread_only(cudaStream_t st, const float* pos4, const float* q, double* rho_out);
+    // see EvalGuard; state_dirty: a clear after a failed evaluation failed as well
+    bool state_dirty = false;
+    int clear_state(cudaStream_t st, cudaStream_t side);
+    void after_failure(cudaStream_t st, cudaStream_t side);
     int build_nlist(cudaStream_t st, const float* pos4, double rlist, int cap, unsigned* head, unsigned* nn,
                     unsigned* nl);
     int info(int s, esp_info* out) const;
@@ -739,6 +743,7 @@ int esp_batch::plan(const esp_params& p, int ns, const int* N_, const double* bo
     ESPB_CK(cudaMemset(d_tcount, 0, n_tiles * sizeof(uint32_t)));
     ESPB_CK(cudaMemset(d_acc, 0, (size_t)ns * ACC_STRIDE * sizeof(double)));
     ESPB_CK(cudaMemset(d_rho, 0, (size_t)std::max<long long>(m_off, 1) * sizeof(double)));
+    state_dirty = false;
     drop_graphs();
     {
         // kernel attributes are set here, outside any stream capture
@@ -847,17 +852,46 @@ int esp_batch::plan64(const std::vector<float2>& tw, long long g_total) {
     return 0;
 }
 
-// The accumulators are zero between evaluations: the totals' kernel clears what
-// it has read, and an evaluation that ends before it clears them itself.
-struct AccGuard {
-    double* acc;
-    size_t bytes;
+// The accumulators, the tile counts and the charge mesh are zero between
+// evaluations: the kernel that reads each of them last clears it. An evaluation
+// that ends early leaves them to clear_state, after the kernels it has launched
+// on its second stream (`side`, once that one waits for the first).
+struct EvalGuard {
+    esp_batch& b;
     cudaStream_t st;
-    bool finalized = false;
-    ~AccGuard() {
-        if (!finalized) cudaMemsetAsync(acc, 0, bytes, st);
+    cudaStream_t side = nullptr;
+    bool done = false;
+    ~EvalGuard() {
+        if (!done) b.after_failure(st, side);
     }
 };
+
+int esp_batch::clear_state(cudaStream_t st, cudaStream_t side) {
+    state_dirty = true;
+    if (side) {
+        ESPB_CK(cudaEventRecord(ev_join, side));
+        ESPB_CK(cudaStreamWaitEvent(st, ev_join, 0));
+    }
+    long long M = 0;
+    for (const SysDev& S : sd) M += (long long)S.nx * S.ny * S.nz;
+    ESPB_CK(cudaMemsetAsync(d_acc, 0, (size_t)nsys * ACC_STRIDE * sizeof(double), st));
+    ESPB_CK(cudaMemsetAsync(d_tcount, 0, (size_t)n_tiles * sizeof(uint32_t), st));
+    ESPB_CK(cudaMemsetAsync(d_rho, 0, (size_t)M * sizeof(double), st));
+    state_dirty = false;
+    return 0;
+}
+
+void esp_batch::after_failure(cudaStream_t st, cudaStream_t side) {
+    // of a failed capture nothing has run
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(st, &cs) == cudaSuccess && cs != cudaStreamCaptureStatusNone) return;
+    cudaGetLastError();
+    const std::string why = g_err;
+    if (clear_state(st, side)) {  // the next evaluation tries again
+        cudaGetLastError();
+        g_err = why;
+    }
+}
 
 int esp_batch::compute_f64(cudaStream_t st, const double* pos4, const double* q, const unsigned* head,
                            const unsigned* nn, const unsigned* nl, double* force4, double* energy, double* virial,
@@ -906,7 +940,11 @@ int esp_batch::compute_f64(cudaStream_t st, const double* pos4, const double* q,
     b.n_xl = n_xl;
     b.n_yl = n_yl;
     b.n_zl = n_zl;
-    AccGuard acc_guard{d_acc, (size_t)nsys * ACC_STRIDE * sizeof(double), st};
+    if (state_dirty) {
+        const int rc = clear_state(st, st_mesh64);
+        if (rc) return rc;
+    }
+    EvalGuard guard{*this, st};
     ESPB_CK(launch64_bin(b, st));
     if (lr && sr) {
         // the pair term, bound by the FP64 pipe, beside the mesh kernels, bound
@@ -916,12 +954,13 @@ int esp_batch::compute_f64(cudaStream_t st, const double* pos4, const double* q,
         // other 593, the pair term's CTAs first 589)
         ESPB_CK(cudaEventRecord(ev_fork, st));
         ESPB_CK(cudaStreamWaitEvent(st_mesh64, ev_fork, 0));
+        guard.side = st_mesh64;
         ESPB_CK(launch64_mesh(b, st_mesh64));
         ESPB_CK(cudaEventRecord(ev_join, st_mesh64));
         ESPB_CK(launch64_pair(b, d_fsr64, st));
         ESPB_CK(cudaStreamWaitEvent(st, ev_join, 0));
         ESPB_CK(launch_add_finalize(a, d_fsr64, b.force, st));
-        acc_guard.finalized = true;
+        guard.done = true;
         return 0;
     }
     if (lr) {
@@ -932,7 +971,7 @@ int esp_batch::compute_f64(cudaStream_t st, const double* pos4, const double* q,
         ESPB_CK(cudaMemsetAsync(d_tcount, 0, (size_t)n_tiles * sizeof(uint32_t), st));
     }
     ESPB_CK(launch_finalize(a, st));
-    acc_guard.finalized = true;
+    guard.done = true;
     return 0;
 }
 
@@ -1041,7 +1080,11 @@ int esp_batch::compute(cudaStream_t st, const float* pos4, const float* q, const
     if (sr && a.row_limit) a.nn_limited = d_nn_limited;
     a.accumulate = lr ? 1 : 0;
     a.add_bg = lr ? 1 : 0;
-    AccGuard acc_guard{d_acc, (size_t)nsys * ACC_STRIDE * sizeof(double), st};
+    if (state_dirty) {
+        const int rc = clear_state(st, st2);
+        if (rc) return rc;
+    }
+    EvalGuard guard{*this, st};
     timer.begin(ESP_STAGE_BIN, st);
     ESPB_CK(launch_bin(a, st));
     timer.end(st);
@@ -1054,6 +1097,7 @@ int esp_batch::compute(cudaStream_t st, const float* pos4, const float* q, const
     if (fork) {
         ESPB_CK(cudaEventRecord(ev_fork, st));
         ESPB_CK(cudaStreamWaitEvent(st2, ev_fork, 0));
+        guard.side = st2;
         LaunchArgs ap = a;
         ap.force = d_fsr;
         ap.accumulate = 0;
@@ -1101,7 +1145,7 @@ int esp_batch::compute(cudaStream_t st, const float* pos4, const float* q, const
         }
         ESPB_CK(launch_finalize(a, st));
     }
-    acc_guard.finalized = true;
+    guard.done = true;
     return 0;
 }
 
@@ -1239,7 +1283,11 @@ int esp_batch::spread_only(cudaStream_t st, const float* pos4, const float* q, d
     long long M = 0;
     for (const SysDev& S : sd) M += (long long)S.nx * S.ny * S.nz;
     ESPB_CK(cudaMemsetAsync(rho_out, 0, (size_t)M * sizeof(double), st));
-    AccGuard acc_guard{d_acc, (size_t)nsys * ACC_STRIDE * sizeof(double), st};  // no totals: cleared on return
+    if (state_dirty) {
+        const int rc = clear_state(st, nullptr);
+        if (rc) return rc;
+    }
+    EvalGuard guard{*this, st};
     LaunchArgs a = args();
     a.pos_in = reinterpret_cast<const float4*>(pos4);
     a.q_in = q;
@@ -1247,6 +1295,9 @@ int esp_batch::spread_only(cudaStream_t st, const float* pos4, const float* q, d
     ESPB_CK(launch_bin(a, st));
     ESPB_CK(launch_sort(a, st));
     ESPB_CK(launch_spread(a, st));
+    // no totals here that would clear what the bin stage summed
+    ESPB_CK(cudaMemsetAsync(d_acc, 0, (size_t)nsys * ACC_STRIDE * sizeof(double), st));
+    guard.done = true;
     return 0;
 }
 

@@ -1,0 +1,94 @@
+"""An evaluation that ends early, because one of its launches failed, does not
+reach into the next one (CPU: the library over a fake CUDA runtime that logs the
+stream operations and fails one of them).
+
+The accumulators, the tile counts and the charge mesh are zero between
+evaluations. After a failed launch the caller's stream first waits for the
+kernels already launched on the second stream, then clears the three; the next
+evaluation is launched as if nothing had happened. When the clear fails too, the
+next evaluation starts with it.
+"""
+import ctypes
+import os
+import subprocess
+import sys
+
+import pytest
+
+HERE = os.path.dirname(os.path.abspath(__file__))
+ROOT = os.path.dirname(HERE)
+CUDA = "/usr/local/cuda/include"
+
+MESH, N = 16, 64
+
+
+def _child():
+    from esp_hoomd_b200 import _lib
+    lib = _lib.get_lib()
+    fake = ctypes.CDLL(None)
+    fake.fake_log.restype = ctypes.c_char_p
+    fake.fake_reset.argtypes = [ctypes.c_long, ctypes.c_long]
+    buf = [(ctypes.c_double * (8 * N)).from_buffer(bytearray(64 * N)) for _ in range(8)]
+    pos, q, head, nn, nl, force = (ctypes.addressof(b) for b in buf[:6])
+
+    def log():
+        return [tuple(line.split(" ", 2)) for line in fake.fake_log().decode().splitlines()]
+
+    for precision in (0, 1):
+        p = _lib.EspParams()
+        assert lib.esp_params_default(ctypes.byref(p)) == 0
+        p.nx = p.ny = p.nz = MESH
+        p.precision = precision
+        h = ctypes.c_void_p()
+        assert lib.esp_create(ctypes.byref(p), 10.0, 10.0, 10.0, N, ctypes.byref(h)) == 0, lib.esp_last_error()
+        compute = lib.esp_compute_f64 if precision else lib.esp_compute
+
+        def run(flags, fail_launch=-1, fail_memset=-1):
+            fake.fake_reset(fail_launch, fail_memset)
+            rc = compute(h, None, pos, q, N, head, nn, nl, force, None, None, flags)
+            return rc, log()
+
+        clears = [str(24 * 8), str(((MESH + 8) // 9) ** 3 * 4), str(MESH ** 3 * 8)]  # 9: the tile edge of support 8
+        for flags in (_lib.ESP_ALL, _lib.ESP_LONG_RANGE, _lib.ESP_SHORT_RANGE):
+            rc, good = run(flags)
+            assert rc == 0
+            n = sum(o[0] == "launch" for o in good)
+            forks = {o[1] for o in good if o[0] == "wait"} - {"0"}
+            assert n >= 3 and len(forks) == (flags == _lib.ESP_ALL)
+            for k in range(n):
+                rc, ops = run(flags, k)
+                assert rc == -2 and b"fake error" in lib.esp_last_error()
+                at = [o[0] for o in ops].index("fail")
+                forked = [o[1] for o in ops if o[0] == "wait" and o[1] != "0"]
+                tail = ops[-3 - 2 * len(forked):]
+                assert at < len(ops) - len(tail) and not any(o[0] == "launch" for o in tail)
+                if forked:  # the caller's stream waits for what the second stream holds
+                    assert tail[0][:2] == ("record", forked[0]) and tail[1] == ("wait", "0", tail[0][2])
+                assert [o for o in tail if o[0] == "memset"] == [("memset", "0", c) for c in clears]
+                assert run(flags) == (0, good)
+            # the clear fails as well: the next evaluation starts with it
+            memsets = sum(o[0] == "memset" for o in run(flags, 1)[1])
+            rc, _ = run(flags, 1, memsets - 1)
+            assert rc == -2 and b"fake error" in lib.esp_last_error()
+            rc, ops = run(flags)
+            assert rc == 0 and ops[-len(good):] == good
+            assert [o for o in ops[:-len(good)] if o[0] == "memset"] == [("memset", "0", c) for c in clears]
+            assert run(flags) == (0, good)
+        lib.esp_destroy(h)
+    print("ok")
+
+
+def test_failed_launch_leaves_clear_state(tmp_path):
+    if not os.path.exists(os.path.join(CUDA, "cuda_runtime.h")):
+        pytest.skip("needs the CUDA headers")
+    so = str(tmp_path / "libfake_cudart.so")
+    subprocess.run(["g++", "-O1", "-std=c++17", "-shared", "-fPIC", "-I" + CUDA,
+                    os.path.join(HERE, "fake_cudart.cpp"), "-o", so], check=True)
+    env = dict(os.environ, LD_PRELOAD=so, PYTHONPATH=ROOT)
+    r = subprocess.run([sys.executable, os.path.abspath(__file__)], env=env, cwd=ROOT, capture_output=True, text=True,
+                       timeout=300)
+    assert r.returncode == 0 and r.stdout.strip() == "ok", r.stdout + r.stderr
+
+
+if __name__ == "__main__":
+    _child()
