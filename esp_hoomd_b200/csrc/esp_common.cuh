@@ -214,6 +214,15 @@ __device__ __forceinline__ void bucket_starts(uint32_t* cnt, uint32_t* beg) {
     cnt[2 * l + 1] = x - b;
 }
 
+// First mesh point of the stencil of a particle at grid coordinate g, from
+// u = g - P/2: floor(u) + 1, in [-P + 1, n + 1]. g lies in [0, n) unless the
+// position is not finite or too large to be wrapped; then some point of that
+// range is returned, so that every index stays inside the mesh, and the stencil
+// coordinate carries the non-finite value on into the forces.
+__device__ __forceinline__ int stencil_origin(double u, int P, int n) {
+    return min(max(__double2int_rd(u), -P), n) + 1;
+}
+
 // Entries of a neighbour row that may be read: n, or the row capacity when
 // *limit is set (the library built the rows and one of them overflowed, so that
 // n may be a count its row does not hold).

@@ -62,7 +62,7 @@ __global__ void k64_bin(const int2* __restrict__ chunks, const SysDev* __restric
         for (int d = 0; d < 3; ++d) {
             double g = x[d] * gd[d];
             if (g >= n[d]) g -= n[d];
-            const int i0 = (int)floor(g - hp) + 1;
+            const int i0 = stencil_origin(g - hp, P, n[d]);
             tt[d] = (double)i0 + hp - g;
             i0m[d] = i0 < 0 ? i0 + n[d] : (i0 >= n[d] ? i0 - n[d] : i0);
         }

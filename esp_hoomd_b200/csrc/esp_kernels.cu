@@ -64,7 +64,7 @@ __global__ void k_bin(const int2* __restrict__ chunks, const SysDev* __restrict_
 #pragma unroll
         for (int d = 0; d < 3; ++d) {
             if (g[d] >= n[d]) g[d] -= n[d];
-            const int i0 = (int)floor(g[d] - hp) + 1;
+            const int i0 = stencil_origin(g[d] - hp, P, n[d]);
             tt[d] = (float)((double)i0 + hp - g[d]);
             i0m[d] = i0 < 0 ? i0 + n[d] : (i0 >= n[d] ? i0 - n[d] : i0);
         }

@@ -5,7 +5,10 @@
   hold, no more (the same bits as over a list cut to the capacity by the caller);
 * a served request whose rows overflow fails alone;
 * a refused pair-list rebuild leaves no list, and the next one works; refused
-  HOOMD-layout rebuilds leave the caller's rows usable.
+  HOOMD-layout rebuilds leave the caller's rows usable;
+* positions that are not finite, or too large to be wrapped, give non-finite
+  forces in their system, and leave the batch's other systems, the next
+  evaluation and other served requests as they are.
 """
 import numpy as np
 import pytest
@@ -175,3 +178,85 @@ def test_refused_row_rebuild_keeps_the_rows():
     b.nlist_check()
     b.compute(pos, q, f[2], nlist=rows, flags=ESP_SHORT_RANGE)
     assert torch.equal(f[0], f[1]) and torch.equal(f[0], f[2])
+
+
+BAD = [float("nan"), float("inf"), -float("inf"), 1e30, -3e38, 2e10]
+
+
+# one-kernel (n = 8) and three-kernel sorts; not FP64 at support 11 and n = 46, where repeated
+# evaluations differ by 2e-12 themselves
+@pytest.mark.parametrize("order,n,f64", [(o, n, f) for o in (4, 6, 8, 11) for n in (8, 46) for f in (False, True)
+                                         if (o, n, f) != (11, 46, True)])
+def test_positions_without_a_place_stay_in_their_system(order, n, f64):
+    dt = torch.float64 if f64 else torch.float32
+    s = systems.rocksalt(n, seed=5)
+    b = native.Batch(native.make_params(order=order, precision=int(f64), mesh=(48, 48, 48)), [s.N] * 2, [s.box] * 2)
+    pos = torch.zeros((2 * s.N, 4), dtype=dt, device="cuda")
+    pos[:, :3] = torch.as_tensor(np.tile(s.pos, (2, 1)), device="cuda")
+    q = torch.as_tensor(np.tile(s.q, 2), dtype=dt, device="cuda")
+    rows = _rows(2 * s.N, CAP)
+    b.build_nlist(pos.float(), RLIST, CAP, *rows)
+
+    def run(p):
+        f = torch.zeros((2 * s.N, 4), dtype=dt, device="cuda")
+        e = torch.zeros(2, dtype=torch.float64, device="cuda")
+        w = torch.zeros((2, 6), dtype=torch.float64, device="cuda")
+        (b.compute_f64 if f64 else b.compute)(p, q, f, e, w, nlist=rows)
+        return f, e, w
+
+    f0, e0, w0 = run(pos)
+    bad = pos.clone()
+    for k, v in enumerate(BAD):
+        bad[s.N + 7 * k, k % 3] = v
+    f1, e1, w1 = run(bad)
+    f2, e2, w2 = run(pos)
+    assert not torch.isfinite(f1[s.N:, :3]).all()
+    tol = 1e-12 if f64 else 1e-6  # the order of the FP64 mesh sums, seen through one FP32 rounding per stage
+    rms = float(f0[:, :3].double().pow(2).mean().sqrt())
+    scale = float(f0[:, 3].double().abs().sum())
+    assert float((f1[:s.N, :3] - f0[:s.N, :3]).double().pow(2).mean().sqrt()) <= tol * rms
+    assert abs(float(e1[0] - e0[0])) <= tol * scale
+    assert float((f2[:, :3] - f0[:, :3]).double().pow(2).mean().sqrt()) <= tol * rms
+    assert float((e2 - e0).abs().max()) <= tol * scale
+    assert float((w2 - w0).abs().max()) <= tol * scale
+
+
+def test_md_steps_from_positions_without_a_place():
+    s, pos, vel, q = _system(8)
+    b = native.Batch(native.make_params(), [s.N], [s.box])
+    f = torch.zeros((s.N, 4), device="cuda")
+    e = torch.zeros(1, dtype=torch.float64, device="cuda")
+    x, v = pos.clone(), vel.clone()
+    for k, u in enumerate(BAD):
+        x[5 * k, k % 3] = u
+    b.build_pairlist(x, RLIST, CAP)
+    b.compute(x, q, f, e)
+    b.md_run(x, v, q, f, e, None, None, 3, 0.002)
+    assert not torch.isfinite(f).all()
+    b.build_pairlist(pos, RLIST, CAP)
+    b.compute(pos, q, f, e)
+    assert torch.isfinite(f).all() and torch.isfinite(e).all()
+
+
+def test_served_request_without_a_place_stays_alone():
+    s = systems.rocksalt(12, seed=78)
+    p4 = np.zeros((s.N, 4), np.float32)
+    p4[:, :3] = s.pos
+    v4 = np.zeros((s.N, 4), np.float32)
+    v4[:, 3] = 1.0
+    bad = p4.copy()
+    for k, u in enumerate(BAD):
+        bad[5 * k, k % 3] = u
+    q = s.q.astype(np.float32)
+    srv = native.Server(native.make_params(), hbm_budget=2 << 30, max_systems=8, max_particles=65536)
+    out = []
+    for p in (p4, bad, p4):
+        f = np.zeros((s.N, 4), np.float32)
+        out.append((srv.submit(p, q, s.box, 3.0, vel4=v4, nsteps=3, out_force4=f), f))
+    srv.start()
+    srv.wait_all(120)
+    assert [srv.status(r)["state"] for r, _ in out] == [2, 2, 2]
+    assert not np.isfinite(out[1][1]).all()
+    a, c = out[0][1][:, :3].astype(np.float64), out[2][1][:, :3].astype(np.float64)
+    assert np.sqrt(((a - c) ** 2).sum() / (c ** 2).sum()) <= 1e-6
+    srv.close()
