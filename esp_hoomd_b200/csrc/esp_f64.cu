@@ -94,9 +94,10 @@ __global__ void k64_bin(const int2* __restrict__ chunks, const SysDev* __restric
 // FP64 records. Indices are bucketed by their range before they are ranked:
 // ranking against the whole tile is n^2, and beside the pair term a coarse
 // mesh's full tiles waited for it (60,000 charges in 64 tiles of 940, support
-// 6: evaluation 637 -> 306 us; 98,304 in 125 tiles 641 -> 407).
+// 6: evaluation 637 -> 306 us; 98,304 in 125 tiles 641 -> 407). Tiles above the
+// shared-memory capacity go by sort_large_tile.
 __global__ void __launch_bounds__(256)
-    k64_tile_sort(const uint32_t* __restrict__ start, const uint32_t* __restrict__ perm_u,
+    k64_tile_sort(const uint32_t* __restrict__ start, uint32_t* __restrict__ perm_u,
                   uint32_t* __restrict__ perm, const double4* __restrict__ trec, const uint32_t* __restrict__ rel,
                   double4* __restrict__ srec, uint32_t* __restrict__ srel) {
     after_previous();
@@ -106,14 +107,7 @@ __global__ void __launch_bounds__(256)
     const uint32_t n = start[blockIdx.x + 1] - s0;
     if (n == 0) return;
     if (n > (uint32_t)SORT_CAP) {
-        for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) {
-            const uint32_t v = perm_u[s0 + i];
-            uint32_t r = 0;
-            for (uint32_t j = 0; j < n; ++j) r += (perm_u[s0 + j] < v) ? 1u : 0u;
-            perm[s0 + r] = v;
-            srec[s0 + r] = trec[v];
-            srel[s0 + r] = rel[v];
-        }
+        sort_large_tile(s0, n, perm_u, perm, trec, rel, srec, srel, sm, sm + LARGE_BUCKETS, &lo, &hi);
         return;
     }
     if (threadIdx.x < SORT_BUCKETS) cnt[threadIdx.x] = 0u;

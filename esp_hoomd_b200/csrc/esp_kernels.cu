@@ -396,23 +396,24 @@ __global__ void __launch_bounds__(DIRECT_THREADS)
     }
     if (n == 0) return;
     if (n > (uint32_t)SORT_CAP) {
-        // a tile above the shared-memory capacity ranks from memory
+        // a tile above the shared-memory capacity: collected in memory first
         __syncthreads();
         if (threadIdx.x == 0) n_in = 0u;
         __syncthreads();
         for (int i = threadIdx.x; i < N; i += DIRECT_THREADS)
             if (key[p_off + i] == t) perm_u[s0 + atomicAdd(&n_in, 1u)] = (uint32_t)(p_off + i);
         __syncthreads();
-        for (uint32_t i = threadIdx.x; i < n; i += DIRECT_THREADS) {
-            const uint32_t v = perm_u[s0 + i], kv = BY_Y ? sort_key(v, rel, p_off) : v;
-            uint32_t r = 0;
-            for (uint32_t j = 0; j < n; ++j) {
-                const uint32_t w = perm_u[s0 + j];
-                r += (BY_Y ? sort_key(w, rel, p_off) : w) < kv ? 1u : 0u;
+        if constexpr (!BY_Y) {
+            sort_large_tile(s0, n, perm_u, perm, trec, rel, srec, srel, sm, sm + LARGE_BUCKETS, &lo, &hi);
+        } else {
+            for (uint32_t i = threadIdx.x; i < n; i += DIRECT_THREADS) {
+                const uint32_t v = perm_u[s0 + i], kv = sort_key(v, rel, p_off);
+                uint32_t r = 0;
+                for (uint32_t j = 0; j < n; ++j) r += sort_key(perm_u[s0 + j], rel, p_off) < kv ? 1u : 0u;
+                perm[s0 + r] = v;
+                srec[s0 + r] = trec[v];
+                srel[s0 + r] = rel[v];
             }
-            perm[s0 + r] = v;
-            srec[s0 + r] = trec[v];
-            srel[s0 + r] = rel[v];
         }
         return;
     }
