@@ -469,6 +469,16 @@ int esp_server::admit(Request* q, Staging& sg) {
     const long long Mp = std::max(M, (long long)halo_extent(q->mesh[0], T, P, true) * halo_extent(q->mesh[1], T, P, false) *
                                          halo_extent(q->mesh[2], T, P, false));
     const double rlist = r.rcut + r.skin;
+    // everything that refuses a request comes before its ranges are taken
+    for (int d = 0; d < 3; ++d)
+        if (2.0 * rlist > L[d]) return fail(ESP_ERR_INVALID, "rcut + skin must not exceed half the box");
+    q->geo = -1;  // rigid water: geometry index, the next one for a geometry not seen so far
+    if (r.rigid_doh > 0) {
+        for (size_t g = 0; g < geos.size(); ++g)
+            if (geos[g].x == r.rigid_doh && geos[g].y == r.rigid_dhh) q->geo = (int)g;
+        if (q->geo < 0) q->geo = (int)geos.size();
+        if (q->geo >= MAX_GEOS) return fail(ESP_ERR_UNSUPPORTED, "more than 16 rigid-water geometries");
+    }
     int cap = r.nlist_cap;
     if (cap <= 0) {
         const double dens = r.N / (r.Lx * r.Ly * r.Lz);
@@ -575,17 +585,10 @@ int esp_server::admit(Request* q, Staging& sg) {
     S.radz = radix_plan(S.nz);
     int rc = upload(sg, d_sys + q->slot, &S, sizeof(SysDev));
     if (rc) return rc;
-    // rigid water: geometry index and the atoms the plain integrator skips
-    q->geo = -1;
-    if (r.rigid_doh > 0) {
-        for (size_t g = 0; g < geos.size(); ++g)
-            if (geos[g].x == r.rigid_doh && geos[g].y == r.rigid_dhh) q->geo = (int)g;
-        if (q->geo < 0) {
-            if ((int)geos.size() >= MAX_GEOS) return fail(ESP_ERR_UNSUPPORTED, "more than 16 rigid-water geometries");
-            q->geo = (int)geos.size();
-            geos.push_back(make_double2(r.rigid_doh, r.rigid_dhh));
-            if ((rc = upload(sg, d_geo + q->geo, &geos.back(), sizeof(double2)))) return rc;
-        }
+    // rigid water: a new geometry, and the atoms the plain integrator skips
+    if (q->geo == (int)geos.size()) {
+        geos.push_back(make_double2(r.rigid_doh, r.rigid_dhh));
+        if ((rc = upload(sg, d_geo + q->geo, &geos.back(), sizeof(double2)))) return rc;
     }
     const int2 skip = make_int2(0, q->geo >= 0 ? r.N : 0);
     if ((rc = upload(sg, d_rskip + q->slot, &skip, sizeof(int2)))) return rc;
@@ -606,10 +609,7 @@ int esp_server::admit(Request* q, Staging& sg) {
     CellDev C{};
     int nc[3];
     double full = 1;
-    for (int d = 0; d < 3; ++d) {
-        if (2.0 * rlist > L[d]) return fail(ESP_ERR_INVALID, "rcut + skin must not exceed half the box");
-        full *= std::max(1.0, std::floor(L[d] / rlist));
-    }
+    for (int d = 0; d < 3; ++d) full *= std::max(1.0, std::floor(L[d] / rlist));
     const bool half = nlist_half_cells(r.N, full);
     for (int d = 0; d < 3; ++d)
         nc[d] = std::min(MAX_CELLS_AXIS, std::max(1, (int)std::floor((half ? 2.0 : 1.0) * L[d] / rlist)));

@@ -4,6 +4,7 @@
   host can know of the overflow: every term reads the entries that the rows
   hold, no more (the same bits as over a list cut to the capacity by the caller);
 * a served request whose rows overflow fails alone;
+* refused requests give back what they had taken: the server goes on admitting;
 * a refused pair-list rebuild leaves no list, and the next one works; refused
   HOOMD-layout rebuilds leave the caller's rows usable;
 * positions that are not finite, or too large to be wrapped, give non-finite
@@ -259,4 +260,20 @@ def test_served_request_without_a_place_stays_alone():
     assert not np.isfinite(out[1][1]).all()
     a, c = out[0][1][:, :3].astype(np.float64), out[2][1][:, :3].astype(np.float64)
     assert np.sqrt(((a - c) ** 2).sum() / (c ** 2).sum()) <= 1e-6
+    srv.close()
+
+
+def test_refused_requests_leave_room():
+    s = systems.rocksalt(8, seed=79)
+    p4 = np.zeros((s.N, 4), np.float32)
+    p4[:, :3] = s.pos
+    q = s.q.astype(np.float32)
+    f = np.zeros((s.N, 4), np.float32)
+    srv = native.Server(native.make_params(), hbm_budget=1 << 30, max_systems=2, max_particles=65536)
+    bad = [srv.submit(p4, q, s.box, 3.0, nsteps=0, skin=1.5) for _ in range(5)]  # rcut + skin above half the box
+    good = srv.submit(p4, q, s.box, 3.0, nsteps=0, out_force4=f)
+    srv.start()
+    srv.wait_all(60)
+    assert [srv.status(r)["state"] for r in bad] == [-1] * 5
+    assert srv.status(good)["state"] == 2 and np.isfinite(f).all() and np.abs(f).max() > 0
     srv.close()
