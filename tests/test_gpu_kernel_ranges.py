@@ -9,13 +9,16 @@ where the rule switches, against the oracle.
 * neighbour rows (HOOMD layout and pair list): cells of half the list radius
   (few cells, or full ones) with 4 and >= 5 cells per axis and both at once and
   with more than 8 and more than 32 particles in a cell; cells of the list
-  radius, sparse and more than 16,384 of them (scanned by several CTAs); capacities that are no multiple of 4, and more
-  excluded partners than the kernel keeps in shared memory: the rows are the
-  oracle's sets.
+  radius, sparse and 27,000 and 125,000 of them (scanned by 7 and 31 CTAs);
+  capacities that are no multiple of 4, and more excluded partners than the
+  kernel keeps in shared memory: the rows are the oracle's sets.
 * tile shares: few tiles, their particles shared out over several CTAs, with
   full, nearly empty and empty tiles at once, supports 5..8 (the rotated walk
-  of the interpolation) and 4 and 10; long-range forces and energy against the
-  oracle within the parity tests' FP32 tolerances (5e-6, 2e-6).
+  of the interpolation) and 4 and 10; long-range forces against the oracle
+  within the parity tests' FP32 tolerance (5e-6), and per-particle and total
+  energies within what the potential's tolerance (5e-6 of the largest mesh
+  value) and 1e-6 for the FP32 stencil sum leave of them: 0.5 |q| 6e-6
+  max|phi| times the sum of the particle's weights.
 * FP64 pair term: a warp per particle up to 148 chunks of 32 particles, 8 lanes
   above, with and without the virial, on the last size of the one and the first
   of the other; against the oracle within the FP64 tests' tolerances (forces
@@ -26,9 +29,10 @@ where the rule switches, against the oracle.
   context gives for each (FP32 1e-6 of the RMS force and of the energies'
   magnitudes, the order of the FP64 mesh sums seen through one FP32 rounding
   per stage; FP64 1e-12).
-* one-kernel sort (small systems): tiles above the shared-memory
-  capacity, both sides of its 64 chunks; long-range forces against the oracle
-  (FP32 5e-6, FP64 1e-8).
+* one-kernel sort (small systems): tiles above the shared-memory capacity, FP32
+  on both sides of its 64 chunks, FP64 (up to 96 chunks; its other side is in
+  test_gpu_tile_sort64) below; long-range forces against the oracle (FP32 5e-6,
+  FP64 1e-8).
 * FFT passes with 256, 512 and 1,024 threads per plane or slab, one and three
   systems: forces, energy and virial against the oracle within the parity
   tests' FP32 tolerances (5e-6, 2e-6, 1e-5).
@@ -142,11 +146,16 @@ def _check_lists(pos, box, rlist, cap, excl=None):
     ((6.2, 20.0, 20.0), 2000, 3.0, 256),  # 4 cells on one axis only
     ((9.0, 9.0, 9.0), 6000, 2.0, 512),    # 8 particles per cell and more
     ((40.0, 40.0, 40.0), 300, 1.5, 16),   # a cell holds a particle rarely: cells enlarged
-    ((60.0, 60.0, 60.0), 20000, 2.0, 64),  # 216,000 cells
+    ((60.0, 60.0, 60.0), 20000, 2.0, 64),  # 27,000 cells of the list radius
 ])
 def test_neighbour_rows(box, n, rlist, cap):
     rng = np.random.default_rng(n)
     _check_lists(rng.uniform(0, 1, (n, 3)) * np.asarray(box), box, rlist, cap)
+
+
+def test_neighbour_rows_of_many_cells():
+    rng = np.random.default_rng(125)
+    _check_lists(rng.uniform(0, 100.0, (20000, 3)), (100.0, 100.0, 100.0), 2.0, 16)
 
 
 def test_neighbour_rows_of_a_dense_cell():
@@ -184,6 +193,35 @@ def test_tile_shares(order, n):
     empty = (np.zeros(n, np.uint32), np.zeros(n, np.uint32), np.zeros(0, np.uint32))
     _, F, _ = R.esp(pos, q, prm, nlist=empty)
     assert R.rel_rms(force.double().cpu().numpy()[:, :3], F) <= 5e-6
+
+
+@pytest.mark.parametrize("order", [4, 5, 6, 7, 8, 10])
+@pytest.mark.parametrize("n", [37, 700])
+def test_tile_shares_energies(order, n):
+    rng = np.random.default_rng(order * 1000 + n)
+    L = 10.0
+    pos = rng.uniform(0, L, (n, 3))
+    pos[: 3 * n // 4] = rng.uniform(0, 3.0, (3 * n // 4, 3))  # most of them in one tile
+    pos = pos.astype(np.float32).astype(np.float64)
+    q = np.where(np.arange(n) % 2 == 0, 1.0, -1.0)
+    ctx = native.Context(native.make_params(order=order, mesh=(24, 24, 24)), (L, L, L), n)
+    inf = ctx.info()
+    p4 = torch.zeros((n, 4), device="cuda")
+    p4[:, :3] = torch.as_tensor(pos, device="cuda")
+    force = torch.zeros((n, 4), device="cuda")
+    energy = torch.zeros(1, dtype=torch.float64, device="cuda")
+    ctx.compute(p4, torch.as_tensor(q, dtype=torch.float32, device="cuda"), force, energy, flags=ESP_LONG_RANGE)
+    prm = tables.ESPParams(mesh=(24, 24, 24), box=(L, L, L), rcut=inf["rcut"],
+                           split=tables.split_cached(inf["c_split"]),
+                           window=tables.window_cached(inf["order"], inf["c_window"], inf["window_degree"]))
+    empty = (np.zeros(n, np.uint32), np.zeros(n, np.uint32), np.zeros(0, np.uint32))
+    E, _, _, parts = R.esp(pos, q, prm, nlist=empty, return_parts=True)
+    e = 0.5 * q * parts["pot"] + R.self_energy(q, prm) / (q * q).sum() * q * q
+    _, t = R.stencil_origin(R.grid_coords(pos, prm.box, prm.mesh), order)
+    weights = np.prod([prm.window.weights(t[:, d]).sum(1) for d in range(3)], 0)
+    tol = 0.5 * np.abs(q) * 6e-6 * np.abs(parts["phi"]).max() * weights
+    assert (np.abs(force.double().cpu().numpy()[:, 3] - e) <= tol).all()
+    assert abs(energy.item() - E) <= tol.sum()
 
 
 @pytest.mark.parametrize("shape", [(16, 16, 18), (18, 17, 16)])  # 4,608 and 4,896 ions
@@ -253,7 +291,8 @@ def test_back_to_back_evaluations(shape, f64):
 @pytest.mark.parametrize("f64", [False, True])
 def test_one_kernel_sort(n, mesh, f64):
     # long-range forces through the sort of a whole evaluation: one kernel up to
-    # 64 chunks (the last size is above; the third has tiles above 2,048 particles)
+    # 64 chunks in FP32 (the last size is above) and 96 in FP64; the third size
+    # has tiles above 2,048 particles
     rng = np.random.default_rng(n)
     L = 10.0
     pos = rng.uniform(0, L, (n, 3)).astype(np.float32).astype(np.float64)
