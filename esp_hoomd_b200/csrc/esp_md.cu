@@ -347,7 +347,8 @@ __global__ void __launch_bounds__(32 * NL_WARPS, EX ? 4 : 7)
         uint32_t mykey = 0, myrow = 0;  // lane k < ng: owner and first entry of the k-th row
 #pragma unroll
         for (int i = 0; i < NL_GROUP; i += 2) {
-            // a missing second particle has a NaN position, which tests false
+            // past the group's last particle: the cell's last one again, which
+            // nl_test leaves out (i >= ng)
             const float4 a = cpos[min(g0 + i, c1 - 1)], b = cpos[min(g0 + i + 1, c1 - 1)];
             g.px[i] = a.x, g.py[i] = a.y, g.pz[i] = a.z;
             g.px[i + 1] = b.x, g.py[i + 1] = b.y, g.pz[i + 1] = b.z;

@@ -14,11 +14,7 @@ namespace espb {
 //   force_divr = qiqj/(4 pi) (1/r^3 + 2 Q'(u)/r_c^3)
 // (the split form of EvaluatorPairPSWF::evalForceAndEnergy).
 // ============================================================================
-// EN: pair energies (per particle and per system); without them the split
-// polynomial Q itself is not needed, only Q', and the kernel (40 registers)
-// keeps 6 CTAs per SM resident so that more position gathers are in flight.
-// Each lane loads its next 16-byte row segment of neighbour indices one
-// iteration ahead of the gathers that use it.
+
 // Rows in 16-byte segments of four entries, one segment per lane and step; the
 // next segment is loaded one step ahead of the gathers that use this one.
 template <int TPP, bool WRAP, typename Eval>
@@ -39,6 +35,9 @@ __device__ __forceinline__ void pair_row(Eval& ev, const uint4* __restrict__ row
     }
 }
 
+// EN: pair energies (per particle and per system); without them the split
+// polynomial Q itself is not needed, only Q', and the kernel (40 registers)
+// keeps 6 CTAs per SM resident so that more position gathers are in flight.
 template <int TPP, int NQ, bool VIR, bool EN>
 __global__ void __launch_bounds__(256, EN ? 5 : 6)
     k_pair(const int2* __restrict__ chunks, const SysDev* __restrict__ sys, const ParamSet* __restrict__ psets,
