@@ -270,9 +270,9 @@ int esp_pswf_eval_pairs(void* stream, int n, const double* rsq, const double* qi
  * be NULL), and by the first esp_batch_compute /
  * esp_batch_md_run over these rows that finds the build finished. Results
  * computed over an overflowed list are invalid; rebuild with a larger cap.
- * Until the overflow is known, this batch's evaluations over the rows read no
- * more than their cap entries; a caller that hands them to another batch or
- * context checks first. */
+ * Until the overflow is known, this batch's evaluations over the rows of its
+ * last build read no more than their cap entries; a caller that hands rows to
+ * another batch or context, or builds others before it uses them, checks first. */
 int esp_batch_build_nlist(esp_batch* b, void* stream, const float* pos4, double rlist, int cap, unsigned* head,
                           unsigned* n_neigh, unsigned* nlist);
 int esp_batch_nlist_check(esp_batch* b, int* needed_cap);
