@@ -223,13 +223,12 @@ __device__ __forceinline__ int stencil_origin(double u, int P, int n) {
     return min(max(__double2int_rd(u), -P), n) + 1;
 }
 
-// Entries of a neighbour row that may be read: n, or the row capacity when
-// *limit is set (the library built the rows and one of them overflowed, so that
+// Entries of a neighbour row that may be read: n, or the row capacity when the
+// limit is set (the library built the rows and one of them overflowed, so that
 // n may be a count its row does not hold).
+__device__ __forceinline__ uint32_t row_entries(uint32_t n, uint32_t limit) { return limit ? min(n, limit) : n; }
 __device__ __forceinline__ uint32_t row_entries(uint32_t n, const uint32_t* __restrict__ limit) {
-    if (!limit) return n;
-    const uint32_t l = *limit;
-    return l ? min(n, l) : n;
+    return limit ? row_entries(n, *limit) : n;
 }
 
 // shift that puts index offsets up to `range` into 2^LOG buckets, in order

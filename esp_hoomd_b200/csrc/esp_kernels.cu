@@ -45,6 +45,11 @@ __global__ void k_bin(const int2* __restrict__ chunks, const SysDev* __restrict_
     if (i < S.p_off + S.N) {
         const float4 p = pos_in[i];
         const float q = q_in[i];
+        uint32_t row = 0u, limit = 0u;  // loaded beside the position
+        if (nn_limited) {
+            row = nn[i];
+            limit = *row_limit;
+        }
         float x = p.x - S.Lx * floorf(p.x * S.inv_Lx);
         float y = p.y - S.Ly * floorf(p.y * S.inv_Ly);
         float z = p.z - S.Lz * floorf(p.z * S.inv_Lz);
@@ -75,7 +80,7 @@ __global__ void k_bin(const int2* __restrict__ chunks, const SysDev* __restrict_
         posq[i] = make_float4(x, y, z, q);
         // the pair list's slot-ordered copy (rows of that list index it)
         if (spos) spos[idx2slot[i]] = make_float4(x, y, z, q);
-        if (nn_limited) nn_limited[i] = row_entries(nn[i], row_limit);
+        if (nn_limited) nn_limited[i] = row_entries(row, limit);
         trec[i] = make_float4(tt[0], tt[1], tt[2], q);
         rel[i] = (uint32_t)(i0m[0] - tx * T) | ((uint32_t)(i0m[1] - ty * T) << 8) |
                  ((uint32_t)(i0m[2] - tz * T) << 16);
