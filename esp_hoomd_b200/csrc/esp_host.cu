@@ -298,7 +298,7 @@ struct esp_batch {
                  *d_slot2idx = nullptr, *d_idx2slot = nullptr, *d_scan = nullptr;
         float4 *d_wpos = nullptr, *d_cpos = nullptr;
     } cg_nl, cg_pl;
-    int setup_cells(CellGrid& g, double rlist, int cap);
+    int setup_cells(CellGrid& g, double rlist, int cap, cudaStream_t st);
     NlistArgs nlist_args(CellGrid& g, const float* pos4, double rlist, int cap) const;
     // overflow states (NLIST_STATE words each) of the last HOOMD-layout and
     // pair-list builds; they outlive cell grids and plans, captured steps
@@ -307,7 +307,7 @@ struct esp_batch {
     int *d_nl_state = nullptr, *d_pl_state = nullptr;
     uint32_t* d_nn_limited = nullptr;
     int nn_limited_n = 0;
-    int list_states();
+    int list_states(cudaStream_t st);
     // how many entries the rows of (head, nl) hold when the library's last
     // build wrote them and overflowed; that build may still be running
     const uint32_t* row_limit(const unsigned* head, const unsigned* nl) const {
@@ -1301,12 +1301,14 @@ int esp_batch::spread_only(cudaStream_t st, const float* pos4, const float* q, d
     return 0;
 }
 
-int esp_batch::setup_cells(CellGrid& g, double rlist, int cap) {
+// On the caller's stream throughout: an earlier build there may still read the
+// cell table, and the builds that follow start from clear counts.
+int esp_batch::setup_cells(CellGrid& g, double rlist, int cap, cudaStream_t st) {
     if (rlist == g.rlist) {
         if (cap == g.cap) return 0;
         // same cells, new row capacity: HOOMD-layout rows of system s start at p_off * cap
         for (int s = 0; s < nsys; ++s) g.h_cells[s].nl_off = (long long)sd[s].p_off * cap;
-        ESPB_CK(cudaMemcpy(g.d_cells, g.h_cells.data(), nsys * sizeof(CellDev), cudaMemcpyHostToDevice));
+        ESPB_CK(cudaMemcpyAsync(g.d_cells, g.h_cells.data(), nsys * sizeof(CellDev), cudaMemcpyHostToDevice, st));
         g.cap = cap;
         return 0;
     }
@@ -1361,15 +1363,15 @@ int esp_batch::setup_cells(CellGrid& g, double rlist, int cap) {
         (rc = g.mem.get(g.d_wpos, totN)) ||
         (rc = g.mem.get(g.d_cpos, totN)))
         return rc;
-    ESPB_CK(cudaMemcpy(g.d_cells, g.h_cells.data(), nsys * sizeof(CellDev), cudaMemcpyHostToDevice));
-    ESPB_CK(cudaMemcpy(g.d_cell_sys, cell_sys.data(), g.n_cells * sizeof(int), cudaMemcpyHostToDevice));
-    ESPB_CK(cudaMemset(g.d_ccount, 0, g.n_cells * sizeof(uint32_t)));
+    ESPB_CK(cudaMemcpyAsync(g.d_cells, g.h_cells.data(), nsys * sizeof(CellDev), cudaMemcpyHostToDevice, st));
+    ESPB_CK(cudaMemcpyAsync(g.d_cell_sys, cell_sys.data(), g.n_cells * sizeof(int), cudaMemcpyHostToDevice, st));
+    ESPB_CK(cudaMemsetAsync(g.d_ccount, 0, g.n_cells * sizeof(uint32_t), st));
     g.rlist = rlist;
     g.cap = cap;
     return 0;
 }
 
-int esp_batch::list_states() {
+int esp_batch::list_states(cudaStream_t st) {
     int rc = 0;
     if (totN > nn_limited_n) {
         if ((rc = ovmem.get(d_nn_limited, totN))) return rc;
@@ -1378,7 +1380,7 @@ int esp_batch::list_states() {
     if (d_nl_state) return 0;
     int* p = nullptr;
     if ((rc = ovmem.get(p, 2 * NLIST_STATE))) return rc;
-    ESPB_CK(cudaMemset(p, 0, 2 * NLIST_STATE * sizeof(int)));
+    ESPB_CK(cudaMemsetAsync(p, 0, 2 * NLIST_STATE * sizeof(int), st));
     d_nl_state = p;
     d_pl_state = p + NLIST_STATE;
     return 0;
@@ -1418,8 +1420,8 @@ int esp_batch::build_nlist(cudaStream_t st, const float* pos4, double rlist, int
     if (!pos4 || !head || !nn || !nl) return fail(ESP_ERR_INVALID, "null pointer");
     if ((double)totN * cap >= 4294967296.0)
         return fail(ESP_ERR_UNSUPPORTED, "HOOMD-layout rows address 32-bit offsets: totN * cap must be below 2^32");
-    int rc = list_states();
-    if (!rc) rc = setup_cells(cg_nl, rlist, cap);
+    int rc = list_states(st);
+    if (!rc) rc = setup_cells(cg_nl, rlist, cap, st);
     if (rc) return rc;
     NlistArgs a = nlist_args(cg_nl, pos4, rlist, cap);
     a.overflow = d_nl_state;
@@ -1474,8 +1476,8 @@ int esp_batch::build_pairlist(cudaStream_t st, const float* pos4, double rlist, 
     pl_ready = pl_pending = pl_overflow = false;
     pl = PairList{};
     if (rlist != cg_pl.rlist) drop_graphs();  // captured steps hold the previous cell grid's slot maps
-    int rc = list_states();
-    if (!rc) rc = setup_cells(cg_pl, rlist, cap);
+    int rc = list_states(st);
+    if (!rc) rc = setup_cells(cg_pl, rlist, cap, st);
     if (rc) return rc;
     if (pl_cap != cap) {
         plmem.release();

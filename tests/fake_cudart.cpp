@@ -70,8 +70,16 @@ cudaError_t cudaMalloc(void** p, size_t n) { return set((*p = calloc(1, n ? n : 
 cudaError_t cudaFree(void* p) { free(p); return cudaSuccess; }
 cudaError_t cudaHostAlloc(void** p, size_t n, unsigned) { return cudaMalloc(p, n); }
 cudaError_t cudaFreeHost(void* p) { return cudaFree(p); }
-cudaError_t cudaMemcpy(void* d, const void* s, size_t n, cudaMemcpyKind) { memcpy(d, s, n); return cudaSuccess; }
-cudaError_t cudaMemset(void* p, int v, size_t n) { memset(p, v, n); return cudaSuccess; }
+cudaError_t cudaMemcpy(void* d, const void* s, size_t n, cudaMemcpyKind) {
+    log("blocking-copy", nullptr, std::to_string(n));
+    memcpy(d, s, n);
+    return cudaSuccess;
+}
+cudaError_t cudaMemset(void* p, int v, size_t n) {
+    log("default-stream-memset", nullptr, std::to_string(n));
+    memset(p, v, n);
+    return cudaSuccess;
+}
 cudaError_t cudaMemcpyAsync(void* d, const void* s, size_t n, cudaMemcpyKind, cudaStream_t st) {
     log("copy", st, std::to_string(n));
     memcpy(d, s, n);

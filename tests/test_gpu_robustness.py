@@ -41,8 +41,8 @@ def _rows(n, cap):
 
 def _overflowing(b, pos, short):
     # the build waits behind a sleeping stream, so that it cannot have completed
-    # when the caller's evaluation is queued (a build with another capacity than
-    # the last one's waits for the stream: the first of the two)
+    # when the caller's evaluation is queued; what a first build with this
+    # capacity sets up is done before
     b.build_nlist(pos, RLIST, SHORT, *_rows(pos.shape[0], SHORT))
     torch.cuda._sleep(100_000_000)
     b.build_nlist(pos, RLIST, SHORT, *short)

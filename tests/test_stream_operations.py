@@ -1,12 +1,15 @@
-"""An evaluation that ends early, because one of its launches failed, does not
-reach into the next one (CPU: the library over a fake CUDA runtime that logs the
-stream operations and fails one of them).
+"""Stream operations of the library over a fake CUDA runtime that logs them and
+fails one of them (CPU).
 
-The accumulators, the tile counts and the charge mesh are zero between
+An evaluation that ends early, because one of its launches failed, does not
+reach into the next one. The accumulators, the tile counts and the charge mesh are zero between
 evaluations. After a failed launch the caller's stream first waits for the
 kernels already launched on the second stream, then clears the three; the next
 evaluation is launched as if nothing had happened. When the clear fails too, the
 next evaluation starts with it.
+
+A list build and its set-up (first build, another capacity, another radius) do
+everything on the caller's stream.
 """
 import ctypes
 import os
@@ -22,12 +25,40 @@ CUDA = "/usr/local/cuda/include"
 MESH, N = 16, 64
 
 
-def _child():
+def _libs():
     from esp_hoomd_b200 import _lib
     lib = _lib.get_lib()
     fake = ctypes.CDLL(None)
     fake.fake_log.restype = ctypes.c_char_p
     fake.fake_reset.argtypes = [ctypes.c_long, ctypes.c_long]
+    return _lib, lib, fake
+
+
+def _child_lists():
+    _lib, lib, fake = _libs()
+    p = _lib.EspParams()
+    assert lib.esp_params_default(ctypes.byref(p)) == 0
+    p.nx = p.ny = p.nz = MESH
+    n = (ctypes.c_int * 2)(N, N)
+    boxes = (ctypes.c_double * 6)(*[10.0] * 6)
+    b = ctypes.c_void_p()
+    assert lib.esp_batch_create(ctypes.byref(p), 2, n, boxes, None, ctypes.byref(b)) == 0, lib.esp_last_error()
+    buf = (ctypes.c_double * (64 * N)).from_buffer(bytearray(8 * 64 * N))
+    ptr = ctypes.addressof(buf)
+    stream = 4711
+    for rlist, cap in ((3.0, 8), (3.0, 16), (3.4, 16), (3.4, 16)):
+        for build in (lambda: lib.esp_batch_build_nlist(b, stream, ptr, rlist, cap, ptr, ptr, ptr),
+                      lambda: lib.esp_batch_build_pairlist(b, stream, ptr, rlist, cap)):
+            fake.fake_reset(-1, -1)
+            assert build() == 0, lib.esp_last_error()
+            ops = [line.split(" ", 2) for line in fake.fake_log().decode().splitlines()]
+            assert len(ops) > 5 and {o[1] for o in ops} == {str(stream)}, ops
+    lib.esp_batch_destroy(b)
+    print("ok")
+
+
+def _child():
+    _lib, lib, fake = _libs()
     buf = [(ctypes.c_double * (8 * N)).from_buffer(bytearray(64 * N)) for _ in range(8)]
     pos, q, head, nn, nl, force = (ctypes.addressof(b) for b in buf[:6])
 
@@ -78,17 +109,25 @@ def _child():
     print("ok")
 
 
-def test_failed_launch_leaves_clear_state(tmp_path):
+def _run(tmp_path, which):
     if not os.path.exists(os.path.join(CUDA, "cuda_runtime.h")):
         pytest.skip("needs the CUDA headers")
     so = str(tmp_path / "libfake_cudart.so")
     subprocess.run(["g++", "-O1", "-std=c++17", "-shared", "-fPIC", "-I" + CUDA,
                     os.path.join(HERE, "fake_cudart.cpp"), "-o", so], check=True)
     env = dict(os.environ, LD_PRELOAD=so, PYTHONPATH=ROOT)
-    r = subprocess.run([sys.executable, os.path.abspath(__file__)], env=env, cwd=ROOT, capture_output=True, text=True,
+    r = subprocess.run([sys.executable, os.path.abspath(__file__), which], env=env, cwd=ROOT, capture_output=True, text=True,
                        timeout=300)
     assert r.returncode == 0 and r.stdout.strip() == "ok", r.stdout + r.stderr
 
 
+def test_failed_launch_leaves_clear_state(tmp_path):
+    _run(tmp_path, "launches")
+
+
+def test_list_builds_keep_to_their_stream(tmp_path):
+    _run(tmp_path, "lists")
+
+
 if __name__ == "__main__":
-    _child()
+    _child_lists() if sys.argv[1] == "lists" else _child()
