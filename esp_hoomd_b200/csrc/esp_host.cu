@@ -305,7 +305,7 @@ struct esp_batch {
     // hold their address
     DevAlloc ovmem;
     int *d_nl_state = nullptr, *d_pl_state = nullptr;
-    uint32_t* d_nn_limited = nullptr;
+    uint32_t* d_nn_limited = nullptr;  // FP32 batches that built HOOMD-layout rows
     int nn_limited_n = 0;
     int list_states(cudaStream_t st);
     // how many entries the rows of (head, nl) hold when the library's last
@@ -1372,14 +1372,10 @@ int esp_batch::setup_cells(CellGrid& g, double rlist, int cap, cudaStream_t st) 
 }
 
 int esp_batch::list_states(cudaStream_t st) {
-    int rc = 0;
-    if (totN > nn_limited_n) {
-        if ((rc = ovmem.get(d_nn_limited, totN))) return rc;
-        nn_limited_n = totN;
-    }
     if (d_nl_state) return 0;
     int* p = nullptr;
-    if ((rc = ovmem.get(p, 2 * NLIST_STATE))) return rc;
+    const int rc = ovmem.get(p, 2 * NLIST_STATE);
+    if (rc) return rc;
     ESPB_CK(cudaMemsetAsync(p, 0, 2 * NLIST_STATE * sizeof(int), st));
     d_nl_state = p;
     d_pl_state = p + NLIST_STATE;
@@ -1422,6 +1418,9 @@ int esp_batch::build_nlist(cudaStream_t st, const float* pos4, double rlist, int
         return fail(ESP_ERR_UNSUPPORTED, "HOOMD-layout rows address 32-bit offsets: totN * cap must be below 2^32");
     int rc = list_states(st);
     if (!rc) rc = setup_cells(cg_nl, rlist, cap, st);
+    if (!rc && !f64 && totN > nn_limited_n) {
+        if (!(rc = ovmem.get(d_nn_limited, totN))) nn_limited_n = totN;
+    }
     if (rc) return rc;
     NlistArgs a = nlist_args(cg_nl, pos4, rlist, cap);
     a.overflow = d_nl_state;
