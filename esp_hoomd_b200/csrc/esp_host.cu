@@ -428,6 +428,12 @@ struct esp_batch {
     }
 
     LaunchArgs args() const;
+    // a plan that fails leaves nothing set up: every call that needs it is
+    // refused until one succeeds
+    bool planned = false;
+    int need_plan() const {
+        return planned ? 0 : fail(ESP_ERR_INVALID, "no plan: the last one failed and released its arrays");
+    }
     int plan(const esp_params& p, int ns, const int* N_, const double* boxes, const int* mesh_);
     int md_run(cudaStream_t st, float* pos4, float* vel4, const float* q, const unsigned* head, const unsigned* nn,
                const unsigned* nl, float* force4, double* energy, double* virial, int nsteps, double dt,
@@ -460,6 +466,8 @@ struct esp_batch {
 };
 
 int esp_batch::plan(const esp_params& p, int ns, const int* N_, const double* boxes, const int* mesh_) {
+    planned = false;
+    drop_graphs();  // captured steps hold the arrays released here
     mem.release();
     mem64.release();
     f64 = false;
@@ -744,7 +752,6 @@ int esp_batch::plan(const esp_params& p, int ns, const int* N_, const double* bo
     ESPB_CK(cudaMemset(d_acc, 0, (size_t)ns * ACC_STRIDE * sizeof(double)));
     ESPB_CK(cudaMemset(d_rho, 0, (size_t)std::max<long long>(m_off, 1) * sizeof(double)));
     state_dirty = false;
-    drop_graphs();
     {
         // kernel attributes are set here, outside any stream capture
         LaunchArgs a = args();
@@ -785,6 +792,7 @@ int esp_batch::plan(const esp_params& p, int ns, const int* N_, const double* bo
         cudaFree(d_wq);
         if (e != cudaSuccess) return fail(ESP_ERR_CUDA, std::string("influence build: ") + cudaGetErrorString(e));
     }
+    planned = true;
     return 0;
 }
 
@@ -887,15 +895,13 @@ void esp_batch::after_failure(cudaStream_t st, cudaStream_t side) {
     if (cudaStreamIsCapturing(st, &cs) == cudaSuccess && cs != cudaStreamCaptureStatusNone) return;
     cudaGetLastError();
     const std::string why = g_err;
-    if (clear_state(st, side)) {  // the next evaluation tries again
-        cudaGetLastError();
-        g_err = why;
-    }
+    if (clear_state(st, side)) g_err = why;  // the next evaluation tries again
 }
 
 int esp_batch::compute_f64(cudaStream_t st, const double* pos4, const double* q, const unsigned* head,
                            const unsigned* nn, const unsigned* nl, double* force4, double* energy, double* virial,
                            int flags) {
+    if (const int rc = need_plan()) return rc;
     if (!f64) return fail(ESP_ERR_UNSUPPORTED, "context planned for FP32: create it with precision ESP_FP64");
     if (!pos4 || !q || !force4) return fail(ESP_ERR_INVALID, "null position, charge or force pointer");
     if (!(flags & ESP_ALL)) return fail(ESP_ERR_INVALID, "flags select no term");
@@ -1047,6 +1053,7 @@ LaunchArgs esp_batch::args() const {
 int esp_batch::compute(cudaStream_t st, const float* pos4, const float* q, const unsigned* head, const unsigned* nn,
                        const unsigned* nl, float* force4, double* energy, double* virial, int flags,
                        bool want_energy, float* virial_pp, int vpp_pitch, double* external) {
+    if (const int rc = need_plan()) return rc;
     if (f64) return fail(ESP_ERR_UNSUPPORTED, "context planned for FP64: use esp_compute_f64");
     if (!pos4 || !q || !force4) return fail(ESP_ERR_INVALID, "null position, charge or force pointer");
     if (!(flags & ESP_ALL)) return fail(ESP_ERR_INVALID, "flags select no term");
@@ -1152,6 +1159,7 @@ int esp_batch::compute(cudaStream_t st, const float* pos4, const float* q, const
 int esp_batch::md_run(cudaStream_t st, float* pos4, float* vel4, const float* q, const unsigned* head,
                       const unsigned* nn, const unsigned* nl, float* force4, double* energy, double* virial, int nsteps,
                       double dt, int use_graph) {
+    if (const int rc = need_plan()) return rc;
     if (nsteps < 0) return fail(ESP_ERR_INVALID, "negative step count");
     if (!pos4 || !vel4 || !q || !force4) return fail(ESP_ERR_INVALID, "null pointer");
     if (!(head && nn && nl) && (head || nn || nl || !pl_ready))
@@ -1183,6 +1191,7 @@ int esp_batch::md_run(cudaStream_t st, float* pos4, float* vel4, const float* q,
 int esp_batch::md_run_f64(cudaStream_t st, double* pos4, double* vel4, const double* q, const unsigned* head,
                           const unsigned* nn, const unsigned* nl, double* force4, double* energy, double* virial,
                           int nsteps, double dt, double lj_eps, double lj_sigma, double lj_rcut, int use_graph) {
+    if (const int rc = need_plan()) return rc;
     if (!f64) return fail(ESP_ERR_UNSUPPORTED, "context planned for FP32: create it with precision ESP_FP64");
     if (nsteps < 0) return fail(ESP_ERR_INVALID, "negative step count");
     if (!pos4 || !vel4 || !q || !force4 || !head || !nn || !nl)
@@ -1279,6 +1288,7 @@ int esp_batch::run_steps(cudaStream_t& st, GraphKey key, const std::function<int
 }
 
 int esp_batch::spread_only(cudaStream_t st, const float* pos4, const float* q, double* rho_out) {
+    if (const int rc = need_plan()) return rc;
     if (!pos4 || !q || !rho_out) return fail(ESP_ERR_INVALID, "null pointer");
     long long M = 0;
     for (const SysDev& S : sd) M += (long long)S.nx * S.ny * S.nz;
@@ -1412,6 +1422,7 @@ NlistArgs esp_batch::nlist_args(CellGrid& g, const float* pos4, double rlist, in
 
 int esp_batch::build_nlist(cudaStream_t st, const float* pos4, double rlist, int cap, unsigned* head, unsigned* nn,
                            unsigned* nl) {
+    if (const int rc = need_plan()) return rc;
     if (!(rlist > 0) || cap <= 0) return fail(ESP_ERR_INVALID, "rlist and cap must be positive");
     if (!pos4 || !head || !nn || !nl) return fail(ESP_ERR_INVALID, "null pointer");
     if ((double)totN * cap >= 4294967296.0)
@@ -1466,6 +1477,7 @@ int esp_batch::nlist_check(bool wait, int* needed) {
 }
 
 int esp_batch::build_pairlist(cudaStream_t st, const float* pos4, double rlist, int cap) {
+    if (const int rc = need_plan()) return rc;
     if (!(rlist > 0) || cap <= 0) return fail(ESP_ERR_INVALID, "rlist and cap must be positive");
     if (!pos4) return fail(ESP_ERR_INVALID, "null position pointer");
     if (f64) return fail(ESP_ERR_UNSUPPORTED, "the library's pair list serves the FP32 path");
@@ -1568,6 +1580,7 @@ int esp_batch::set_rigid(const int* first, const int* count, double d_oh, double
 }
 
 int esp_batch::nve1(cudaStream_t st, void* pos4, void* vel4, const void* force4, double dt, bool is64) {
+    if (const int rc = need_plan()) return rc;
     const int2* skip = n_mols ? d_rskip : nullptr;
     if (is64)
         ESPB_CK(launch_nve64(1, d_chunks, n_chunks, d_sys, reinterpret_cast<double4*>(pos4),
@@ -1580,6 +1593,7 @@ int esp_batch::nve1(cudaStream_t st, void* pos4, void* vel4, const void* force4,
 }
 
 int esp_batch::nve2(cudaStream_t st, const void* pos4, void* vel4, const void* force4, double dt, bool is64) {
+    if (const int rc = need_plan()) return rc;
     if (is64)
         ESPB_CK(launch_nve64(2, d_chunks, n_chunks, d_sys, nullptr, reinterpret_cast<double4*>(vel4),
                              reinterpret_cast<const double4*>(force4), dt, st));
@@ -1598,6 +1612,7 @@ int esp_batch::autotune(cudaStream_t st, const float* pos4, const float* q, cons
     const std::vector<int> Nv = N;
     const std::vector<double> boxv = box;
     const std::vector<int> meshv = mesh;  // candidates keep the meshes (and so the accuracy)
+    const esp_params given = prm;
     esp_params cur = prm;
     cur.tile = T;
     cur.threads_per_particle = tpp;
@@ -1683,8 +1698,13 @@ done:
     cudaEventDestroy(e1);
     cudaFree(d_force);
     cudaFree(d_e);
-    if (rc) return rc;
-    if ((rc = plan(best, (int)Nv.size(), Nv.data(), boxv.data(), meshv.data()))) return rc;
+    if (!rc) rc = plan(best, (int)Nv.size(), Nv.data(), boxv.data(), meshv.data());
+    if (rc) {
+        // back to the plan that the batch came with
+        const std::string why = g_err;
+        plan(given, (int)Nv.size(), Nv.data(), boxv.data(), meshv.data());
+        return fail(rc, why);
+    }
     if (chosen) *chosen = best;
     return 0;
 }
@@ -1717,6 +1737,18 @@ struct esp_ctx {
     bool dirty = true;
     esp_batch b;
 };
+
+// Plans a context anew when its particle count or anything else has changed; one
+// whose plan failed plans again at the next call.
+static int replan(esp_ctx* c, int N) {
+    if (N == c->N && !c->dirty) return 0;
+    c->dirty = true;
+    c->N = N;
+    const int rc = c->b.plan(c->prm, 1, &c->N, c->L, nullptr);
+    if (rc) return rc;
+    c->dirty = false;
+    return 0;
+}
 
 extern "C" {
 
@@ -1778,12 +1810,7 @@ int esp_compute(esp_ctx* c, void* stream, const float* pos4, const float* charge
                 int flags) {
     if (!c) return fail(ESP_ERR_INVALID, "null context");
     if (N < 0) return fail(ESP_ERR_INVALID, "negative particle count");
-    if (N != c->N || c->dirty) {
-        c->N = N;
-        int rc = c->b.plan(c->prm, 1, &c->N, c->L, nullptr);
-        if (rc) return rc;
-        c->dirty = false;
-    }
+    if (const int rc = replan(c, N)) return rc;
     if (N == 0) {
         cudaStream_t st = (cudaStream_t)stream;
         if (energy) ESPB_CK(cudaMemsetAsync(energy, 0, sizeof(double), st));
@@ -1799,12 +1826,7 @@ int esp_compute_hoomd(esp_ctx* c, void* stream, const float* pos4, const float* 
     if (!c) return fail(ESP_ERR_INVALID, "null context");
     if (N <= 0) return fail(ESP_ERR_INVALID, "particle count must be positive");
     if (!virial_pp || !external7) return fail(ESP_ERR_INVALID, "null virial or external-term pointer");
-    if (N != c->N || c->dirty) {
-        c->N = N;
-        int rc = c->b.plan(c->prm, 1, &c->N, c->L, nullptr);
-        if (rc) return rc;
-        c->dirty = false;
-    }
+    if (const int rc = replan(c, N)) return rc;
     return c->b.compute((cudaStream_t)stream, pos4, charge, head, n_neigh, nlist, force4, nullptr, nullptr, flags,
                         true, virial_pp, virial_pitch, external7);
 }
@@ -1814,12 +1836,7 @@ int esp_compute_f64(esp_ctx* c, void* stream, const double* pos4, const double* 
                     int flags) {
     if (!c) return fail(ESP_ERR_INVALID, "null context");
     if (N < 0) return fail(ESP_ERR_INVALID, "negative particle count");
-    if (N != c->N || c->dirty) {
-        c->N = N;
-        int rc = c->b.plan(c->prm, 1, &c->N, c->L, nullptr);
-        if (rc) return rc;
-        c->dirty = false;
-    }
+    if (const int rc = replan(c, N)) return rc;
     if (N == 0) {
         cudaStream_t st = (cudaStream_t)stream;
         if (energy) ESPB_CK(cudaMemsetAsync(energy, 0, sizeof(double), st));
@@ -1842,17 +1859,13 @@ int esp_destroy(esp_ctx* c) {
 int esp_spread(esp_ctx* c, void* stream, const float* pos4, const float* charge, int N, double* rho) {
     if (!c) return fail(ESP_ERR_INVALID, "null context");
     if (N <= 0) return fail(ESP_ERR_INVALID, "particle count must be positive");
-    if (N != c->N || c->dirty) {
-        c->N = N;
-        int rc = c->b.plan(c->prm, 1, &c->N, c->L, nullptr);
-        if (rc) return rc;
-        c->dirty = false;
-    }
+    if (const int rc = replan(c, N)) return rc;
     return c->b.spread_only((cudaStream_t)stream, pos4, charge, rho);
 }
 
 int esp_get_sort(const esp_ctx* c, void* stream, unsigned* key, unsigned* perm) {
     if (!c || !key || !perm) return fail(ESP_ERR_INVALID, "null argument");
+    if (const int rc = c->b.need_plan()) return rc;
     const int N = c->b.totN;
     cudaStream_t st = (cudaStream_t)stream;
     ESPB_CK(cudaMemcpyAsync(key, c->b.d_key, N * sizeof(unsigned), cudaMemcpyDeviceToDevice, st));
@@ -1862,6 +1875,7 @@ int esp_get_sort(const esp_ctx* c, void* stream, unsigned* key, unsigned* perm) 
 
 int esp_get_potential(const esp_ctx* c, void* stream, float* phi) {
     if (!c || !phi) return fail(ESP_ERR_INVALID, "null argument");
+    if (const int rc = c->b.need_plan()) return rc;
     const SysDev& S = c->b.sd[0];
     // the interior of the halo-padded mesh, plane by plane
     for (int z = 0; z < S.nz; ++z)
@@ -1907,6 +1921,7 @@ int esp_batch_build_pairlist(esp_batch* b, void* stream, const float* pos4, doub
 
 int esp_batch_device_errors(esp_batch* b, int* flags) {
     if (!b || !flags) return fail(ESP_ERR_INVALID, "null argument");
+    if (const int rc = b->need_plan()) return rc;
     ESPB_CK(cudaDeviceSynchronize());
     ESPB_CK(cudaMemcpy(flags, b->d_kerr, sizeof(int), cudaMemcpyDeviceToHost));
     ESPB_CK(cudaMemset(b->d_kerr, 0, sizeof(int)));
@@ -2027,6 +2042,7 @@ int esp_batch_lj(esp_batch* b, void* stream, const float* pos4, const unsigned* 
                  const unsigned* nlist, double epsilon, double sigma, double r_cut, float* force4, double* energy) {
     if (!b || !pos4 || !head || !n_neigh || !nlist || !force4) return fail(ESP_ERR_INVALID, "null argument");
     if (!(sigma > 0) || !(r_cut > 0)) return fail(ESP_ERR_INVALID, "sigma and r_cut must be positive");
+    if (const int rc = b->need_plan()) return rc;
     ESPB_CK(launch_lj(b->d_chunks, b->n_chunks, b->d_sys, pos4, head, n_neigh, nlist, b->row_limit(head, nlist),
                       epsilon, sigma, r_cut, force4, energy, false, (cudaStream_t)stream));
     return 0;
@@ -2037,6 +2053,7 @@ int esp_batch_lj_f64(esp_batch* b, void* stream, const double* pos4, const unsig
                      double* energy) {
     if (!b || !pos4 || !head || !n_neigh || !nlist || !force4) return fail(ESP_ERR_INVALID, "null argument");
     if (!(sigma > 0) || !(r_cut > 0)) return fail(ESP_ERR_INVALID, "sigma and r_cut must be positive");
+    if (const int rc = b->need_plan()) return rc;
     ESPB_CK(launch_lj(b->d_chunks, b->n_chunks, b->d_sys, pos4, head, n_neigh, nlist, b->row_limit(head, nlist),
                       epsilon, sigma, r_cut, force4, energy, true, (cudaStream_t)stream));
     return 0;

@@ -18,10 +18,15 @@ namespace espb {
 // Records `msg` as this thread's last error and returns `code`.
 int fail(int code, const std::string& msg);
 
-#define ESPB_CK(x)                                                                                             \
-    do {                                                                                                       \
-        cudaError_t e_ = (x);                                                                                  \
-        if (e_ != cudaSuccess) return ::espb::fail(ESP_ERR_CUDA, std::string(#x) + ": " + cudaGetErrorString(e_)); \
+// The runtime's last-error word is taken with the error: left there, the next
+// launch check would find it.
+#define ESPB_CK(x)                                                                                         \
+    do {                                                                                                   \
+        cudaError_t e_ = (x);                                                                              \
+        if (e_ != cudaSuccess) {                                                                           \
+            cudaGetLastError();                                                                            \
+            return ::espb::fail(ESP_ERR_CUDA, std::string(#x) + ": " + cudaGetErrorString(e_));            \
+        }                                                                                                  \
     } while (0)
 
 // Required k-space resolution kappa_N = pi r_c / h for a relative RMS force
@@ -49,6 +54,7 @@ struct DevAlloc {
         if (n == 0) n = 1;
         cudaError_t e = cudaMalloc((void**)&p, n * sizeof(T));
         if (e != cudaSuccess) {
+            cudaGetLastError();
             p = nullptr;
             return fail(ESP_ERR_ALLOC, std::string("cudaMalloc of ") + std::to_string(n * sizeof(T)) +
                                            " bytes failed: " + cudaGetErrorString(e));

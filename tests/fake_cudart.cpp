@@ -1,6 +1,6 @@
 // A CUDA runtime without a GPU, preloaded over the library's: memory is host
-// memory, nothing runs, every stream operation is logged, and one launch or
-// asynchronous memset can be made to fail.
+// memory, nothing runs, every stream operation is logged, and one launch,
+// asynchronous memset or allocation (or all from one on) can be made to fail.
 #include <cuda_runtime.h>
 
 #include <cstdio>
@@ -15,6 +15,7 @@ static std::map<const void*, std::string>& kernels() {
 }
 static std::string g_log;
 static long g_next = 1, g_launch = 0, g_fail_launch = -1, g_memset = 0, g_fail_memset = -1;
+static long g_malloc = 0, g_fail_malloc_from = -1, g_fail_malloc_to = -1;
 static cudaError_t g_last = cudaSuccess;
 static struct { dim3 g, b; size_t s; cudaStream_t st; } g_call;
 
@@ -37,6 +38,11 @@ void fake_reset(long fail_launch, long fail_memset) {
     g_launch = g_memset = 0;
     g_fail_launch = fail_launch;
     g_fail_memset = fail_memset;
+}
+void fake_fail_mallocs(long from, long to) {  // [from, to) counted from here
+    g_malloc = 0;
+    g_fail_malloc_from = from;
+    g_fail_malloc_to = to;
 }
 const char* fake_log() { return g_log.c_str(); }
 
@@ -66,7 +72,11 @@ cudaError_t cudaGetLastError() {
     return e;
 }
 const char* cudaGetErrorString(cudaError_t) { return "fake error"; }
-cudaError_t cudaMalloc(void** p, size_t n) { return set((*p = calloc(1, n ? n : 1)) ? cudaSuccess : cudaErrorMemoryAllocation); }
+cudaError_t cudaMalloc(void** p, size_t n) {
+    const long k = g_malloc++;
+    *p = k >= g_fail_malloc_from && k < g_fail_malloc_to ? nullptr : calloc(1, n ? n : 1);
+    return set(*p ? cudaSuccess : cudaErrorMemoryAllocation);
+}
 cudaError_t cudaFree(void* p) { free(p); return cudaSuccess; }
 cudaError_t cudaHostAlloc(void** p, size_t n, unsigned) { return cudaMalloc(p, n); }
 cudaError_t cudaFreeHost(void* p) { return cudaFree(p); }

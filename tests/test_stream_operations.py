@@ -8,6 +8,10 @@ kernels already launched on the second stream, then clears the three; the next
 evaluation is launched as if nothing had happened. When the clear fails too, the
 next evaluation starts with it.
 
+A plan that fails (allocations, sizes) leaves nothing that a later call launches
+over: contexts plan again, a failed autotuning goes back to the plan it came
+with, and where that fails too every call is refused.
+
 A list build and its set-up (first build, another capacity, another radius) do
 everything on the caller's stream.
 """
@@ -53,6 +57,63 @@ def _child_lists():
             assert build() == 0, lib.esp_last_error()
             ops = [line.split(" ", 2) for line in fake.fake_log().decode().splitlines()]
             assert len(ops) > 5 and {o[1] for o in ops} == {str(stream)}, ops
+    lib.esp_batch_destroy(b)
+    print("ok")
+
+
+def _child_plans():
+    _lib, lib, fake = _libs()
+    fake.fake_fail_mallocs.argtypes = [ctypes.c_long, ctypes.c_long]
+    p = _lib.EspParams()
+    assert lib.esp_params_default(ctypes.byref(p)) == 0
+    p.nx = p.ny = p.nz = MESH
+    buf = (ctypes.c_double * (64 * N)).from_buffer(bytearray(8 * 64 * N))
+    ptr = ctypes.addressof(buf)
+    forever = 1 << 40
+
+    def launches():
+        return sum(line.split(" ")[0] == "launch" for line in fake.fake_log().decode().splitlines())
+
+    # a context whose plan for a new particle count fails plans again at the next call
+    h = ctypes.c_void_p()
+    assert lib.esp_create(ctypes.byref(p), 10.0, 10.0, 10.0, N, ctypes.byref(h)) == 0
+    compute = lambda n: lib.esp_compute(h, None, ptr, ptr, n, ptr, ptr, ptr, ptr, None, None, 3)  # noqa: E731
+    assert compute(N) == 0
+    fake.fake_fail_mallocs(5, forever)
+    fake.fake_reset(-1, -1)
+    assert [compute(N // 2), compute(N // 2)] == [-3, -3]
+    assert lib.esp_get_sort(h, None, ptr, ptr) == -1 and lib.esp_get_potential(h, None, ptr) == -1
+    assert compute(1 << 26) == -4 and compute(1 << 26) == -4  # too many particles
+    assert launches() == 0
+    fake.fake_fail_mallocs(-1, -1)
+    assert compute(N // 2) == 0 and compute(N) == 0
+    lib.esp_destroy(h)
+    # autotuning: the k-th allocation fails alone, then everything from it on
+    n = (ctypes.c_int * 1)(N)
+    box = (ctypes.c_double * 3)(10.0, 10.0, 10.0)
+    b = ctypes.c_void_p()
+    assert lib.esp_batch_create(ctypes.byref(p), 1, n, box, None, ctypes.byref(b)) == 0
+    tune = lambda: lib.esp_batch_autotune(b, None, ptr, ptr, ptr, ptr, ptr, 3, 1, None, None, 0)  # noqa: E731
+    calls = [lambda: lib.esp_batch_compute(b, None, ptr, ptr, ptr, ptr, ptr, ptr, None, None, 3),
+             lambda: lib.esp_batch_build_nlist(b, None, ptr, 3.0, 8, ptr, ptr, ptr),
+             lambda: lib.esp_batch_build_pairlist(b, None, ptr, 3.0, 8),
+             lambda: lib.esp_batch_nve_step1(b, None, ptr, ptr, ptr, 0.1),
+             lambda: lib.esp_batch_nve_step2(b, None, ptr, ptr, ptr, 0.1),
+             lambda: lib.esp_batch_lj(b, None, ptr, ptr, ptr, ptr, 1.0, 1.0, 2.5, ptr, None),
+             lambda: lib.esp_batch_md_run(b, None, ptr, ptr, ptr, ptr, ptr, ptr, ptr, None, None, 1, 0.1, 0)]
+    fake.fake_fail_mallocs(-1, -1)
+    assert tune() == 0 and [c() for c in calls] == [0] * 7
+    for k in (2, 9, 40, 60):  # the trial's outputs and plans
+        fake.fake_fail_mallocs(k, k + 1)
+        assert tune() == -3
+        fake.fake_fail_mallocs(-1, -1)
+        assert [c() for c in calls] == [0] * 7, k
+    fake.fake_fail_mallocs(9, forever)
+    assert tune() == -3
+    fake.fake_reset(-1, -1)
+    assert [c() for c in calls] == [-1] * 7 and launches() == 0
+    fake.fake_fail_mallocs(-1, -1)
+    assert tune() == 0 and [c() for c in calls] == [0] * 7
     lib.esp_batch_destroy(b)
     print("ok")
 
@@ -129,5 +190,9 @@ def test_list_builds_keep_to_their_stream(tmp_path):
     _run(tmp_path, "lists")
 
 
+def test_failed_plans_are_not_used(tmp_path):
+    _run(tmp_path, "plans")
+
+
 if __name__ == "__main__":
-    _child_lists() if sys.argv[1] == "lists" else _child()
+    {"lists": _child_lists, "plans": _child_plans, "launches": _child}[sys.argv[1]]()
